@@ -114,38 +114,36 @@ void free_all_locked(DevCache& C) {
   C.bytes = 0;
 }
 
-// Side L when the coupling graph is exactly the periodic square (d = 2) or
-// cubic (d = 3) lattice of side 16 or 32 in the file's site order (site
+// Side L (3 to 32) when the coupling graph is exactly the periodic square
+// (d = 2) or cubic (d = 3) lattice in the file's site order (site
 // x L^2 + y L + z, z fastest; every row the 2d neighbours at +-1 along each
-// axis modulo L, in any order, no self-coupling), else 0.  Rows of such a
-// lattice fill half or whole 32-bit words, which the plain form's bitmap
-// Houdayer search relies on.
+// axis modulo L, in any order, no self-coupling), else 0.  The Houdayer
+// searches on bitmaps rely on it: a lattice row fits a 32-bit word (and, with
+// L 16 or 32, fills half or all of it, which the plain form's needs).
 uint32_t lattice_side(const HostInstance& h, uint32_t udeg) {
   if (udeg != 4 && udeg != 6) return 0;
   const uint32_t d = udeg / 2;
-  for (uint32_t L : {16u, 32u}) {
-    const uint64_t n = d == 2 ? (uint64_t)L * L : (uint64_t)L * L * L;
-    if (n != h.n) continue;
-    for (uint32_t i = 0; i < h.n; ++i) {
-      const uint32_t r0 = h.row_ptr[i], r1 = h.row_ptr[i + 1];
-      if (r1 - r0 != udeg) return 0;
-      uint32_t want[6];
-      uint32_t k = 0, stride = 1;
-      for (uint32_t a = 0; a < d; ++a, stride *= L) {
-        const uint32_t c = (i / stride) % L;
-        want[k++] = i - c * stride + ((c + 1) % L) * stride;
-        want[k++] = i - c * stride + ((c + L - 1) % L) * stride;
-      }
-      std::sort(want, want + udeg);
-      uint32_t got[6];
-      for (uint32_t e = 0; e < udeg; ++e) got[e] = h.col[r0 + e];
-      std::sort(got, got + udeg);
-      for (uint32_t e = 0; e < udeg; ++e)
-        if (got[e] != want[e]) return 0;
+  uint32_t L = 3;
+  while (L < 32 && (d == 2 ? L * L : L * L * L) < h.n) ++L;
+  if ((d == 2 ? L * L : L * L * L) != h.n) return 0;
+  for (uint32_t i = 0; i < h.n; ++i) {
+    const uint32_t r0 = h.row_ptr[i], r1 = h.row_ptr[i + 1];
+    if (r1 - r0 != udeg) return 0;
+    uint32_t want[6];
+    uint32_t k = 0, stride = 1;
+    for (uint32_t a = 0; a < d; ++a, stride *= L) {
+      const uint32_t c = (i / stride) % L;
+      want[k++] = i - c * stride + ((c + 1) % L) * stride;
+      want[k++] = i - c * stride + ((c + L - 1) % L) * stride;
     }
-    return L;
+    std::sort(want, want + udeg);
+    uint32_t got[6];
+    for (uint32_t e = 0; e < udeg; ++e) got[e] = h.col[r0 + e];
+    std::sort(got, got + udeg);
+    for (uint32_t e = 0; e < udeg; ++e)
+      if (got[e] != want[e]) return 0;
   }
-  return 0;
+  return L;
 }
 }  // namespace
 
@@ -250,6 +248,54 @@ void tamc_inst_release(tamc_inst* d) {
   tamc_gpu_release(g);
 }
 
+// Sliced rows of the colour-ordered CSR (FastInst::sl_*): the sites of a class
+// by descending row length (a counting sort), 32 to a slice as long as its
+// longest row (made even).  On rows of uneven length the lanes of a warp then run loops of
+// about the same length and read consecutive entries.
+static void slice_rows(tamc_inst* d, const std::vector<uint32_t>& frp, const std::vector<uint2>& fent,
+                       UploadPack& pack) {
+  const uint32_t n = d->n, len_max = d->max_deg;
+  std::vector<uint32_t> cls(d->ncolors + 1, 0), off(1, 0);
+  std::vector<uint16_t> site, pos(n);
+  site.reserve(n + 32 * d->ncolors);
+  std::vector<uint32_t> first(len_max + 2);
+  for (uint32_t c = 0; c < d->ncolors; ++c) {
+    const uint32_t s0 = d->color_off[c], s1 = d->color_off[c + 1];
+    const uint32_t base = (uint32_t)site.size();
+    std::fill(first.begin(), first.end(), 0);
+    for (uint32_t s = s0; s < s1; ++s) ++first[len_max - (frp[s + 1] - frp[s]) + 1];
+    for (uint32_t k = 1; k < first.size(); ++k) first[k] += first[k - 1];
+    site.resize(base + (s1 - s0 + 31) / 32 * 32, 0xffff);
+    for (uint32_t s = s0; s < s1; ++s) {
+      const uint32_t p = base + first[len_max - (frp[s + 1] - frp[s])]++;
+      site[p] = (uint16_t)s;
+      pos[s] = (uint16_t)p;
+    }
+    for (uint32_t p = base; p < site.size(); p += 32)  // a slice's first site has its longest row
+      off.push_back(off.back() + (frp[site[p] + 1] - frp[site[p]] + 1) / 2 * 2);
+    cls[c + 1] = (uint32_t)(site.size() / 32);
+  }
+  // positions are 16 bits; many small classes of long rows would be mostly padding
+  if (site.size() > 65535 || (uint64_t)off.back() * 32 > std::max<uint64_t>(2 * fent.size(), 65536)) return;
+  d->sl_n = (uint32_t)off.size() - 1;
+  d->sl_rows = off.back();
+  std::vector<uint2> ent((size_t)d->sl_rows * 32);
+  for (uint32_t x = 0; x < 32 * d->sl_n; ++x) {
+    const uint32_t g = x / 32, w = off[g + 1] - off[g];
+    const uint32_t s = site[x] == 0xffff ? site[32 * g] : site[x];
+    const uint32_t len = site[x] == 0xffff ? 0 : frp[s + 1] - frp[s];
+    for (uint32_t e = 0; e < w; ++e) {
+      const uint2 v = e < len ? fent[frp[s] + e] : make_uint2(s, 0);
+      ent[((size_t)off[g] + e) * 32 + x % 32] = make_uint2(4 * v.x, v.y);
+    }
+  }
+  pack.add(&d->d_sl_cls, cls.data(), cls.size());
+  pack.add(&d->d_sl_off, off.data(), off.size());
+  pack.add(&d->d_sl_site, site.data(), site.size());
+  pack.add(&d->d_sl_pos, pos.data(), pos.size());
+  pack.add(&d->d_sl_ent, ent.data(), ent.size());
+}
+
 // Host side of an upload: every array of the instance (reference order, ICM
 // graph, colour order, lattice layouts) into `pack`, and the host fields of
 // `d`.  Touches no device state, so uploads of several instances prepare in
@@ -331,7 +377,8 @@ static void inst_prepare(tamc_inst* d, const HostInstance& h, UploadPack& pack) 
     if (fbias[s] != 0.0f) d->pmj = 0;
   for (size_t e = 0; e < fent.size() && d->pmj; ++e)
     if ((fent[e].y & 0x7fffffffu) != 0x3f800000u) d->pmj = 0;  // |J| == 1.0f
-  d->lat_L = lattice_side(h, d->udeg);
+  d->lat_any = lattice_side(h, d->udeg);
+  d->lat_L = d->lat_any == 16 || d->lat_any == 32 ? d->lat_any : 0;
   std::vector<float> fJt;
   std::vector<uint16_t> fcolt;
   if (d->lat_L) {
@@ -349,6 +396,8 @@ static void inst_prepare(tamc_inst* d, const HostInstance& h, UploadPack& pack) 
     pack.add(&d->d_fJt, fJt.data(), fJt.size());
     pack.add(&d->d_fcolt, fcolt.data(), fcolt.size());
   }
+  if (h.n <= 65535 && (d->self_loops || (d->udeg != 3 && d->udeg != 4 && d->udeg != 6)))
+    slice_rows(d, frp, fent, pack);
   pack.add(&d->d_fbias, fbias.data(), fbias.size());
   pack.add(&d->d_fkd, fkd.data(), fkd.size());
   pack.add(&d->d_fsus, fsus.data(), fsus.size());

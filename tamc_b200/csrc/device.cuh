@@ -288,6 +288,11 @@ struct tamc_inst {
   uint32_t udeg = 0;                 // entries per row when every row has the same count, else 0
   int pmj = 0;                       // +-1 couplings, no field, no self-loop, rows of 4 or 6 entries
   uint32_t lat_L = 0;                // periodic L^d lattice in file order (L 16 or 32, d = udeg / 2), else 0
+  uint32_t lat_any = 0;              // the same for any side from 3 to 32
+  uint32_t sl_n = 0, sl_rows = 0;    // sliced rows (FastInst::sl_*)
+  uint32_t *d_sl_cls = nullptr, *d_sl_off = nullptr;
+  uint16_t *d_sl_site = nullptr, *d_sl_pos = nullptr;
+  uint2* d_sl_ent = nullptr;
   float* d_fbias = nullptr;          // n
   void* arena = nullptr;             // one allocation holding every array above
   size_t arena_bytes = 0;

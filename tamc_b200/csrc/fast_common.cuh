@@ -24,6 +24,16 @@ struct FastInst {  // colour-ordered instance (device pointers)
   uint32_t udeg;              // entries per row if uniform (row s = [s*udeg, (s+1)*udeg)), else 0
   int pmj;                    // +-1 couplings, zero field, no self-loop, udeg 4 or 6 (multi-spin coding)
   uint32_t lat_L;             // side of a periodic square / cubic lattice in file order (16 or 32), else 0
+  uint32_t lat_any;           // side of such a lattice of any side from 3 to 32, else 0
+  // sliced rows (instances whose rows are not all of 3, 4 or 6 entries without
+  // self-couplings, n <= 65535): each colour class sorted by row length and
+  // cut into slices of 32 sites
+  uint32_t sl_n, sl_rows;     // slices; their lengths summed
+  const uint32_t* sl_cls;     // [ncolors + 1] first slice of each class
+  const uint32_t* sl_off;     // [sl_n + 1] first row of 32 entries of each slice
+  const uint16_t* sl_site;    // [sl_n][32] sites (65535 beyond a class's last)
+  const uint16_t* sl_pos;     // [n] position of each site in sl_site
+  const uint2* sl_ent;        // [sl_rows][32] (4 * column, J bits) in row order, padded with (own column, 0)
   const float* fJt;           // lattice instances: couplings [udeg][n] (entry m of colour row s at m n + s)
   const uint16_t* fcolt;      // lattice instances: columns [udeg][n], same layout
   const float* bias;          // n

@@ -38,6 +38,11 @@ struct tamc_pt::FastState {
   int head_stage = 0;  // the head kernel stages replica words for measurements
   uint32_t grid_cap = 0;
   std::map<uint32_t, cudaGraphExec_t> graphs;  // captured chunks of K rounds
+  // ladder form (one run over many CTAs, ladder_pt.cu)
+  bool ladder = false;
+  tamc::LadJob lad{};
+  tamc::DBuf<char> lad_mem;
+  tamc::DBuf<tamc::LadJob> d_lad;
   tamc::DBuf<unsigned long long> prof;          // per-phase cycles (TAMC_PHASE_PROF=1)
   ~FastState() {
     for (auto& kv : graphs) cudaGraphExecDestroy(kv.second);
@@ -420,19 +425,127 @@ static bool choose_plain(tamc_pt* pt) {
   return plain;
 }
 
-void fast_pt_create(tamc_pt* pt, uint64_t seed) {
-  pt->fast = new tamc_pt::FastState();
-  fill_job(pt, seed, pt->fast);
-  if (choose_plain(pt)) {
-    plain_setup(pt);
-    plain_init_energies(pt, true);
-    return;
-  }
+static void fused_setup(tamc_pt* pt) {
   const TileChoice t = tune_tile(pt->g, pt->fast->job);
   pt->fast->T = t.T;
   pt->fast->job.csr_smem = t.csr;
   pt->fast->smem = fused_smem_bytes(pt->fast->job, t.T, t.csr);
   if (pt->fast->smem > pt->g->smem_optin) fail(TAMC_E_UNSUPPORTED, "instance too large for the fused PT kernel");
+}
+
+// ---- ladder form: a replica per CTA
+// Whether the other forms take the run (what they refuse is refused).
+static bool other_forms_take(const tamc_gpu* g, const PtJob& j) {
+  if (fused_smem_bytes(j, 128, false) <= g->smem_optin) {
+    const TileChoice t = heuristic_tile(g, j);
+    return fits(g, j, t.T, t.csr);
+  }
+  return plain_head_bytes(j, false) <= g->smem_optin && plain_icm_bytes(j) <= g->smem_optin;
+}
+
+// Sets the run up in the ladder form if it takes it: all its CTAs, one per
+// replica, are resident at once; rows in shared memory where they fit.
+// A single run takes it whenever it can: over square and cubic lattices, random
+// regular graphs and QUBOs of 16 to 8000 sites, 8 to 64 temperatures, 2 and 4
+// chains, with and without Houdayer moves, a round took 5.0-70 us against the
+// better of 5.9-113 us in the other two forms, at best 7.3 times less (3-D
+// Gaussian, 512 sites, 64 temperatures: 12.6 against 39 us plain, 81 fused) and
+// nowhere more (least gain: 4 sites' worth of work, 10.3 against 11.0 us).
+// CTA size: a thread per site up to 512, 1024 from 4096 sites on (1728 sites
+// Gaussian: 15.4 us at 512, 16.2 at 1024; 6000-site QUBO: 69 and 61 us).
+static bool ladder_setup(tamc_pt* pt) {
+  auto* F = pt->fast;
+  const PtJob& j = F->job;
+  const char* f = getenv("TAMC_PT_FORM");
+  if (f && (!strcmp(f, "plain") || !strcmp(f, "fused"))) return false;
+  if (g_no_autotune || g_defer_init || j.icm_uf || !other_forms_take(pt->g, j)) return false;
+  uint32_t T0 = j.n >= 4096 ? 1024u : j.n >= 512 ? 512u : j.n >= 256 ? 256u : 128u;
+  if (const char* e = getenv("TAMC_PT_T")) T0 = (uint32_t)std::min(1024, std::max(128, atoi(e) / 128 * 128));
+  for (uint32_t T = T0; T >= 128; T /= 2)
+    for (int rows : {1, 0}) {
+      const size_t smem = ladder_smem(j, rows);
+      if (smem > pt->g->smem_optin - 512) continue;  // (the kernel's static shared memory is above 1 KB)
+      F->lad.J = j;
+      ladder_shape(F->lad, rows, 0);
+      if (F->lad.ncta > ladder_capacity(pt->g, T, smem)) continue;
+      F->T = T;
+      F->smem = smem;
+      F->lad_mem.alloc(ladder_scratch_bytes(j));
+      ladder_bind(F->lad, F->lad_mem.p);
+      F->lad.err = pt->out.err_flag();
+      F->d_lad.alloc(1);
+      F->ladder = true;
+      if (getenv("TAMC_DEBUG"))
+        fprintf(stderr, "[tamc] PT form n=%u nt=%u C=%u: ladder, %u CTAs of %u threads, rows in smem %d\n", j.n, j.nt,
+                j.C, F->lad.ncta, T, rows);
+      return true;
+    }
+  return false;
+}
+
+// Rounds [begin, end) (none: only the initial state, init != 0).
+static void ladder_rounds(tamc_pt* pt, uint32_t begin, uint32_t end, int init) {
+  TraceRange tr("tamc ladder rounds");
+  auto* F = pt->fast;
+  cudaStream_t st = pt->g->stream;
+  PtJob& j = F->job;
+  j.init = init;
+  j.sweep_begin = begin;
+  j.sweep_end = end;
+  j.m_base = pt->m_next;
+  j.s_base = pt->s_next;
+  F->lad.J = j;
+  TAMC_CUDA(tamc::copy_async(F->d_lad.p, &F->lad, sizeof(LadJob), cudaMemcpyHostToDevice, st));
+  TAMC_CUDA(cudaMemsetAsync(F->lad.bar, 0, ladder_sync_bytes(j), st));
+  const uint32_t blocks = (uint32_t)(((uint64_t)((j.n + 31) / 32) * j.nw + 7) / 8);
+  ladder_launch(st, F->d_lad.p, nullptr, 1, F->lad.ncta, F->T, F->smem, std::min(blocks, 592u));
+  pt->g->count(3);
+}
+
+// The run's CTAs gave a round up (they were not all running within the
+// barrier's limit): its state is the one before those rounds, and it goes on in
+// one of the other forms.
+static void ladder_leave(tamc_pt* pt) {
+  auto* F = pt->fast;
+  cudaStream_t st = pt->g->stream;
+  F->ladder = false;
+  if (fused_smem_bytes(F->job, 128, false) <= pt->g->smem_optin) {
+    fused_setup(pt);
+    return;
+  }
+  plain_setup(pt);
+  const PlainCtl c{pt->next_sweep, pt->m_next, pt->s_next, 0, 0, 0};
+  TAMC_CUDA(tamc::copy_async(F->ctl.p, &c, sizeof(c), cudaMemcpyHostToDevice, st));
+  TAMC_CUDA(cudaStreamSynchronize(st));
+}
+
+// Draws (init 1) or takes over (init 2) the replicas and sets their energies.
+static void init_state(tamc_pt* pt, int init) {
+  auto* F = pt->fast;
+  if (F->ladder) {
+    ladder_rounds(pt, pt->next_sweep, pt->next_sweep, init);
+    pt->out.dirty = true;
+    pt->out.drain(pt->g->stream);
+    if (!pt->out.gave_up) return;
+    ladder_leave(pt);
+  }
+  if (F->plain) plain_init_energies(pt, init == 1);
+  else launch_one(pt, pt->next_sweep, pt->next_sweep, init);
+}
+
+void fast_pt_create(tamc_pt* pt, uint64_t seed) {
+  pt->fast = new tamc_pt::FastState();
+  fill_job(pt, seed, pt->fast);
+  if (ladder_setup(pt)) {  // the initial replicas are drawn with the first rounds
+    pt->fast->init_pending = true;
+    return;
+  }
+  if (choose_plain(pt)) {
+    plain_setup(pt);
+    plain_init_energies(pt, true);
+    return;
+  }
+  fused_setup(pt);
   if (g_defer_init) {  // drawn by the batch's first chunk launch (same chain)
     pt->fast->init_pending = true;
     return;
@@ -440,28 +553,42 @@ void fast_pt_create(tamc_pt* pt, uint64_t seed) {
   launch_one(pt, 0, 0, 1);  // random initial replicas and their energies
 }
 
-// The deferred initial replicas of a batch run, when something reads or runs
-// the run before the batch's first chunk.
+// Deferred initial replicas, when something reads or runs the run before its
+// first rounds draw them.
 static void ensure_init(tamc_pt* pt) {
   if (pt->fast && pt->fast->init_pending) {
     pt->fast->init_pending = false;
-    launch_one(pt, pt->next_sweep, pt->next_sweep, 1);
+    init_state(pt, 1);
   }
 }
 
 void fast_pt_run(tamc_pt* pt, uint32_t sweep_end) {
-  ensure_init(pt);
+  if (!pt->fast->ladder) ensure_init(pt);
   const PtCfg& c = pt->cfg;
   while (pt->next_sweep < sweep_end) {
     const uint32_t b = pt->next_sweep;
     const uint32_t e = std::min(sweep_end, b + pt->out.cap);
-    if (pt->fast->plain) plain_run_chunk(pt, e - b);
-    else launch_one(pt, b, e, 0);
+    if (pt->fast->ladder) {
+      ladder_rounds(pt, b, e, pt->fast->init_pending ? 1 : 0);
+      pt->out.dirty = true;
+      pt->out.drain(pt->g->stream);
+      if (pt->out.gave_up) {
+        ladder_leave(pt);
+        ensure_init(pt);
+        continue;
+      }
+      pt->fast->init_pending = false;
+    } else if (pt->fast->plain) {
+      plain_run_chunk(pt, e - b);
+    } else {
+      launch_one(pt, b, e, 0);
+    }
     pt->out.dirty = true;
     pt->m_next += count_sched(c.sample, c.meas_init, c.num_sweeps, b, e);
     pt->s_next += count_sched(c.sample_states, c.meas_init, c.num_sweeps, b, e);
     pt->next_sweep = e;
-    pt->out.drain(pt->g->stream);
+    if (pt->fast->ladder) pt->out.dirty = false;  // drained above
+    else pt->out.drain(pt->g->stream);
   }
 }
 
@@ -501,8 +628,7 @@ void fast_pt_set_state(tamc_pt* pt, const int8_t* spins) {
     }
   TAMC_CUDA(tamc::copy_async(F->W.p, W.data(), W.size() * 4, cudaMemcpyHostToDevice, st));
   F->init_pending = false;  // the set state replaces the initial replicas
-  if (F->plain) plain_init_energies(pt, false);
-  else launch_one(pt, pt->next_sweep, pt->next_sweep, 2);  // recompute energies
+  init_state(pt, 2);        // their energies
 }
 
 void fast_pt_acceptance(tamc_pt* pt, uint32_t* acc) {

@@ -91,6 +91,63 @@ void plain_launch_sweep(cudaStream_t st, const PtJob& j, const PtJob* d_job, Pla
                         uint32_t ntask, long long* acc, uint32_t grid_cap);
 void plain_launch_init(cudaStream_t st, const PtJob* d_job, long long* acc, int random, uint32_t grid);
 
+// Ladder form (ladder_pt.cu): one run over the GPU, a CTA per replica.
+struct LadGs {
+  int have;
+  float minE;
+  uint32_t count;
+};
+struct LadBook {  // a run's bookkeeping between the round kernel and the commit
+  uint8_t* tags;
+  uint32_t *acc, *dhist, *rtrips;
+  LadGs* gs;
+};
+__host__ __device__ inline size_t lad_book_bytes(uint32_t C, uint32_t nt) {
+  const size_t R = (size_t)C * nt;
+  return R * 12 + (size_t)C * 4 + sizeof(LadGs) + R;
+}
+__host__ __device__ inline LadBook lad_book_view(char* b, uint32_t C, uint32_t nt) {
+  const size_t R = (size_t)C * nt;
+  LadBook B;
+  B.acc = (uint32_t*)b;
+  B.dhist = B.acc + R;
+  B.rtrips = B.dhist + 2 * R;
+  B.gs = (LadGs*)(B.rtrips + C);
+  B.tags = (uint8_t*)(B.gs + 1);
+  return B;
+}
+struct LadJob {
+  PtJob J;
+  uint32_t cta0, ncta;     // the run's CTAs in the launch: chain-major, one per slot
+  int32_t mode, rows_smem; // row kind; rows kept in shared memory
+  uint32_t* bits;          // [2][C][nt][ceil(n/32)] replicas published for the exchange, by round parity
+  uint32_t* post;          // [C][nt][ceil(n/32)] replicas after their sweep, for the slot's other replica
+  double* pe;              // [2][C][nt][2] published energies (cached, energy_ref)
+  float* pg;               // [2][C][nt] energies after the sweep (ground-state tracking)
+  uint32_t* cand;          // [2][C][nt][2 ceil(n/64)] states of replicas below the running minimum
+  char* book;
+  uint32_t* bar;           // barrier arrivals; zero at launch
+  uint32_t* flag;          // [C][nt] rounds whose `post` is there; zero at launch
+  uint32_t* err;           // set by a CTA that gave up; zero at launch
+  uint32_t polls, pad_;    // polls of a wait before a CTA gives up
+};
+// Bytes of the arrays above for a run; ladder_bind places them at `base`.
+size_t ladder_scratch_bytes(const PtJob& j);
+size_t ladder_bind(LadJob& a, char* base);
+// Bytes from `bar` on that are zero at launch (the barrier and the flags).
+size_t ladder_sync_bytes(const PtJob& j);
+// Shared memory of a CTA (`rows`: rows kept in shared memory).
+size_t ladder_smem(const PtJob& j, int rows);
+void ladder_shape(LadJob& a, int rows, uint32_t cta0);
+// CTAs of T threads and `smem` bytes that are resident at once.
+uint32_t ladder_capacity(const tamc_gpu* g, uint32_t T, size_t smem);
+// The three launches of a range of rounds: bitmaps from the words, the rounds
+// (one cooperative launch of `grid` CTAs), results back.  The runs' barrier
+// counters and error flags must be zero.  A run whose error flag is set
+// afterwards keeps the state it had.
+void ladder_launch(cudaStream_t st, const LadJob* d_jobs, const uint32_t* d_cta_job, uint32_t njobs, uint32_t grid,
+                   uint32_t T, size_t smem, uint32_t open_grid);
+
 // tamc_pt glue (single-instance handle in fast mode)
 void fast_pt_create(tamc_pt* pt, uint64_t seed);
 void fast_pt_run(tamc_pt* pt, uint32_t sweep_end);

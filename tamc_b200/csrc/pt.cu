@@ -92,9 +92,12 @@ GsLog PtOutputs::log() const {
 
 void PtOutputs::drain(cudaStream_t st) {
   if (!dirty) return;  // nothing has run since the last drain: the host copy is current
-  uint32_t cnt = 0;
-  TAMC_CUDA(tamc::copy_async(&cnt, gs_count.p, 4, cudaMemcpyDeviceToHost, st));
+  uint32_t cells[4] = {};
+  TAMC_CUDA(tamc::copy_async(cells, gs_cells.p, sizeof(cells), cudaMemcpyDeviceToHost, st));
   TAMC_CUDA(cudaStreamSynchronize(st));
+  const uint32_t cnt = cells[0];
+  gave_up = cells[3] != 0;
+  if (gave_up) TAMC_CUDA(cudaMemsetAsync(err_flag(), 0, 4, st));
   if (cnt > cap) fail(TAMC_E_INVAL, "ground-state log overflow");
   if (cnt) {
     const size_t nw = (n + 63) / 64;

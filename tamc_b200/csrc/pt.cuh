@@ -67,7 +67,7 @@ struct PtOutputs {
   DBuf<int32_t> q;
   DBuf<float> sus;
   DBuf<uint8_t> samp;
-  DBuf<char> gs_cells;  // one block holding the three cells below
+  DBuf<char> gs_cells;  // one block holding the three cells below and a fourth, the ladder form's error flag
   DBuf<uint32_t> gs_count;
   DBuf<int> gs_have;
   DBuf<float> gs_min;
@@ -77,12 +77,14 @@ struct PtOutputs {
   uint32_t cap = 0;
   uint32_t pending = 0;  // tracked sweeps since the last drain
   bool dirty = true;     // rounds may have logged entries since the last drain
+  bool gave_up = false;  // the last drain found the error flag set (and cleared it)
   std::vector<uint32_t> h_steps;
   std::vector<float> h_E;
   std::vector<uint64_t> h_words;  // concatenated
   void init(const PtCfg& c, uint32_t n_, uint32_t nchi_, cudaStream_t st);
   MeasOut meas(const PtCfg& c) const;
   GsLog log() const;
+  uint32_t* err_flag() const { return reinterpret_cast<uint32_t*>(gs_cells.p) + 3; }
   void drain(cudaStream_t st);  // synchronous
 };
 

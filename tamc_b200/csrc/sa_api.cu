@@ -38,6 +38,14 @@ FastInst make_fast_inst(const tamc_inst* d) {
   F.udeg = d->udeg;
   F.pmj = d->pmj;
   F.lat_L = d->lat_L;
+  F.lat_any = d->lat_any;
+  F.sl_n = d->sl_n;
+  F.sl_rows = d->sl_rows;
+  F.sl_cls = d->d_sl_cls;
+  F.sl_off = d->d_sl_off;
+  F.sl_site = d->d_sl_site;
+  F.sl_pos = d->d_sl_pos;
+  F.sl_ent = d->d_sl_ent;
   F.fJt = d->d_fJt;
   F.fcolt = d->d_fcolt;
   F.bias = d->d_fbias;
