@@ -148,6 +148,7 @@ static void ref_create(tamc_pt* pt, Xo master) {
   pt->visited.alloc(std::max(n, I->g_nodes));
   pt->queue.alloc(std::max(n, I->g_nodes));
   pt->rows.alloc(n);
+  pt->pick.alloc((size_t)c.C / 2 * c.nt);
   pt->rng.alloc(rv.size());
   pt->err.alloc(1);
   std::vector<uint32_t> perm(R);
@@ -192,6 +193,7 @@ static RefPt ref_view(tamc_pt* pt) {
   P.visited = pt->visited.p;
   P.queue = pt->queue.p;
   P.rows = pt->rows.p;
+  P.pick = pt->pick.p;
   return P;
 }
 
@@ -212,13 +214,13 @@ static void ref_round(tamc_pt* pt, uint32_t i) {
   const ExpTable& X = pt->g->exp;
   uint64_t k = 0;
   if (c.threads > 1) {  // parallel_pt_loop (src/pt.rs:446-450)
-    if (c.icm) { ref_icm(st, I, P, X, pt->rng.p, pt->err.p); ++k; }
+    if (c.icm) k += ref_icm(st, I, pt->inst->nnz, P, X, pt->rng.p, pt->err.p);
     ref_exchange_threaded(st, P, X, pt->rng.p);
-    ref_sweep_threaded(st, I, P, X, pt->rng.p);
-    k += 3;
+    ref_sweep_threaded(st, I, pt->inst->nnz, P, X, pt->rng.p);
+    k += 2;
   } else {  // pt_loop (src/pt.rs:493-497)
-    if (c.icm) { ref_icm(st, I, P, X, pt->rng.p, pt->err.p); ++k; }
-    ref_serial_round(st, I, P, X, pt->rng.p);
+    if (c.icm) k += ref_icm(st, I, pt->inst->nnz, P, X, pt->rng.p, pt->err.p);
+    ref_serial_round(st, I, pt->inst->nnz, P, X, pt->rng.p);
     ++k;
   }
   if (i >= c.meas_init) {

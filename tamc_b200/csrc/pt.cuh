@@ -122,6 +122,7 @@ struct tamc_pt {
   tamc::DBuf<uint32_t> visited;
   tamc::DBuf<uint32_t> queue;
   tamc::DBuf<float> rows;
+  tamc::DBuf<uint32_t> pick;
   tamc::DBuf<tamc::Xo> rng;
   tamc::DBuf<int> err;
   // fast-mode state lives behind an opaque pointer (fast_pt.cu)

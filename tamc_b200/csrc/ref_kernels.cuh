@@ -32,6 +32,7 @@ struct RefPt {  // replica state of one PT run (device pointers)
   uint32_t* visited;  // scratch [max(n, 1)]
   uint32_t* queue;    // scratch [max(n, 1)]
   float* rows;        // scratch [max(n, 1)]
+  uint32_t* pick;     // scratch [C / 2 * nt] Houdayer seed indices of a round
 };
 
 struct MeasOut {  // PtIcmThermalSamples buffers on the device
@@ -54,10 +55,11 @@ struct GsLog {  // ground-state trajectory ring for one run
 
 RefInst make_ref_inst(const tamc_inst* d);
 void ref_energy_all(cudaStream_t st, const RefInst& I, const int8_t* spins, float* energy, uint32_t R);
-void ref_icm(cudaStream_t st, const RefInst& I, const RefPt& P, const ExpTable& X, Xo* rng, int* err);
+// Each enqueues one step of a round; ref_icm returns how many launches it took.
+uint32_t ref_icm(cudaStream_t st, const RefInst& I, uint64_t nnz, const RefPt& P, const ExpTable& X, Xo* rng, int* err);
 void ref_exchange_threaded(cudaStream_t st, const RefPt& P, const ExpTable& X, Xo* rngs);
-void ref_sweep_threaded(cudaStream_t st, const RefInst& I, const RefPt& P, const ExpTable& X, Xo* rngs);
-void ref_serial_round(cudaStream_t st, const RefInst& I, const RefPt& P, const ExpTable& X, Xo* rng);
+void ref_sweep_threaded(cudaStream_t st, const RefInst& I, uint64_t nnz, const RefPt& P, const ExpTable& X, Xo* rngs);
+void ref_serial_round(cudaStream_t st, const RefInst& I, uint64_t nnz, const RefPt& P, const ExpTable& X, Xo* rng);
 void ref_measure(cudaStream_t st, const RefInst& I, const RefPt& P, const MeasOut& O, uint32_t m, bool meas,
                  uint32_t smp, bool samp);
 void ref_gs_track(cudaStream_t st, const RefInst& I, const RefPt& P, const GsLog& L, uint32_t step);
