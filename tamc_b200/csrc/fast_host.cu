@@ -915,6 +915,22 @@ struct ChunkRunner {
     return L;
   }
 
+  // The round each run of a chunk ends before (see enqueue).
+  static std::vector<uint32_t> chunk_ends(const std::vector<tamc_pt*>& act, uint32_t chunk, bool balance) {
+    double c_max = 1.0;  // the largest cost of one round among the runs
+    for (auto* pt : act) c_max = std::max(c_max, (double)pt->fast->job.cost / std::max(1u, pt->cfg.num_sweeps));
+    std::vector<uint32_t> ends;
+    for (auto* pt : act) {
+      uint32_t rounds = chunk;
+      if (balance) {
+        const double c_x = (double)pt->fast->job.cost / std::max(1u, pt->cfg.num_sweeps);
+        rounds = (uint32_t)std::min<double>(8.0 * chunk, chunk * std::max(1.0, c_max / std::max(c_x, 1.0)));
+      }
+      ends.push_back(std::min(pt->cfg.num_sweeps, pt->next_sweep + std::min(rounds, pt->out.cap)));
+    }
+    return ends;
+  }
+
   // Advances every run in `act` by up to `chunk` rounds.  With `balance`, a run
   // whose rounds cost less than the costliest run's gets proportionally more
   // rounds (up to 8x), so that every run does about the same work per launch
@@ -931,9 +947,13 @@ struct ChunkRunner {
   // Enqueues one chunk into slot `sl` (which must not be busy) and returns
   // without waiting; the runs' host-side progress is advanced at once.
   // Returns false when no run has rounds left.
+  // (`ends`: the round each run of `act` ends before, instead of `chunk`.)
   bool enqueue(tamc_gpu* g, Slot& sl, std::vector<tamc_pt*> act, uint32_t chunk, bool use_graph, bool balance,
-               bool by_size = false) {
+               bool by_size = false, const std::vector<uint32_t>* given = nullptr) {
     cudaStream_t st = g->stream;
+    std::map<tamc_pt*, uint32_t> given_end;
+    if (given)
+      for (size_t x = 0; x < act.size(); ++x) given_end[act[x]] = (*given)[x];
     act.erase(std::remove_if(act.begin(), act.end(),
                              [](tamc_pt* p) { return p->next_sweep >= p->cfg.num_sweeps; }),
               act.end());
@@ -990,27 +1010,23 @@ struct ChunkRunner {
       reserve(na);
     }
     PtJob* const h_jobs = sl.h_jobs;
-    std::vector<uint32_t> ends(na);
-    double c_max = 1.0;  // the largest cost of one round among the runs
-    for (auto* pt : act) c_max = std::max(c_max, (double)pt->fast->job.cost / std::max(1u, pt->cfg.num_sweeps));
+    std::vector<uint32_t> ends;
+    if (given)
+      for (auto* pt : act) ends.push_back(given_end[pt]);
+    else
+      ends = chunk_ends(act, chunk, balance);
     for (uint32_t x = 0; x < na; ++x) {
       tamc_pt* pt = act[x];
       PtJob j = pt->fast->job;
       j.init = pt->fast->init_pending ? 1 : 0;  // a batch run's deferred initial replicas
       j.sweep_begin = pt->next_sweep;
-      uint32_t rounds = chunk;
-      if (balance) {
-        const double c_x = (double)pt->fast->job.cost / std::max(1u, pt->cfg.num_sweeps);
-        rounds = (uint32_t)std::min<double>(8.0 * chunk, chunk * std::max(1.0, c_max / std::max(c_x, 1.0)));
-      }
-      ends[x] = std::min(pt->cfg.num_sweeps, pt->next_sweep + std::min(rounds, pt->out.cap));
       j.sweep_end = ends[x];
       j.m_base = pt->m_next;
       j.s_base = pt->s_next;
       j.count_out = counts.p + x;
       h_jobs[x] = j;
     }
-    sl.next = balance ? 8 * chunk : chunk;
+    sl.next = given ? 1024 : balance ? 8 * chunk : chunk;
     if (split && !aux) {
       int least = 0, greatest = 0;
       TAMC_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
@@ -1108,17 +1124,233 @@ struct ChunkRunner {
     finish(g, *b, lazy, 1);
   }
 
+  // ---- several runs in the ladder form (ladder_pt.cu): launches of as many
+  // runs as have all their CTAs resident at once, one after another.
+  DBuf<LadJob> d_lad;
+  DBuf<uint32_t> d_map;  // CTA -> run of its launch
+  DBuf<char> d_sync;     // the runs' barriers and flags
+  struct LadGroup {
+    size_t first = 0, count = 0;
+    uint32_t T = 0, grid = 0;
+    size_t smem = 0;
+  };
+  // How the rounds of a step are launched: the first `ladder` runs (by
+  // descending size) in ladder groups, the others in one fused launch.
+  struct Plan {
+    std::vector<LadGroup> groups;
+    size_t ladder = 0;
+    double us = 0.0;
+  };
+  // Expected microseconds per round.  Ladder, in a launch that fills the GPU with
+  // CTAs of T threads (48 replicas a run; rows of a QUBO / 3-D Gaussian and 2-D
+  // +-J lattices): 512 threads 200 sites 20, 700 38, 2000 45, 6000 80 / 12^3 19,
+  // 32^2 14; 256: 30, 35, 57, 95 / 27, 18; 128: 32, 43, 78, 152 / 38, 20.
+  // Fused, one run to an SM: QUBO 30, 80, 195, 670; 12^3 Gaussian 113; 32^2 +-J 22.
+  static double ladder_us(const PtJob& j, uint32_t T) {
+    const double n = j.n;
+    if (j.F.lat_any) return T >= 512 ? 11 + 0.0045 * n : T >= 256 ? 13 + 0.008 * n : 16 + 0.013 * n;
+    return T >= 512 ? 25 + 0.0092 * n : T >= 256 ? 26 + 0.0125 * n : 27 + 0.022 * n;
+  }
+  static double fused_us(const PtJob& j) {
+    const double nr = (double)j.n * j.C * j.ntp;
+    return 12 + nr * (j.msc ? 0.16e-3 : j.F.udeg ? 1.2e-3 : j.n > 2048 ? 2.3e-3 : 2e-3);
+  }
+  // The ladder launches of runs [k, k1) of `act`: as many runs at a time as have
+  // all their CTAs resident.  The CTA size of a launch is the one with the most
+  // replica rounds per expected time, or the fastest that takes all that remain.
+  static bool ladder_groups(tamc_gpu* g, const std::vector<tamc_pt*>& act, const std::vector<uint32_t>& rounds,
+                            size_t k, size_t k1, Plan& P) {
+    const char* t_env = getenv("TAMC_PT_T");
+    while (k < k1) {
+      LadGroup best;
+      double best_us = 0.0, best_rate = 0.0;
+      bool best_all = false;
+      for (uint32_t T : {512u, 256u, 128u}) {
+        if (t_env && (uint32_t)atoi(t_env) != T) continue;
+        LadGroup G;
+        G.first = k;
+        G.T = T;
+        double us = 0.0, work = 0.0;
+        for (size_t x = k; x < k1; ++x) {
+          const PtJob& j = act[x]->fast->job;
+          const size_t own = ladder_smem(j, 0), smem = std::max(G.smem, own);
+          if (j.icm_uf || own > g->smem_optin - 512) return false;
+          if (G.grid + j.C * j.nt > ladder_capacity(g, T, smem)) break;
+          G.smem = smem;
+          G.grid += j.C * j.nt;
+          ++G.count;
+          us = std::max(us, ladder_us(j, T) * rounds[x]);
+          work += (double)j.C * j.nt * ladder_us(j, 512) * rounds[x];
+        }
+        if (!G.count) continue;
+        const bool all = k + G.count == k1;
+        const double rate = work / us;
+        if (!best.count || (all && (!best_all || us < best_us)) || (!all && !best_all && rate > best_rate)) {
+          best = G;
+          best_us = us;
+          best_rate = rate;
+          best_all = all;
+        }
+      }
+      if (!best.count) return false;
+      P.groups.push_back(best);
+      P.us += best_us;
+      k += best.count;
+    }
+    P.ladder = k1;
+    return true;
+  }
+  // The plan with the least expected time for the runs `act` (by descending
+  // size) and their rounds: up to 24 places to split them at.  The ladder form
+  // has to promise a tenth less than the fused one.
+  static Plan make_plan(tamc_gpu* g, const std::vector<tamc_pt*>& act, const std::vector<uint32_t>& rounds,
+                        bool split = true) {
+    const size_t na = act.size();
+    const char* f = getenv("TAMC_PT_FORM");
+    Plan best;
+    if (f && !strcmp(f, "fused")) return best;
+    std::vector<double> most(na + 1, 0.0), sum(na + 1, 0.0);  // of the fused runs from x on
+    for (size_t x = na; x-- > 0;) {
+      const double us = fused_us(act[x]->fast->job) * rounds[x];
+      most[x] = std::max(most[x + 1], us);
+      sum[x] = sum[x + 1] + us;
+    }
+    auto fused_from = [&](size_t x) { return std::max(most[x], sum[x] / g->num_sms); };
+    const bool force = f && !strcmp(f, "ladder");
+    best.us = force ? 1e30 : 0.9 * fused_from(0);
+    size_t last = 0;
+    for (size_t c = 1; c <= 24; ++c) {
+      const size_t k = split && !force ? (na * c + 23) / 24 : na;
+      if (k == last) continue;
+      last = k;
+      Plan P;
+      if (!ladder_groups(g, act, rounds, 0, k, P)) break;
+      if (k < na) P.us += fused_from(k);
+      if (P.us < best.us) best = std::move(P);
+    }
+    if (getenv("TAMC_DEBUG")) {
+      fprintf(stderr, "[tamc] plan for %zu runs: fused %.0f us, chosen %.0f us, %zu in the ladder form:", na, fused_from(0),
+              best.us, best.ladder);
+      for (const LadGroup& G : best.groups)
+        fprintf(stderr, " %zu runs, %u CTAs of %u threads, %zu bytes;", G.count, G.grid, G.T, G.smem);
+      fprintf(stderr, "\n");
+    }
+    return best;
+  }
+  // Advances the runs act[0 .. plan.ladder) to `ends` in the plan's launches and
+  // waits.  Runs whose rounds were given up take theirs in the fused form.
+  void run_ladder(tamc_gpu* g, const std::vector<tamc_pt*>& all, const std::vector<uint32_t>& ends, const Plan& plan) {
+    cudaStream_t st = g->stream;
+    const std::vector<LadGroup>& groups = plan.groups;
+    const std::vector<tamc_pt*> act(all.begin(), all.begin() + plan.ladder);
+    const size_t na = act.size();
+    reserve((uint32_t)na);
+    if (d_lad.n < na) d_lad.alloc(na);
+    std::vector<LadJob> lad(na);
+    std::vector<uint32_t> map;
+    std::vector<size_t> sync_off(na);
+    size_t sync = 0;
+    for (size_t x = 0; x < na; ++x) {
+      sync_off[x] = sync;
+      sync += (ladder_sync_bytes(act[x]->fast->job) + 15) & ~(size_t)15;
+    }
+    if (d_sync.n < sync) d_sync.alloc(sync);
+    TAMC_CUDA(cudaMemsetAsync(d_sync.p, 0, sync, st));
+    for (const LadGroup& G : groups) {
+      uint32_t cta0 = 0;
+      for (size_t k = 0; k < G.count; ++k) {
+        const size_t x = G.first + k;
+        tamc_pt* pt = act[x];
+        auto* F = pt->fast;
+        if (!F->lad_mem.p) F->lad_mem.alloc(ladder_scratch_bytes(F->job));
+        LadJob& L = lad[x];
+        L.J = F->job;
+        L.J.init = F->init_pending ? 1 : 0;
+        L.J.sweep_begin = pt->next_sweep;
+        L.J.sweep_end = ends[x];
+        L.J.m_base = pt->m_next;
+        L.J.s_base = pt->s_next;
+        L.J.count_out = counts.p + x;
+        ladder_bind(L, F->lad_mem.p);
+        L.bar = reinterpret_cast<uint32_t*>(d_sync.p + sync_off[x]);
+        L.flag = L.bar + 1;
+        L.err = pt->out.err_flag();
+        ladder_shape(L, 0, cta0);
+        cta0 += L.ncta;
+        map.insert(map.end(), L.ncta, (uint32_t)k);
+      }
+    }
+    if (d_map.n < map.size()) d_map.alloc(map.size());
+    TAMC_CUDA(tamc::copy_async(d_lad.p, lad.data(), na * sizeof(LadJob), cudaMemcpyHostToDevice, st));
+    TAMC_CUDA(tamc::copy_async(d_map.p, map.data(), map.size() * 4, cudaMemcpyHostToDevice, st));
+    size_t m0 = 0;
+    Slot& sl = slots[0];
+    TAMC_CUDA(cudaEventRecord(sl.ev[0], st));
+    for (const LadGroup& G : groups) {
+      ladder_launch(st, d_lad.p + G.first, d_map.p + m0, (uint32_t)G.count, G.grid, G.T, G.smem, 32);
+      g->count(3);
+      m0 += G.grid;
+    }
+    TAMC_CUDA(cudaEventRecord(sl.ev[1], st));
+    TAMC_CUDA(tamc::copy_async(sl.h_counts, counts.p, na * 4, cudaMemcpyDeviceToHost, st));
+    TAMC_CUDA(cudaStreamSynchronize(st));
+    float ms = 0.0f;
+    TAMC_CUDA(cudaEventElapsedTime(&ms, sl.ev[0], sl.ev[1]));
+    dev_ms += ms;
+    launches += groups.size();
+    std::vector<tamc_pt*> again;
+    std::vector<uint32_t> again_ends;
+    for (size_t x = 0; x < na; ++x) {
+      tamc_pt* pt = act[x];
+      if (sl.h_counts[x] == LAD_GAVE_UP) {
+        TAMC_CUDA(cudaMemsetAsync(pt->out.err_flag(), 0, 4, st));
+        again.push_back(pt);
+        again_ends.push_back(ends[x]);
+        continue;
+      }
+      const PtCfg& c = pt->cfg;
+      pt->fast->init_pending = false;
+      pt->m_next += count_sched(c.sample, c.meas_init, c.num_sweeps, pt->next_sweep, ends[x]);
+      pt->s_next += count_sched(c.sample_states, c.meas_init, c.num_sweeps, pt->next_sweep, ends[x]);
+      pt->next_sweep = ends[x];
+      pt->out.dirty = sl.h_counts[x] != 0;
+      if (sl.h_counts[x]) pt->out.drain(st);
+      else pt->out.pending = 0;
+    }
+    if (!again.empty() && enqueue(g, slots[0], std::move(again), 0, false, false, false, &again_ends))
+      finish(g, slots[0], false, 1);
+  }
+
   // Advances every run in `act` by up to `chunk` rounds (one chunk) and waits.
   void run(tamc_gpu* g, std::vector<tamc_pt*> act, uint32_t chunk, bool use_graph, bool balance = false,
            bool lazy_logs = false) {
     if (enqueue(g, slots[0], std::move(act), chunk, use_graph, balance)) finish(g, slots[0], lazy_logs, 1);
   }
 
+  bool run_all_ladder(tamc_gpu* g, const std::vector<tamc_pt*>& jobs) {
+    std::vector<tamc_pt*> act(jobs);
+    std::stable_sort(act.begin(), act.end(), [](tamc_pt* x, tamc_pt* y) { return x->fast->job.n > y->fast->job.n; });
+    if (act.empty()) return false;
+    for (bool first = true;; first = false) {
+      act.erase(std::remove_if(act.begin(), act.end(), [](tamc_pt* p) { return p->next_sweep >= p->cfg.num_sweeps; }),
+                act.end());
+      if (act.empty()) return true;
+      const std::vector<uint32_t> ends = chunk_ends(act, 1024, false);
+      std::vector<uint32_t> rounds;
+      for (size_t x = 0; x < act.size(); ++x) rounds.push_back(ends[x] - act[x]->next_sweep);
+      const Plan plan = make_plan(g, act, rounds, false);
+      if (plan.ladder != act.size() || (first && plan.groups.size() != 1)) return false;
+      run_ladder(g, act, ends, plan);
+    }
+  }
+
   // Runs every run in `jobs` to its end, chunk after chunk, with the next
   // chunk enqueued before the previous one has finished (two buffer sets, so
   // no host gap between chunks); the logs are drained lazily, looking two
   // chunks ahead, and once at the end.
+  // A small batch whose CTAs are all resident in the ladder form runs there.
   void run_all(tamc_gpu* g, const std::vector<tamc_pt*>& jobs, uint32_t chunk) {
+    if (run_all_ladder(g, jobs)) return;
     uint32_t k = 0;
     for (;; k ^= 1) {
       TraceRange tr("tamc batch chunk");
@@ -1130,8 +1362,25 @@ struct ChunkRunner {
   }
 };
 
+// One step of a server: every run by up to `chunk` rounds (balanced), in the
+// forms of the plan with the least expected time.
 void chunk_run(ChunkRunner* r, tamc_gpu* g, std::vector<tamc_pt*>& act, uint32_t chunk) {
-  r->run(g, act, chunk, false, true);
+  std::vector<tamc_pt*> by_size;
+  for (auto* pt : act)
+    if (pt->next_sweep < pt->cfg.num_sweeps) by_size.push_back(pt);
+  if (by_size.empty()) return;
+  std::stable_sort(by_size.begin(), by_size.end(),
+                   [](tamc_pt* x, tamc_pt* y) { return x->fast->job.n > y->fast->job.n; });
+  const std::vector<uint32_t> ends = ChunkRunner::chunk_ends(by_size, chunk, true);
+  std::vector<uint32_t> rounds;
+  for (size_t x = 0; x < by_size.size(); ++x) rounds.push_back(ends[x] - by_size[x]->next_sweep);
+  const ChunkRunner::Plan plan = ChunkRunner::make_plan(g, by_size, rounds);
+  if (plan.ladder) r->run_ladder(g, by_size, ends, plan);
+  if (plan.ladder < by_size.size()) {
+    const std::vector<tamc_pt*> rest(by_size.begin() + plan.ladder, by_size.end());
+    const std::vector<uint32_t> rest_ends(ends.begin() + plan.ladder, ends.end());
+    if (r->enqueue(g, r->slots[0], rest, 0, false, false, false, &rest_ends)) r->finish(g, r->slots[0], false, 1);
+  }
 }
 ChunkRunner* chunk_runner_new() { return new ChunkRunner(); }
 void chunk_runner_free(ChunkRunner* r) { delete r; }

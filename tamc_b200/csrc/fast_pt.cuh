@@ -116,6 +116,7 @@ __host__ __device__ inline LadBook lad_book_view(char* b, uint32_t C, uint32_t n
   B.tags = (uint8_t*)(B.gs + 1);
   return B;
 }
+constexpr uint32_t LAD_GAVE_UP = 0xffffffffu;  // PtJob::count_out of a run whose rounds were given up
 struct LadJob {
   PtJob J;
   uint32_t cta0, ncta;     // the run's CTAs in the launch: chain-major, one per slot

@@ -149,12 +149,12 @@ __host__ __device__ inline LadSm lad_carve(const LadDims d) {
     S.site = take(d.nslice * 64);
     S.pos = take(n * 2);
     S.soff = take((d.nslice + 1) * 4);
-    S.kd = take(d.self ? n * 4 : 0);
   }
   if (d.rows) {
     S.bias = take(d.msc ? 0 : n * 4);
     S.colp = take(d.deg ? (d.deg + 1) / 2 * n * 4 : d.nsl * 64);
     S.J = take(d.msc ? 0 : d.deg ? d.deg * n * 4 : d.nsl * 128);
+    S.kd = take(d.self && !d.deg ? n * 4 : 0);
   }
   S.bytes = o;
   return S;
@@ -755,7 +755,7 @@ __device__ __noinline__ longlong2 lad_sweep(const PtJob& J, const LadSm S, uint3
   const uint32_t* const soff = lad_at<uint32_t>(S.soff);
   const uint16_t* const site = lad_at<uint16_t>(S.site);
   const bool self = MODE == LAD_ROWS && J.self_loops;
-  const float* const kd = lad_at<float>(S.kd);
+  const float* const kd = RS ? lad_at<float>(S.kd) : J.F.kd;
   long long* const red = lad_at<long long>(S.red);
   long long a = 0, q = 0;
   int units = 0;
@@ -962,7 +962,7 @@ __device__ void lad_run(const LadJob& A) {
     for (uint32_t x = tid; x <= J.F.sl_n; x += T) lad_at<uint32_t>(S.soff)[x] = J.F.sl_off[x];
     for (uint32_t x = tid; x < n; x += T) {
       lad_at<uint16_t>(S.pos)[x] = J.F.sl_pos[x];
-      if (J.self_loops) lad_at<float>(S.kd)[x] = J.F.kd[x];
+      if (RS && J.self_loops) lad_at<float>(S.kd)[x] = J.F.kd[x];
     }
   }
   if (J.F.lat_any)
@@ -1255,11 +1255,14 @@ __global__ void k_ladder_open(const LadJob* __restrict__ jobs) {
 }
 
 // The results of the runs' rounds into their words, energies and bookkeeping;
-// nothing where a CTA gave up.
+// nothing (and LAD_GAVE_UP as the log count) where a CTA gave up.
 __global__ void k_ladder_commit(const LadJob* __restrict__ jobs) {
   const LadJob& A = jobs[blockIdx.y];
   const PtJob& J = A.J;
-  if (*A.err) return;
+  if (*A.err) {
+    if (blockIdx.x == 0 && threadIdx.x == 0 && J.count_out) *J.count_out = LAD_GAVE_UP;
+    return;
+  }
   const uint32_t lane = threadIdx.x & 31u, nwb = (J.n + 31) / 32;
   const uint64_t total = (uint64_t)nwb * J.nw;
   const uint32_t par = (J.sweep_end - J.sweep_begin) & 1u;

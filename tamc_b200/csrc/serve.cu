@@ -3,12 +3,13 @@
 // Requests (instance + PT-ICM method) arrive at any time.  A scheduling step
 // admits queued requests while the number of active requests stays under
 // `max_active` and their estimated HBM footprint stays under the budget, runs
-// one chunk of PT rounds for every active request in a single fused launch
-// (each request's replica state stays on the device between steps), and
-// retires requests that reached their sweep budget or their target energy.
-// Every request runs exactly the Markov chain it would run alone: its Philox
-// streams depend only on its own seed and sweep index, and its state is only
-// touched by the CTA that owns it during a launch.
+// one chunk of PT rounds for every active request -- in one fused launch, in
+// launches of the ladder form, or the largest in those and the others in that,
+// whichever promises to take least time -- (each request's replica state stays
+// on the device between steps), and retires requests that reached their sweep
+// budget or their target energy.  Every request runs exactly the Markov chain it
+// would run alone: its Philox streams depend only on its own seed and sweep
+// index, and its state is only touched by its own CTAs during a launch.
 #include <algorithm>
 #include <chrono>
 #include <cmath>
@@ -20,7 +21,7 @@
 #include "fast_pt.cuh"
 
 namespace tamc {
-extern thread_local bool g_no_autotune;
+extern thread_local bool g_no_autotune, g_defer_init;
 struct ChunkRunner;
 void chunk_run(ChunkRunner* r, tamc_gpu* g, std::vector<tamc_pt*>& act, uint32_t chunk);
 ChunkRunner* chunk_runner_new();
@@ -156,35 +157,55 @@ int tamc_serve_step(tamc_server* s, uint32_t* active, uint32_t* queued) {
   TraceRange tr("tamc serve step");
   if (!s) fail(TAMC_E_INVAL, "null server");
   TAMC_CUDA(cudaSetDevice(s->g->device));
-  // admission: FIFO while slots and HBM budget allow
-  // A request that cannot be set up (its instance or run is refused) fails
-  // alone: it is marked TAMC_REQ_FAILED with the reason and the others go on.
-  while (!s->queue.empty() && s->active.size() < s->max_active && s->used + s->queue.front()->footprint <= s->budget) {
-    Request* r = s->queue.front();
-    s->queue.pop_front();
-    int rc = tamc_gpu_instance_upload(s->g, r->h, &r->dinst);
-    if (rc == TAMC_OK) {
-      g_no_autotune = true;
-      rc = tamc_gpu_pt_create(r->dinst, &r->p, r->seed, TAMC_MODE_FAST, &r->pt);
-      g_no_autotune = false;
+  // admission: FIFO while slots and HBM budget allow.  The requests admitted
+  // together are uploaded together (host preparation on several threads).  A
+  // request that cannot be set up (its instance or run is refused) fails alone:
+  // it is marked TAMC_REQ_FAILED with the reason, and what it held is offered to
+  // the queue again.
+  for (bool more = true; more;) {
+    more = false;
+    std::vector<Request*> in;
+    while (!s->queue.empty() && s->active.size() + in.size() < s->max_active &&
+           s->used + s->queue.front()->footprint <= s->budget) {
+      in.push_back(s->queue.front());
+      s->queue.pop_front();
+      s->used += in.back()->footprint;
     }
-    if (rc == TAMC_OK && r->pt->fast && r->pt->fast_plain()) {
-      rc = TAMC_E_UNSUPPORTED;
-      set_error("request too large for the fused PT kernel");
+    if (in.size() >= 4) {  // (fewer are not worth the threads: 24 QUBOs of 64-8192 sites 11 -> 4 ms)
+      std::vector<const tamc_host_instance*> hs;
+      for (auto* r : in) hs.push_back(r->h);
+      std::vector<tamc_inst*> ds(in.size(), nullptr);
+      if (tamc_gpu_instance_upload_many(s->g, (uint32_t)in.size(), hs.data(), ds.data()) == TAMC_OK)
+        for (size_t k = 0; k < in.size(); ++k) in[k]->dinst = ds[k];
     }
-    if (rc != TAMC_OK) {
-      r->error = tamc_last_error();
-      if (r->pt) tamc_gpu_pt_destroy(r->pt);
-      if (r->dinst) tamc_gpu_instance_destroy(r->dinst);
-      r->pt = nullptr;
-      r->dinst = nullptr;
-      r->state = TAMC_REQ_FAILED;
-      r->t_done = Clock::now();
-      continue;
+    for (Request* r : in) {
+      int rc = r->dinst ? TAMC_OK : tamc_gpu_instance_upload(s->g, r->h, &r->dinst);
+      if (rc == TAMC_OK) {
+        g_no_autotune = true;
+        g_defer_init = true;  // its first rounds draw the initial replicas
+        rc = tamc_gpu_pt_create(r->dinst, &r->p, r->seed, TAMC_MODE_FAST, &r->pt);
+        g_no_autotune = false;
+        g_defer_init = false;
+      }
+      if (rc == TAMC_OK && r->pt->fast && r->pt->fast_plain()) {
+        rc = TAMC_E_UNSUPPORTED;
+        set_error("request too large for the fused PT kernel");
+      }
+      if (rc != TAMC_OK) {
+        r->error = tamc_last_error();
+        if (r->pt) tamc_gpu_pt_destroy(r->pt);
+        if (r->dinst) tamc_gpu_instance_destroy(r->dinst);
+        r->pt = nullptr;
+        r->dinst = nullptr;
+        r->state = TAMC_REQ_FAILED;
+        r->t_done = Clock::now();
+        s->used -= r->footprint;
+        more = true;
+        continue;
+      }
+      r->state = TAMC_REQ_ACTIVE;
+      s->active.push_back(r);
     }
-    r->state = TAMC_REQ_ACTIVE;
-    s->used += r->footprint;
-    s->active.push_back(r);
   }
   if (!s->active.empty()) {
     std::vector<tamc_pt*> pts;

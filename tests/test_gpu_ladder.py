@@ -105,3 +105,41 @@ def test_ladder_rounds_that_are_given_up_run_in_another_form(tb, gpu, monkeypatc
     monkeypatch.setenv("TAMC_PT_FORM", "ladder")
     monkeypatch.setenv("TAMC_LADDER_POLLS", "0")
     _same(want, _everything(tb.PtRun(d, p, 3).run()))
+
+
+# ladder: several runs a launch, two launches where 296 CTAs of 512 threads are
+# resident at once; polls 0: every run's rounds are given up and run fused
+@pytest.mark.parametrize("form,threads,polls", [("ladder", "512", None), ("ladder", "128", None), ("", None, None),
+                                                ("ladder", "256", "0")])
+@pytest.mark.parametrize("how", ["serve", "batch"])
+def test_several_runs_in_the_ladder_form_equal_the_fused_form(tb, gpu, monkeypatch, how, form, threads, polls):
+    kinds = ["qubo:61", "pm2:12", "gauss3:6", "qubo:300", "rrg:130", "gauss2:9", "pm2:16", "qubo:700", "site:1",
+             "pm3:6", "rrg:40", "gauss2:17"]
+    if how == "batch":
+        kinds = kinds[:4]
+    hosts = [_host(tb, k) for k in kinds]
+    params = [tb.PtParams(70, tb.geometric_betas(0.2, 5.0, 12 + k), 5, 0.5, True, 2, 8, None, None, 0)
+              for k in range(len(kinds))]
+
+    def run():
+        if how == "serve":
+            srv = tb.Server(gpu, 8 << 30, 64, 25)
+            ids = [srv.submit(h, p, 3 + k) for k, (h, p) in enumerate(zip(hosts, params))]
+            while any(srv.step()):
+                pass
+            return [x for i in ids for x in (*srv.state(i), np.float32(srv.result(i)[1]), np.uint32(srv.result(i)[2]))]
+        b = tb.Batch(gpu)
+        for k, (d, p) in enumerate(zip(gpu.upload_many(hosts), params)):
+            b.add(d, p, 3 + k)
+        b.run()
+        logs = b.gs_all()
+        return [x for k in range(len(kinds)) for x in (*b.state(k), b.acceptance(k), *b.round_trips(k), *logs[k])]
+
+    monkeypatch.setenv("TAMC_PT_FORM", "fused")
+    want = run()
+    monkeypatch.setenv("TAMC_PT_FORM", form)
+    if threads:
+        monkeypatch.setenv("TAMC_PT_T", threads)
+    if polls:
+        monkeypatch.setenv("TAMC_LADDER_POLLS", polls)
+    _same(want, run())
