@@ -12,13 +12,77 @@
 #include "fast_sa.cuh"
 
 #include <cstdio>
+#include <cstring>
 #include <map>
 #include <mutex>
 #include <tuple>
+#include <type_traits>
 
 namespace tamc {
 
 namespace {
+
+// The end of an anneal: energy_ref of every replica of the CTA (f32 row terms
+// accumulated in fixed point) and the states in original site order, from the
+// words W (bits 0 .. 4 NQ - 1); `red`: (T / 32) * 4 NQ sums.
+template <int NQ>
+__device__ void sa_finish(const SaFastArgs& a, const FastInst& F, const uint32_t* W, long long* red, uint32_t r0) {
+  constexpr uint32_t G = 4 * NQ;
+  const uint32_t T = blockDim.x, tid = threadIdx.x, n = a.F.n;
+  const uint32_t shift = 4 * (tid % NQ), stride = T / NQ;
+  long long e0 = 0, e1 = 0, e2 = 0, e3 = 0;
+  for (uint32_t s = tid / NQ; s < n; s += stride) {
+    const float4 t = energy_terms4(s, shift, F, W, 1, 0);
+    e0 += to_fx(t.x);
+    e1 += to_fx(t.y);
+    e2 += to_fx(t.z);
+    e3 += to_fx(t.w);
+  }
+#pragma unroll
+  for (uint32_t off = 16; off >= NQ; off >>= 1) {
+    e0 += __shfl_xor_sync(0xffffffffu, e0, off);
+    e1 += __shfl_xor_sync(0xffffffffu, e1, off);
+    e2 += __shfl_xor_sync(0xffffffffu, e2, off);
+    e3 += __shfl_xor_sync(0xffffffffu, e3, off);
+  }
+  const uint32_t lane = tid & 31u, warp = tid >> 5, nw = T >> 5;
+  if (lane < NQ) {
+    red[(warp * NQ + lane) * 4 + 0] = e0;
+    red[(warp * NQ + lane) * 4 + 1] = e1;
+    red[(warp * NQ + lane) * 4 + 2] = e2;
+    red[(warp * NQ + lane) * 4 + 3] = e3;
+  }
+  __syncthreads();
+  if (tid < G) {
+    long long E = 0;
+    for (uint32_t w = 0; w < nw; ++w) E += red[(w * NQ + tid / 4) * 4 + (tid & 3u)];
+    const uint32_t r = r0 + tid;
+    if (r < a.R) a.energies_out[r] = (float)((double)a.F.offset + (double)E * TAMC_FX_INV);
+  }
+  const uint32_t keep = (a.R - r0 >= 32u) ? 0xffffffffu : ((1u << (a.R - r0)) - 1u);
+  for (uint32_t s = tid; s < n; s += T) {
+    const uint32_t v = (W[s] & (G < 32 ? ((1u << G) - 1u) : 0xffffffffu) & keep) << (r0 & 31u);
+    uint32_t* dst = a.words_out + (size_t)(r0 >> 5) * n + a.F.perm[s];
+    if (G == 32) *dst = v;
+    else atomicOr(dst, v);
+  }
+}
+
+// The initial word of site s (bits 0 .. 4 NQ - 1).
+template <int NQ>
+__device__ __forceinline__ uint32_t sa_init_word(const SaFastArgs& a, uint32_t s, uint32_t r0) {
+  constexpr uint32_t G = 4 * NQ;
+  uint32_t w = 0;
+  if (a.init_words) {
+    w = a.init_words[(size_t)(r0 >> 5) * a.F.n + a.F.perm[s]] >> (r0 & 31u);
+    if (G < 32) w &= (1u << G) - 1u;
+  } else {
+#pragma unroll
+    for (uint32_t q = 0; q < NQ; ++q)
+      w |= init_nibble(philox4x32_10(make_uint4(s, 0xffffffffu, (r0 >> 2) + q, PTAG_INIT), a.key)) << (4 * q);
+  }
+  return w;
+}
 
 template <int NQ, bool SMEM, uint32_t DEG>
 __global__ void __launch_bounds__(1024) k_sa_fast(SaFastArgs a) {
@@ -77,7 +141,8 @@ __global__ void __launch_bounds__(1024) k_sa_fast(SaFastArgs a) {
       __syncthreads();
     }
   }
-  // energy_ref of every replica: f32 row terms accumulated in fixed point
+  // as sa_finish; in a function of its own it cost the sweeps' code 4 % (1728 sites
+  // with 6 entries, 256 restarts, 200 sweeps: 548 us, 580 with the call)
   long long e0 = 0, e1 = 0, e2 = 0, e3 = 0;
   for (uint32_t s = tid / NQ; s < n; s += stride) {
     const float4 t = energy_terms4(s, shift, F, W, 1, 0);
@@ -119,6 +184,247 @@ __global__ void __launch_bounds__(1024) k_sa_fast(SaFastArgs a) {
   }
 }
 
+// ---- rows of 3 or 4 entries on small instances: the local field from a table
+// A site's field takes 2^DEG values, one per combination of its neighbours'
+// spins; with its own spin in the index the table holds s f, the number the
+// acceptance wants, for 2^(DEG+1) combinations: the same float sums as
+// local_field4_deg, made once.  A replica then costs one lookup instead of a
+// shift, an XOR and an add per neighbour.  A site's four spins of a quad are the
+// bytes of one word (0 or 1), so the neighbours' words added with weights 1, 2,
+// 4, ... give the four indices at once, and a word belongs to one thread (no
+// atomics).  Columns of the table run over the sites: lanes on consecutive
+// sites hit different banks whatever their indices.
+// Of Philox's ten rounds, what depends on the site alone (the first product and
+// the second's) is kept per site, what depends on the sweep alone is computed
+// once per sweep: 16 wide products a call instead of 20.
+// Bound: issue.  (2000 sites of 3 entries, 1024 restarts, 1000 sweeps: 3.87 ms
+// with k_sa_fast, 3.29 so; 1600 sites of 4, 300 restarts, 300 sweeps: 792 us, 530.)
+struct SaTab {
+  uint32_t W, cols, pre, tab, red, bytes;  // byte offsets
+};
+__host__ __device__ inline SaTab sa_tab_carve(uint32_t n, uint32_t nq, uint32_t deg, bool half, uint32_t T) {
+  const uint32_t np = (n + 31) / 32 * 32;
+  SaTab S;
+  S.W = 0;                            // [nq][np] spins, a byte per replica of the quad
+  S.cols = nq * np * 4;               // [np] uint2: byte offsets of the neighbours' words, 16 bits each
+  S.pre = S.cols + np * 8;            // [3][np] Philox products of the site
+  S.tab = S.pre + np * 12;            // [2^(deg+1)][np] s f (half: [2^deg][np] f); at the end the replica words [n] and `red`
+  const uint32_t tab = (1u << (deg + !half)) * np * 4;
+  S.red = S.tab + np * 4;
+  const uint32_t fin = np * 4 + (T / 32) * nq * 32;
+  S.bytes = S.tab + (tab > fin ? tab : fin);
+  return S;
+}
+template <int NQ, uint32_t DEG, bool HALF>
+__global__ void __launch_bounds__(1024) k_sa_tab(SaFastArgs a) {
+  extern __shared__ __align__(16) unsigned char sa_smem[];
+  const uint32_t T = blockDim.x, tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+  const uint32_t n = a.F.n, np = (n + 31) / 32 * 32;
+  const SaTab S = sa_tab_carve(n, NQ, DEG, HALF, T);
+  uint32_t* const pre = reinterpret_cast<uint32_t*>(sa_smem + S.pre);
+  uint2* const cols = reinterpret_cast<uint2*>(sa_smem + S.cols);
+  const uint32_t r0 = blockIdx.x * 4 * NQ;
+  const PhiloxKeys K = philox_schedule(a.key);
+  for (uint32_t s = tid; s < n; s += T) {
+    float J[DEG];
+    uint32_t c[4] = {0, 0, 0, 0};
+#pragma unroll
+    for (uint32_t m = 0; m < DEG; ++m) {
+      const uint2 v = a.F.ent[s * DEG + m];
+      c[m] = 4 * v.x;
+      J[m] = __uint_as_float(v.y);
+    }
+    cols[s] = make_uint2(c[0] | (c[1] << 16), c[2] | (c[3] << 16));
+    float* tab = reinterpret_cast<float*>(sa_smem + S.tab) + s;
+    for (uint32_t x = 0; x < (1u << (DEG + !HALF)); ++x) {
+      float f = a.F.bias[s];
+#pragma unroll
+      for (uint32_t m = 0; m < DEG; ++m) f += __uint_as_float(__float_as_uint(J[m]) ^ ((x >> m) << 31));
+      tab[x * np] = __uint_as_float(__float_as_uint(f) ^ ((x >> DEG) << 31));  // (HALF: x >> DEG is 0)
+    }
+    const uint64_t p0 = (uint64_t)0xD2511F53u * s;
+    const uint64_t p1 = (uint64_t)0xCD9E8D57u * ((uint32_t)(p0 >> 32) ^ PTAG_SWEEP ^ K.y[0]);
+    pre[s] = (uint32_t)p0;
+    pre[np + s] = (uint32_t)(p1 >> 32);
+    pre[2 * np + s] = (uint32_t)p1;
+    const uint32_t w = sa_init_word<NQ>(a, s, r0);
+#pragma unroll
+    for (uint32_t q = 0; q < NQ; ++q)  // bit r of the quad to byte r
+      reinterpret_cast<uint32_t*>(sa_smem)[q * np + s] = (((w >> (4 * q)) & 15u) * 0x00204081u) & 0x01010101u;
+  }
+  __syncthreads();
+  const uint32_t q = warp % NQ, qid = (r0 >> 2) + q;
+  unsigned char* const Wq = sa_smem + q * np * 4;
+  const unsigned char* const tab = sa_smem + S.tab;
+  const uint32_t first = warp / NQ * 32 + lane, stride = T / NQ;
+  const uint64_t pq = (uint64_t)0xCD9E8D57u * qid;
+  const uint32_t kz = (uint32_t)pq ^ K.x[1];  // joins the site's part in round 2
+  for (uint32_t sw = 0; sw < a.nbeta; ++sw) {
+    const float b2 = a.betas[sw] * TAMC_2LOG2E;  // 2 beta log2(e)
+    const uint64_t ps = (uint64_t)0xD2511F53u * ((uint32_t)(pq >> 32) ^ sw ^ K.x[0]);
+    const uint32_t sz = (uint32_t)(ps >> 32) ^ K.y[1];
+    for (uint32_t c = 0; c < a.F.ncolors; ++c) {
+      const uint32_t c1 = a.F.color_off[c + 1];
+      for (uint32_t s = a.F.color_off[c] + first; s < c1; s += stride) {
+        const uint2 cc = cols[s];
+        uint32_t* const Ws = reinterpret_cast<uint32_t*>(Wq + 4 * s);
+        uint32_t own = *Ws;
+        uint32_t x = *reinterpret_cast<const uint32_t*>(Wq + (cc.x & 0xffffu)) +
+                     2 * *reinterpret_cast<const uint32_t*>(Wq + (cc.x >> 16)) +
+                     4 * *reinterpret_cast<const uint32_t*>(Wq + (cc.y & 0xffffu)) + (HALF ? 0u : own << DEG);
+        if (DEG == 4) x += 8 * *reinterpret_cast<const uint32_t*>(Wq + (cc.y >> 16));
+        uint4 r = make_uint4(pre[np + s] ^ kz, pre[2 * np + s], pre[s] ^ sz, (uint32_t)ps);
+#pragma unroll
+        for (int k = 2; k < 10; ++k) {
+          const uint64_t p0 = (uint64_t)0xD2511F53u * r.x, p1 = (uint64_t)0xCD9E8D57u * r.z;
+          r = make_uint4((uint32_t)(p1 >> 32) ^ r.y ^ K.x[k], (uint32_t)p1, (uint32_t)(p0 >> 32) ^ r.w ^ K.y[k],
+                         (uint32_t)p0);
+        }
+        const unsigned char* const row = tab + 4 * s;
+        auto step = [&](uint32_t k, uint32_t rnd) {  // accept_g of replica k
+          float g = *reinterpret_cast<const float*>(row + ((x >> (8 * k)) & 0xffu) * (4 * np));
+          if (HALF) g = __uint_as_float(__float_as_uint(g) ^ ((own << (31 - 8 * k)) & 0x80000000u));
+          const float p1 = ex2_approx(b2 * g) + 1.0f;
+          if (__uint_as_float(__funnelshift_r(rnd, 0x7fu, 9)) < p1) own ^= 1u << (8 * k);  // 0x3f800000 | rnd >> 9
+        };
+        step(0, r.x);
+        step(1, r.y);
+        step(2, r.z);
+        step(3, r.w);
+        *Ws = own;
+      }
+      __syncthreads();
+    }
+  }
+  // bytes back to bits, in place of the table
+  uint32_t* const W = reinterpret_cast<uint32_t*>(sa_smem + S.tab);
+  for (uint32_t s = tid; s < n; s += T) {
+    uint32_t w = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < NQ; ++k) {
+      const uint32_t v = reinterpret_cast<const uint32_t*>(sa_smem)[k * np + s];
+      w |= ((v | (v >> 7) | (v >> 14) | (v >> 21)) & 15u) << (4 * k);
+    }
+    W[s] = w;
+  }
+  __syncthreads();
+  sa_finish<NQ>(a, a.F, W, reinterpret_cast<long long*>(sa_smem + S.red), r0);
+}
+
+// ---- rows of uneven length, as slices of 32 sites (FastInst::sl_*): a warp per
+// (slice, quad), a lane per site.  The lanes' rows have about the same length and
+// read consecutive entries, and up to eight entries' loads are ahead of their
+// sums.  With CS the rows are in shared memory (16-bit byte offsets of the
+// words, couplings), else in L2.
+// Bound: the serial chain of loads and sums of a row.  (With k_sa_fast, whose
+// warps wait for their longest row, and here: 251 sites, 100 restarts, 200
+// sweeps 1586 us and 855; 8192 sites, 512 restarts, 100 sweeps 3282 us and 2197.)
+struct SaSl {
+  uint32_t W, site, soff, bias, colp, J, red, bytes;
+};
+__host__ __device__ inline SaSl sa_sl_carve(const FastInst& F, bool cs, uint32_t nq, uint32_t T) {
+  uint32_t o = 0;
+  auto take = [&](uint32_t b) {
+    const uint32_t p = o;
+    o = (o + b + 15u) & ~15u;
+    return p;
+  };
+  SaSl S{};
+  S.W = take(F.n * 4);
+  S.site = take(F.sl_n * 64);
+  S.soff = take((F.sl_n + 1) * 4);
+  S.bias = take(F.n * 4);
+  if (cs) {
+    S.colp = take(F.sl_rows * 64);
+    S.J = take(F.sl_rows * 128);
+  }
+  S.red = take((T / 32) * nq * 32);
+  S.bytes = o;
+  return S;
+}
+template <int NQ, bool CS>
+__global__ void __launch_bounds__(1024) k_sa_sl(SaFastArgs a) {
+  extern __shared__ __align__(16) unsigned char sa_smem[];
+  const uint32_t T = blockDim.x, tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+  const uint32_t n = a.F.n;
+  const SaSl S = sa_sl_carve(a.F, CS, NQ, T);
+  uint32_t* const W = reinterpret_cast<uint32_t*>(sa_smem);
+  uint16_t* const site = reinterpret_cast<uint16_t*>(sa_smem + S.site);
+  uint32_t* const soff = reinterpret_cast<uint32_t*>(sa_smem + S.soff);
+  float* const bias = reinterpret_cast<float*>(sa_smem + S.bias);
+  uint16_t* const colp = reinterpret_cast<uint16_t*>(sa_smem + S.colp);
+  float* const Js = reinterpret_cast<float*>(sa_smem + S.J);
+  const uint2* __restrict__ const ent = a.F.sl_ent;
+  const uint32_t r0 = blockIdx.x * 4 * NQ;
+  for (uint32_t x = tid; x < 32 * a.F.sl_n; x += T) site[x] = a.F.sl_site[x];
+  for (uint32_t x = tid; x <= a.F.sl_n; x += T) soff[x] = a.F.sl_off[x];
+  if (CS)
+    for (uint32_t x = tid; x < 32 * a.F.sl_rows; x += T) {
+      const uint2 v = ent[x];
+      colp[x] = (uint16_t)v.x;
+      Js[x] = __uint_as_float(v.y);
+    }
+  for (uint32_t s = tid; s < n; s += T) {
+    bias[s] = a.F.bias[s];
+    W[s] = sa_init_word<NQ>(a, s, r0);
+  }
+  __syncthreads();
+  const uint32_t q = warp % NQ, shift = 4 * q, qid = (r0 >> 2) + q;
+  const uint32_t first = warp / NQ, stride = (T >> 5) / NQ;
+  const PhiloxKeys K = philox_schedule(a.key);
+  Fx4 acc{0, 0, 0, 0};  // unused: SA energies are computed once at the end
+  for (uint32_t sw = 0; sw < a.nbeta; ++sw) {
+    const float b = a.betas[sw] * TAMC_2LOG2E;  // 2 beta log2(e)
+    const float4 b2 = make_float4(b, b, b, b);
+    for (uint32_t c = 0; c < a.F.ncolors; ++c) {
+      const uint32_t g1 = a.F.sl_cls[c + 1];
+      for (uint32_t g = a.F.sl_cls[c] + first; g < g1; g += stride) {
+        const uint32_t s = site[32 * g + lane];
+        if (s == 0xffffu) continue;  // beyond the class's last site
+        uint32_t x = soff[g], w = soff[g + 1] - x;
+        x = 32 * x + lane;
+        const float h = bias[s];
+        float4 f = make_float4(h, h, h, h);
+        auto entries = [&](auto count) {
+          constexpr uint32_t N = decltype(count)::value;
+          uint32_t c4[N], j[N], v[N];
+#pragma unroll
+          for (uint32_t m = 0; m < N; ++m) {
+            if (CS) {
+              c4[m] = colp[x + 32 * m];
+              j[m] = __float_as_uint(Js[x + 32 * m]);
+            } else {
+              const uint2 e = __ldg(ent + x + 32 * m);
+              c4[m] = e.x;
+              j[m] = e.y;
+            }
+          }
+#pragma unroll
+          for (uint32_t m = 0; m < N; ++m) v[m] = *reinterpret_cast<const uint32_t*>(sa_smem + c4[m]) >> shift;
+#pragma unroll
+          for (uint32_t m = 0; m < N; ++m) {
+            f.x += __uint_as_float(j[m] ^ (v[m] << 31));
+            f.y += __uint_as_float(j[m] ^ ((v[m] << 30) & 0x80000000u));
+            f.z += __uint_as_float(j[m] ^ ((v[m] << 29) & 0x80000000u));
+            f.w += __uint_as_float(j[m] ^ ((v[m] << 28) & 0x80000000u));
+          }
+          x += 32 * N;
+        };
+#pragma unroll 1
+        for (; w >= 8; w -= 8) entries(std::integral_constant<uint32_t, 8>());
+        if (w & 4u) entries(std::integral_constant<uint32_t, 4>());
+        if (w & 2u) entries(std::integral_constant<uint32_t, 2>());
+        const uint4 rnd = philox4x32_10(make_uint4(s, sw, qid, PTAG_SWEEP), K);
+        const uint32_t m = quad_accept<false>(f, W[s] >> shift, b2, rnd, acc);
+        if (NQ == 1) W[s] ^= m;
+        else if (m) atomicXor(&W[s], m << shift);
+      }
+      __syncthreads();
+    }
+  }
+  sa_finish<NQ>(a, a.F, W, reinterpret_cast<long long*>(sa_smem + S.red), r0);
+}
+
 // words [ceil(R/32)][n] (bit r%32 = replica r) -> packed [R][ceil(n/8)] bytes
 // (bit i%8 of byte i/8 = site i), the IsingState::write_to_bytes layout
 // (src/ising.rs:102-115).  One thread per output byte.
@@ -133,12 +439,16 @@ __global__ void k_pack_states(const uint32_t* __restrict__ words, uint32_t n, ui
   out[x] = (uint8_t)v;
 }
 
-template <int NQ, bool SMEM, uint32_t DEG>
-void launch_d(cudaStream_t st, const SaFastArgs& a, uint32_t ncta, uint32_t T, size_t smem) {
-  auto k = k_sa_fast<NQ, SMEM, DEG>;
+template <class K>
+void launch_k(K k, cudaStream_t st, const SaFastArgs& a, uint32_t ncta, uint32_t T, size_t smem) {
   TAMC_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   k<<<ncta, T, smem, st>>>(a);
   TAMC_CUDA(cudaGetLastError());
+}
+
+template <int NQ, bool SMEM, uint32_t DEG>
+void launch_d(cudaStream_t st, const SaFastArgs& a, uint32_t ncta, uint32_t T, size_t smem) {
+  launch_k(k_sa_fast<NQ, SMEM, DEG>, st, a, ncta, T, smem);
 }
 
 // rows of uniform length 3, 4 or 6 (random regular graphs, square and cubic
@@ -167,11 +477,87 @@ void sa_pack_states(cudaStream_t st, const uint32_t* words, uint32_t n, uint32_t
   TAMC_CUDA(cudaGetLastError());
 }
 
-// Heuristic tile: 256 threads and the smallest replica group (quads per CTA)
-// that gives no SM more than two CTAs.  (On 1024 restarts of a 2000-spin
-// instance: 256 CTAs of 4 restarts, measured fastest of the 12 tiles.)
-static SaTile heuristic(const tamc_gpu* g, const FastInst& F, uint32_t R) {
+// Shared memory of a tile's kernel (SIZE_MAX where it does not take the instance).
+static size_t sa_tile_smem(const FastInst& F, const SaTile& t) {
+  if (t.kind == SA_TABLE) {
+    if ((F.udeg != 3 && F.udeg != 4) || F.n > 16383) return SIZE_MAX;  // 16-bit byte offsets
+    return sa_tab_carve(F.n, t.nq, F.udeg, t.smem_csr, t.T).bytes;
+  }
+  if (t.kind == SA_SLICED) {
+    if (!F.sl_ent || (t.smem_csr && F.n > 16383) || (uint64_t)F.sl_rows * 192 > (8u << 20)) return SIZE_MAX;
+    return sa_sl_carve(F, t.smem_csr, t.nq, t.T).bytes;
+  }
+  return sa_fast_smem(F, t.nq, t.T, t.smem_csr);
+}
+
+// The tile of the table or sliced kernel (kind set, and smem_csr where there is
+// a choice): of the replica groups that leave the busiest SM the fewest quads,
+// the largest one that a CTA can give a warp per 32 sites of a class, else the
+// smallest; a warp per (32 sites, quad) of the largest class, as far as all of an
+// SM's CTAs stay resident at 64 registers.  Measured against all groups of 4, 8
+// and 16 restarts and CTAs of 64 to 1024 threads on 64 and 300 sweeps: 3-regular
+// 300, 1000 and 2000 sites, 2-D lattices of 15, 16 and 40, QUBOs of 64 to 8192
+// sites, 64 to 2048 restarts; within 3 % of the best but for 64 sites x 2048
+// (274 us against 256).
+static bool sa_rule(const tamc_gpu* g, const FastInst& F, uint32_t R, uint32_t largest_class, SaTile& t) {
+  const uint32_t Q = (R + 3) / 4, sms = (uint32_t)g->num_sms, per = (largest_class + 31) / 32 * 32;
+  auto busiest = [&](uint32_t nq) { return nq * (((Q + nq - 1) / nq + sms - 1) / sms); };
+  const uint32_t least = std::min({busiest(1), busiest(2), busiest(4)});
+  t.nq = 1;
+  t.T = std::min(per, 1024u);
+  const size_t one = sa_tile_smem(F, t);
+  const bool ones = busiest(1) == least && one <= g->smem_optin && busiest(1) <= g->smem_optin / one;
+  for (uint32_t nq : {4u, 2u, 1u}) {
+    // (groups of 4 restarts whose CTAs of an SM run side by side need no sharing)
+    if (busiest(nq) != least || (nq > 1 && nq * per > 1024 && ones)) continue;
+    t.nq = nq;
+    t.T = 1024;
+    const size_t most = sa_tile_smem(F, t);
+    if (most > g->smem_optin) continue;
+    // CTAs of the busiest SM that are there at once
+    const uint32_t ctas = (uint32_t)std::min<size_t>({busiest(nq) / nq, g->smem_optin / most, 8});
+    const uint32_t room = 1024u / std::max(ctas, 1u);
+    t.T = std::max(nq * per, 32 * nq);
+    // several sites a warp in turn, in equal numbers
+    for (uint32_t k = 2; t.T > room && t.T > 32 * nq; ++k) t.T = nq * ((per / 32 + k - 1) / k) * 32;
+    t.smem = sa_tile_smem(F, t);
+    if (t.smem <= g->smem_optin) return true;
+  }
+  return false;
+}
+
+// Heuristic tile.  Rows of 3 or 4 entries take the table kernel where its table
+// fits (the one with the site's own spin in it first), rows of uneven length the
+// sliced one.  3-regular instances stay with the words where SMs have few warps
+// of work, whose latency the table does not shorten (300 sites, 100 restarts:
+// 393 us against 407), and above 2600 sites, where only the smaller table fits
+// (2700 sites, 800 restarts: 1141 us against 1359).  For the words: 256
+// threads and the smallest replica group (quads per CTA) that gives no SM more
+// than two CTAs.
+static SaTile heuristic(const tamc_gpu* g, const FastInst& F, uint32_t R, uint32_t largest_class) {
   SaTile t;
+  const uint32_t Q = (R + 3) / 4, sms = (uint32_t)g->num_sms;
+  const uint32_t warps = (Q + sms - 1) / sms * ((largest_class + 31) / 32);  // of 32 sites x a quad, busiest SM
+  const char* env = getenv("TAMC_SA_KERNEL");  // "words": k_sa_fast whatever the rows (tests, profiling)
+  const bool words = env && !strcmp(env, "words");
+  if (!words && (F.udeg == 4 || (F.udeg == 3 && warps >= 10))) {
+    t.kind = SA_TABLE;
+    for (bool half : {false, true}) {
+      t.smem_csr = half;
+      if (!(half && F.udeg == 3) && sa_rule(g, F, R, largest_class, t)) return t;
+    }
+  } else if (!words && F.sl_ent) {
+    t.kind = SA_SLICED;
+    for (bool rows : {true, false}) {
+      t.smem_csr = rows;
+      // (in shared memory only if the SM's CTAs still fit side by side)
+      if (sa_rule(g, F, R, largest_class, t) &&
+          (!rows || t.smem * std::min<size_t>(((R + 4 * t.nq - 1) / (4 * t.nq) + g->num_sms - 1) / g->num_sms, 4) <=
+                        g->smem_optin))
+        return t;
+    }
+  }
+  t = SaTile();
   t.T = 256;
   t.smem_csr = sa_fast_smem(F, 8, 1024, true) <= g->smem_optin;
   t.nq = 8;
@@ -179,11 +565,11 @@ static SaTile heuristic(const tamc_gpu* g, const FastInst& F, uint32_t R) {
     const uint32_t ncta = (R + 4 * nq - 1) / (4 * nq);
     if (ncta <= 2u * (uint32_t)g->num_sms) { t.nq = nq; break; }
   }
-  t.smem = sa_fast_smem(F, t.nq, t.T, t.smem_csr);
+  t.smem = sa_tile_smem(F, t);
   return t;
 }
 
-// Autotuner: times a short anneal (a few sweeps) of each candidate tile --
+// Autotuner (k_sa_fast): times a short anneal (a few sweeps) of each candidate tile --
 // replicas per CTA (4*nq) x CTA size -- on scratch buffers the first time a
 // (device, n, nnz, R) shape is seen, and caches the fastest.  The choice does
 // not change results: spins depend only on (seed, site, sweep, replica) and
@@ -191,16 +577,16 @@ static SaTile heuristic(const tamc_gpu* g, const FastInst& F, uint32_t R) {
 static std::mutex g_sa_mu;
 static std::map<std::tuple<int, uint32_t, uint32_t, uint32_t>, SaTile> g_sa_tune;
 
-SaTile sa_fast_choose(tamc_gpu* g, const FastInst& F, uint32_t R) {
+SaTile sa_fast_choose(tamc_gpu* g, const FastInst& F, uint32_t R, uint32_t largest_class) {
+  SaTile best = heuristic(g, F, R, largest_class);
   const auto key = std::make_tuple(g->device, F.n, F.nnz, R);
-  {
+  if (best.kind == SA_WORDS) {
     std::lock_guard<std::mutex> lk(g_sa_mu);
     auto it = g_sa_tune.find(key);
     if (it != g_sa_tune.end()) return it->second;
   }
-  SaTile best = heuristic(g, F, R);
   const char* env = getenv("TAMC_AUTOTUNE");
-  if ((!env || env[0] != '0') && R >= 64) {
+  if (best.kind == SA_WORDS && (!env || env[0] != '0') && R >= 64) {
     // long enough that the per-sweep cost, not the start-up, decides
     const uint32_t nb = 64;
     float* d_b = nullptr;
@@ -222,7 +608,7 @@ SaTile sa_fast_choose(tamc_gpu* g, const FastInst& F, uint32_t R) {
         t.nq = nq;
         t.T = T;
         t.smem_csr = best.smem_csr;
-        t.smem = sa_fast_smem(F, nq, T, t.smem_csr);
+        t.smem = sa_tile_smem(F, t);
         if (t.smem > g->smem_optin) continue;
         const uint32_t ncta = (R + 4 * nq - 1) / (4 * nq);
         if (ncta * 4 < (uint32_t)g->num_sms && nq > 1) continue;  // too few CTAs to fill the GPU
@@ -261,19 +647,22 @@ SaTile sa_fast_choose(tamc_gpu* g, const FastInst& F, uint32_t R) {
   }
   if (const char* e = getenv("TAMC_SA_NQ")) {  // manual override (profiling)
     const int v = atoi(e);
-    if (v == 1 || v == 2 || v == 4 || v == 8) best.nq = (uint32_t)v;
+    if (v == 1 || v == 2 || v == 4 || (v == 8 && best.kind == SA_WORDS)) best.nq = (uint32_t)v;
   }
   if (const char* e = getenv("TAMC_SA_T")) {
     const int v = atoi(e);
     if (v == 128 || v == 256 || v == 512 || v == 1024) best.T = (uint32_t)v;
   }
-  best.smem = sa_fast_smem(F, best.nq, best.T, best.smem_csr);
+  if (best.kind != SA_WORDS) best.T = std::max(best.T / (32 * best.nq), 1u) * 32 * best.nq;
+  best.smem = sa_tile_smem(F, best);
   if (best.smem > g->smem_optin) fail(TAMC_E_UNSUPPORTED, "instance too large for the fast SA kernel");
   if (getenv("TAMC_DEBUG"))
-    fprintf(stderr, "[tamc] SA tile n=%u R=%u: replicas/CTA=%u threads=%u csr_smem=%d smem=%zu\n", F.n, R,
+    fprintf(stderr, "[tamc] SA tile n=%u R=%u: kernel %d replicas/CTA=%u threads=%u csr_smem=%d smem=%zu\n", F.n, R, best.kind,
             4 * best.nq, best.T, (int)best.smem_csr, best.smem);
-  std::lock_guard<std::mutex> lk(g_sa_mu);
-  g_sa_tune[key] = best;
+  if (best.kind == SA_WORDS) {
+    std::lock_guard<std::mutex> lk(g_sa_mu);
+    g_sa_tune[key] = best;
+  }
   return best;
 }
 
@@ -281,6 +670,32 @@ void sa_fast_launch(cudaStream_t st, const SaFastArgs& a, const SaTile& t) {
   const uint32_t G = 4 * t.nq;
   const uint32_t ncta = (a.R + G - 1) / G;
   if (!ncta) return;
+  if (t.kind == SA_TABLE) {
+    auto go = [&](auto deg, auto half) {
+      constexpr uint32_t D = decltype(deg)::value;
+      constexpr bool H = decltype(half)::value;
+      if (t.nq == 1) launch_k(k_sa_tab<1, D, H>, st, a, ncta, t.T, t.smem);
+      else if (t.nq == 2) launch_k(k_sa_tab<2, D, H>, st, a, ncta, t.T, t.smem);
+      else launch_k(k_sa_tab<4, D, H>, st, a, ncta, t.T, t.smem);
+    };
+    using D3 = std::integral_constant<uint32_t, 3>;
+    using D4 = std::integral_constant<uint32_t, 4>;
+    if (a.F.udeg == 3) go(D3(), std::false_type());
+    else t.smem_csr ? go(D4(), std::true_type()) : go(D4(), std::false_type());
+    return;
+  }
+  if (t.kind == SA_SLICED) {
+    switch (t.nq * 2 + (t.smem_csr ? 1 : 0)) {
+      case 2: launch_k(k_sa_sl<1, false>, st, a, ncta, t.T, t.smem); break;
+      case 3: launch_k(k_sa_sl<1, true>, st, a, ncta, t.T, t.smem); break;
+      case 4: launch_k(k_sa_sl<2, false>, st, a, ncta, t.T, t.smem); break;
+      case 5: launch_k(k_sa_sl<2, true>, st, a, ncta, t.T, t.smem); break;
+      case 8: launch_k(k_sa_sl<4, false>, st, a, ncta, t.T, t.smem); break;
+      case 9: launch_k(k_sa_sl<4, true>, st, a, ncta, t.T, t.smem); break;
+      default: fail(TAMC_E_INVAL, "bad SA tile");
+    }
+    return;
+  }
   switch (t.nq * 2 + (t.smem_csr ? 1 : 0)) {
     case 2: launch_t<1, false>(st, a, ncta, t.T, t.smem); break;
     case 3: launch_t<1, true>(st, a, ncta, t.T, t.smem); break;
@@ -294,13 +709,14 @@ void sa_fast_launch(cudaStream_t st, const SaFastArgs& a, const SaTile& t) {
   }
 }
 
-SaTile sa_fast_peek(const tamc_gpu* g, const FastInst& F, uint32_t R) {
-  {
+SaTile sa_fast_peek(const tamc_gpu* g, const FastInst& F, uint32_t R, uint32_t largest_class) {
+  const SaTile t = heuristic(g, F, R, largest_class);
+  if (t.kind == SA_WORDS) {
     std::lock_guard<std::mutex> lk(g_sa_mu);
     auto it = g_sa_tune.find(std::make_tuple(g->device, F.n, F.nnz, R));
     if (it != g_sa_tune.end()) return it->second;
   }
-  return heuristic(g, F, R);
+  return t;
 }
 
 }  // namespace tamc
