@@ -145,6 +145,23 @@ uint32_t lattice_side(const HostInstance& h, uint32_t udeg) {
   }
   return L;
 }
+
+// FastInst::cb_L of a +-J square lattice of side L (lattice_side), from its
+// colour order and its colour-ordered rows.
+uint32_t checkerboard_side(uint32_t L, const std::vector<uint32_t>& perm, const std::vector<uint2>& ent) {
+  if (L < 4 || L % 2) return 0;
+  const uint32_t n = L * L;
+  for (uint32_t s = 0; s < n; ++s) {
+    const uint32_t f = perm[s];
+    if (s != ((f / L + f % L) & 1u) * (n / 2) + f / 2) return 0;
+    for (uint32_t e = 4 * s; e < 4 * s + 4; ++e) {
+      const uint2* back = &ent[4 * (size_t)ent[e].x];
+      for (uint32_t k = 0; k < 4; ++k)
+        if (back[k].x == s && back[k].y != ent[e].y) return 0;
+    }
+  }
+  return L;
+}
 }  // namespace
 
 void* dev_alloc(size_t bytes) {
@@ -378,6 +395,7 @@ static void inst_prepare(tamc_inst* d, const HostInstance& h, UploadPack& pack) 
   for (size_t e = 0; e < fent.size() && d->pmj; ++e)
     if ((fent[e].y & 0x7fffffffu) != 0x3f800000u) d->pmj = 0;  // |J| == 1.0f
   d->lat_any = lattice_side(h, d->udeg);
+  if (d->pmj && d->udeg == 4) d->cb_L = checkerboard_side(d->lat_any, d->h_perm, fent);
   d->lat_L = d->lat_any == 16 || d->lat_any == 32 ? d->lat_any : 0;
   std::vector<float> fJt;
   std::vector<uint16_t> fcolt;

@@ -289,6 +289,7 @@ struct tamc_inst {
   int pmj = 0;                       // +-1 couplings, no field, no self-loop, rows of 4 or 6 entries
   uint32_t lat_L = 0;                // periodic L^d lattice in file order (L 16 or 32, d = udeg / 2), else 0
   uint32_t lat_any = 0;              // the same for any side from 3 to 32
+  uint32_t cb_L = 0;                 // side of a +-J square lattice in checkerboard colour order, else 0
   uint32_t sl_n = 0, sl_rows = 0;    // sliced rows (FastInst::sl_*)
   uint32_t *d_sl_cls = nullptr, *d_sl_off = nullptr;
   uint16_t *d_sl_site = nullptr, *d_sl_pos = nullptr;

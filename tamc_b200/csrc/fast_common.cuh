@@ -25,6 +25,10 @@ struct FastInst {  // colour-ordered instance (device pointers)
   int pmj;                    // +-1 couplings, zero field, no self-loop, udeg 4 or 6 (multi-spin coding)
   uint32_t lat_L;             // side of a periodic square / cubic lattice in file order (16 or 32), else 0
   uint32_t lat_any;           // side of such a lattice of any side from 3 to 32, else 0
+  // side (even, 4 to 32) of a +-J square lattice with symmetric couplings whose
+  // colour order is the checkerboard's: file site f at row r, column x is colour
+  // site ((r + x) & 1) n / 2 + f / 2; else 0
+  uint32_t cb_L;
   // sliced rows (instances whose rows are not all of 3, 4 or 6 entries without
   // self-couplings, n <= 65535): each colour class sorted by row length and
   // cut into slices of 32 sites

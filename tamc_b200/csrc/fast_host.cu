@@ -72,7 +72,9 @@ static bool fits(const tamc_gpu* g, const PtJob& j, uint32_t T, bool csr) {
 
 // 512 threads with the instance in shared memory if that fits, else the
 // largest CTA (512, 256, 128) whose shared memory fits without it.
+static TileChoice rows_tile(const PtJob& j);
 static TileChoice heuristic_tile(const tamc_gpu* g, const PtJob& j) {
+  if (j.rows) return rows_tile(j);
   if (fits(g, j, 512, true)) return TileChoice{512, true};
   for (uint32_t T : {512u, 256u, 128u})
     if (T >= j.qps && fits(g, j, T, false)) return TileChoice{T, false};
@@ -119,7 +121,7 @@ static float time_tile(tamc_gpu* g, const PtJob& proto, TileChoice t, uint32_t r
     TAMC_CUDA(tamc::copy_async(dj.p, &j, sizeof(PtJob), cudaMemcpyHostToDevice, st));
     ctr.zero(st);
     TAMC_CUDA(cudaEventRecord(e0, st));
-    fused_launch(st, dj.p, 1, ctr.p, 1, t.T, smem);
+    fused_launch(st, dj.p, 1, ctr.p, 1, t.T, smem, j.rows);
     TAMC_CUDA(cudaEventRecord(e1, st));
     g->count();
     TAMC_CUDA(cudaEventSynchronize(e1));  // also keeps the host copy of j unchanged until it is read
@@ -138,9 +140,16 @@ thread_local bool g_no_autotune = false;
 // Set while a batch adds a run: its initial replicas wait for the first chunk.
 thread_local bool g_defer_init = false;
 
+// On lattice rows: 256 threads up to 256 sites, else 512 (microseconds a round,
+// 2 x 32 replicas: 16 x 16 sites 9.1 at 128 threads, 6.5 at 256, 6.3 at 512;
+// 32 x 32 sites 22.2, 13.3, 10.2, and 10.7 at 1024).
+static TileChoice rows_tile(const PtJob& j) { return TileChoice{j.n > 256 ? 512u : 256u, false}; }
+
 static TileChoice tune_tile(tamc_gpu* g, const PtJob& j) {
+  if (j.rows) return rows_tile(j);
   if (g_no_autotune) return heuristic_tile(g, j);
-  const auto key = std::make_tuple(g->device, j.n, j.F.nnz, j.nt, j.C, (int)j.self_loops, (int)j.icm_uf);
+  const auto key = std::make_tuple(g->device, j.n, j.F.nnz, j.nt, j.C, (int)j.self_loops,
+                                   (int)j.icm_uf + 2 * j.msc);
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
     auto it = g_tune.find(key);
@@ -259,6 +268,7 @@ static void fill_job(tamc_pt* pt, uint64_t seed, tamc_pt::FastState* F) {
   // labelling (same clusters; BFS touches only the clusters)
   j.icm_uf = 0;
   if (const char* e = getenv("TAMC_ICM")) j.icm_uf = strcmp(e, "uf") == 0;
+  j.rows = fused_rows(j);
   const size_t budget = std::min<size_t>(pt->g->smem_optin, 110 * 1024);
   j.icm_group = std::max(1u, active);
   while (j.icm_group > 1 && fused_smem_bytes(j, 512, false) > budget) --j.icm_group;
@@ -282,7 +292,7 @@ static void launch_one(tamc_pt* pt, uint32_t begin, uint32_t end, int init) {
   j.s_base = pt->s_next;
   TAMC_CUDA(tamc::copy_async(F->d_job.p, &j, sizeof(PtJob), cudaMemcpyHostToDevice, st));
   F->ctr.zero(st);
-  fused_launch(st, F->d_job.p, 1, F->ctr.p, 1, F->T, F->smem);
+  fused_launch(st, F->d_job.p, 1, F->ctr.p, 1, F->T, F->smem, F->job.rows);
   pt->g->count();
   // the job struct is read by the kernel; keep the host copy alive until done
   TAMC_CUDA(cudaStreamSynchronize(st));
@@ -366,10 +376,17 @@ static void plain_init_energies(tamc_pt* pt, bool random) {
 // same results; the autotuner times a few rounds of each on this shape.
 static std::map<std::tuple<int, uint32_t, uint32_t, uint32_t, uint32_t, int>, bool> g_form;
 
+// Runs on lattice rows of at most 2048 words take neither the plain nor the
+// ladder form (microseconds a round on rows / in the ladder form, 8 to 32
+// temperatures: 2 chains on 8 x 8 sites 5.0-5.1 / 9.6-10.6, 16 x 16 5.6-6.4 /
+// 10.9-11.9, 32 x 32 8.8-10.1 / 13.8-15.0; 4 chains on 16 x 16 9.3-10.7 /
+// 11.5-12.2; above, 4 chains on 24 x 24 13.9-16.2 / 13.4-14.1).
+static bool rows_first(const PtJob& j) { return j.rows && j.n * j.nw <= 2048; }
+
 static bool choose_plain(tamc_pt* pt) {
   const char* f = getenv("TAMC_PT_FORM");
   if (f && !strcmp(f, "plain")) return true;
-  if (f && !strcmp(f, "fused")) return false;
+  if ((f && !strcmp(f, "fused")) || rows_first(pt->fast->job)) return false;
   if (g_no_autotune) return fused_smem_bytes(pt->fast->job, 128, false) > pt->g->smem_optin;
   const PtJob& j = pt->fast->job;
   const bool fused_fits = fused_smem_bytes(j, 128, false) <= pt->g->smem_optin;
@@ -445,7 +462,7 @@ static bool other_forms_take(const tamc_gpu* g, const PtJob& j) {
 
 // Sets the run up in the ladder form if it takes it: all its CTAs, one per
 // replica, are resident at once; rows in shared memory where they fit.
-// A single run takes it whenever it can: over square and cubic lattices, random
+// A single run takes it whenever it can and is not on lattice rows: over square and cubic lattices, random
 // regular graphs and QUBOs of 16 to 8000 sites, 8 to 64 temperatures, 2 and 4
 // chains, with and without Houdayer moves, a round took 5.0-70 us against the
 // better of 5.9-113 us in the other two forms, at best 7.3 times less (3-D
@@ -458,6 +475,7 @@ static bool ladder_setup(tamc_pt* pt) {
   const PtJob& j = F->job;
   const char* f = getenv("TAMC_PT_FORM");
   if (f && (!strcmp(f, "plain") || !strcmp(f, "fused"))) return false;
+  if (rows_first(j) && !(f && !strcmp(f, "ladder"))) return false;
   if (g_no_autotune || g_defer_init || j.icm_uf || !other_forms_take(pt->g, j)) return false;
   uint32_t T0 = j.n >= 4096 ? 1024u : j.n >= 512 ? 512u : j.n >= 256 ? 256u : 128u;
   if (const char* e = getenv("TAMC_PT_T")) T0 = (uint32_t)std::min(1024, std::max(128, atoi(e) / 128 * 128));
@@ -546,11 +564,7 @@ void fast_pt_create(tamc_pt* pt, uint64_t seed) {
     return;
   }
   fused_setup(pt);
-  if (g_defer_init) {  // drawn by the batch's first chunk launch (same chain)
-    pt->fast->init_pending = true;
-    return;
-  }
-  launch_one(pt, 0, 0, 1);  // random initial replicas and their energies
+  pt->fast->init_pending = true;  // random initial replicas: drawn by the first launch
 }
 
 // Deferred initial replicas, when something reads or runs the run before its
@@ -563,7 +577,7 @@ static void ensure_init(tamc_pt* pt) {
 }
 
 void fast_pt_run(tamc_pt* pt, uint32_t sweep_end) {
-  if (!pt->fast->ladder) ensure_init(pt);
+  if (pt->fast->plain) ensure_init(pt);
   const PtCfg& c = pt->cfg;
   while (pt->next_sweep < sweep_end) {
     const uint32_t b = pt->next_sweep;
@@ -581,7 +595,8 @@ void fast_pt_run(tamc_pt* pt, uint32_t sweep_end) {
     } else if (pt->fast->plain) {
       plain_run_chunk(pt, e - b);
     } else {
-      launch_one(pt, b, e, 0);
+      launch_one(pt, b, e, pt->fast->init_pending ? 1 : 0);
+      pt->fast->init_pending = false;
     }
     pt->out.dirty = true;
     pt->m_next += count_sched(c.sample, c.meas_init, c.num_sweeps, b, e);
@@ -886,6 +901,7 @@ struct ChunkRunner {
     uint32_t T = 0, grid = 0;
     size_t smem = 0;
     int per_sm = 0;
+    bool rows = true;  // every run is on lattice rows
   };
   static Launch shape(tamc_gpu* g, std::vector<tamc_pt*>& grp, uint32_t T) {
     const char* csr_env = getenv("TAMC_PT_CSR");
@@ -910,7 +926,8 @@ struct ChunkRunner {
     Launch L;
     L.T = T;
     L.smem = smem;
-    L.per_sm = fused_blocks_per_sm(T, smem);
+    for (auto* pt : grp) L.rows = L.rows && pt->fast->job.rows;
+    L.per_sm = fused_blocks_per_sm(T, smem, L.rows);
     L.grid = std::min<uint32_t>((uint32_t)grp.size(), (uint32_t)(g->num_sms * std::max(L.per_sm, 1)));
     return L;
   }
@@ -972,13 +989,17 @@ struct ChunkRunner {
       // on C3 that measured 27.6 ms per 1000 sweeps against 35.0 ms at the
       // small runs' own autotuned 256 threads (two per SM), which time one
       // run alone on an otherwise idle SM
+      // (all on lattice rows, whose kernel takes half the registers: 256 measured
+      // 11.7 ms against 12.1 at 128, with one class of 512 threads 15.8)
       std::vector<tamc_pt*> big, small;
-      uint32_t Ts = 128;
       // (`by_size`: runs of at most 512 sites also go to the small class
       // whatever their tile, so that a batch built with heuristic tiles, all
       // of 512 threads, still splits)
       for (auto* pt : act)
         (pt->fast->T >= 512 && !(by_size && pt->fast->job.n <= 512) ? big : small).push_back(pt);
+      uint32_t Ts = 256;
+      for (auto* pt : small)
+        if (!pt->fast->job.rows) Ts = 128;
       if (const char* e = getenv("TAMC_PT_TSMALL")) {  // the small class's CTA size, for measurements
         const int t = atoi(e);
         if (t == 128 || t == 256) Ts = (uint32_t)t;
@@ -1039,19 +1060,20 @@ struct ChunkRunner {
     // the kernel launches of one chunk (both classes, or one launch)
     auto launch_all = [&]() {
       if (!split) {
-        fused_launch(st, d_jobs.p, na, ctr.p, A.grid, A.T, A.smem);
+        fused_launch(st, d_jobs.p, na, ctr.p, A.grid, A.T, A.smem, A.rows);
         return;
       }
-      fused_smem_limit(std::max(A.smem, B.smem));
+      fused_smem_limit(std::max(A.smem, B.smem), A.rows);
+      if (B.rows != A.rows) fused_smem_limit(B.smem, B.rows);
       TAMC_CUDA(cudaEventRecord(fork, st));
       TAMC_CUDA(cudaStreamWaitEvent(aux, fork, 0));
-      fused_launch_prio(st, d_jobs.p, nb, ctr.p, A.grid, A.T, A.smem, prio_hi);
-      fused_launch_prio(aux, d_jobs.p + nb, na - nb, ctr.p + 1, B.grid, B.T, B.smem, prio_lo);
+      fused_launch_prio(st, d_jobs.p, nb, ctr.p, A.grid, A.T, A.smem, prio_hi, A.rows);
+      fused_launch_prio(aux, d_jobs.p + nb, na - nb, ctr.p + 1, B.grid, B.T, B.smem, prio_lo, B.rows);
       TAMC_CUDA(cudaEventRecord(join, aux));
       TAMC_CUDA(cudaStreamWaitEvent(st, join, 0));
     };
     if (use_graph) {
-      const uint32_t key[8] = {na, nb, A.grid, A.T, (uint32_t)A.smem, B.grid, B.T, (uint32_t)B.smem};
+      const uint32_t key[8] = {na, nb, A.grid, 2 * A.T + A.rows, (uint32_t)A.smem, B.grid, 2 * B.T + B.rows, (uint32_t)B.smem};
       if (!sl.exec || memcmp(key, sl.key, sizeof(key)) != 0) {
         if (sl.exec) cudaGraphExecDestroy(sl.exec);
         if (sl.graph) cudaGraphDestroy(sl.graph);
@@ -1151,7 +1173,10 @@ struct ChunkRunner {
     if (j.F.lat_any) return T >= 512 ? 11 + 0.0045 * n : T >= 256 ? 13 + 0.008 * n : 16 + 0.013 * n;
     return T >= 512 ? 25 + 0.0092 * n : T >= 256 ? 26 + 0.0125 * n : 27 + 0.022 * n;
   }
+  // (on lattice rows, pairs of words: 8^2 sites 5, 32^2 10; two pairs 7, 17)
   static double fused_us(const PtJob& j) {
+    if (j.rows)
+      return 3 + 1.8 * ((j.C + 1) / 2 * j.wpc) + 2e-3 * j.n * j.nw + 2.4e-5 * ((double)j.n * j.C * j.ntp);
     const double nr = (double)j.n * j.C * j.ntp;
     return 12 + nr * (j.msc ? 0.16e-3 : j.F.udeg ? 1.2e-3 : j.n > 2048 ? 2.3e-3 : 2e-3);
   }

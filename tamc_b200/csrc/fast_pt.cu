@@ -981,6 +981,98 @@ __device__ void icm_phase(const PtJob& J, const FastInst& F, Smem& S, uint32_t i
   }
 }
 
+// The exchange decisions of chain c (bit j: slots j and j + 1 swap), by a warp:
+// energy(j) is slot j's cached energy as the reference compares it, dbeta(j)
+// the difference of the inverse temperatures.
+template <typename E, typename B>
+__device__ __forceinline__ uint64_t exchange_bits(const PtJob& J, uint32_t c, uint32_t i, E energy, B dbeta) {
+  const uint32_t lane = threadIdx.x & 31u, nt = J.nt;
+  uint64_t D = 0;
+  if (J.threaded) {
+    bool d[2] = {false, false};
+    for (int h = 0; h < 2; ++h) {
+      const uint32_t j = lane + 32u * h;
+      if (j + 1 < nt) {
+        const float des = energy(j + 1) - energy(j);
+        const float dlt = (dbeta(j)) * des;
+        d[h] = dlt >= 0.0f ||
+               u24(philox4x32_10(make_uint4(j, i, c, PTAG_EXCH), J.key).x) < __expf(dlt);
+      }
+    }
+    D = (uint64_t)__ballot_sync(0xffffffffu, d[0]) | ((uint64_t)__ballot_sync(0xffffffffu, d[1]) << 32);
+  } else {
+    // Serial semantics: pair j sees ΔE_j plus the carried ΔE_{j-1} when pair
+    // j - 1 swapped (tamc-core/src/pt.rs:138-141).  The draws, Δβ, ΔE_j and
+    // the decisions without a carry do not depend on earlier pairs, so lane
+    // j % 32 computes them for pair j in parallel; the walk over the pairs
+    // then redoes only the decisions whose lower pair swapped, with the same
+    // float operations as a plain sequential loop (same decisions).
+    float des0[2], db[2], u[2];
+    bool d0[2];
+    for (int h = 0; h < 2; ++h) {
+      const uint32_t j = lane + 32u * h;
+      des0[h] = 0.0f;
+      db[h] = 0.0f;
+      u[h] = 1.0f;
+      d0[h] = false;
+      if (j + 1 < nt) {
+        des0[h] = energy(j + 1) - energy(j);
+        db[h] = dbeta(j);
+        u[h] = u24(philox4x32_10(make_uint4(j, i, c, PTAG_EXCH), J.key).x);
+        const float dlt = db[h] * des0[h];
+        d0[h] = dlt >= 0.0f || u[h] < __expf(dlt);
+      }
+    }
+    const uint64_t D0 =
+        (uint64_t)__ballot_sync(0xffffffffu, d0[0]) | ((uint64_t)__ballot_sync(0xffffffffu, d0[1]) << 32);
+    float carry = 0.0f;
+    bool prev = false;
+    for (uint32_t j = 0; j + 1 < nt; ++j) {  // warp-uniform: every lane walks the same values
+      const bool hi = j >= 32u;
+      const float e = __shfl_sync(0xffffffffu, hi ? des0[1] : des0[0], j & 31u);
+      const float b = __shfl_sync(0xffffffffu, hi ? db[1] : db[0], j & 31u);
+      const float uj = __shfl_sync(0xffffffffu, hi ? u[1] : u[0], j & 31u);
+      float des = e;
+      bool dj;
+      if (prev) {
+        des = e + carry;
+        const float dlt = b * des;
+        dj = dlt >= 0.0f || uj < __expf(dlt);
+      } else {
+        dj = (D0 >> j) & 1ull;
+      }
+      if (dj) D |= 1ull << j;
+      prev = dj;
+      carry = des;
+    }
+  }
+  return D;
+}
+
+// Round trips of chain c after its tags moved (by a warp).
+__device__ __forceinline__ void exchange_trips(const XchgSm& XS, uint32_t c, uint32_t nt) {
+  const uint32_t lane = threadIdx.x & 31u;
+  uint8_t* tg = XS.tags + (size_t)c * nt;
+  if (lane == 0) {  // PTState::update_round_trips (tamc-core/src/pt.rs:54-72)
+    uint8_t lo = tg[0];
+    if (lo == 0) lo = 1;
+    else if (lo == 4) { XS.rtrips[c] += 1; lo = 1; }
+    else if (lo == 2) lo = 3;
+    tg[0] = lo;
+    uint8_t hi = tg[nt - 1];
+    if (hi == 0) hi = 2;
+    else if (hi == 3) { XS.rtrips[c] += 1; hi = 2; }
+    else if (hi == 1) hi = 4;
+    tg[nt - 1] = hi;
+  }
+  __syncwarp();
+  for (uint32_t k = lane; k < nt; k += 32) {
+    const uint8_t v = tg[k];
+    if (v == 1 || v == 3) XS.dhist[((size_t)c * nt + k) * 2] += 1;
+    else if (v == 2 || v == 4) XS.dhist[((size_t)c * nt + k) * 2 + 1] += 1;
+  }
+}
+
 // Exchange decisions of round i (threaded or serial semantics), acceptance
 // counts, the slot permutation of energies and tags, round trips; S.Dm[c]
 // receives the swapped pairs of chain c.
@@ -992,65 +1084,9 @@ __device__ void exchange_decide(const PtJob& J, Smem& S, uint32_t i) {
   for (uint32_t c = warp; c < J.C; c += nwarp) {
     double* Ec = S.Ec + c * J.ntp;
     double* Er = S.Er + c * J.ntp;
-    uint64_t D = 0;
-    if (J.threaded) {
-      bool d[2] = {false, false};
-      for (int h = 0; h < 2; ++h) {
-        const uint32_t j = lane + 32u * h;
-        if (j + 1 < nt) {
-          const float des = (float)Ec[j + 1] - (float)Ec[j];
-          const float dlt = (S.xb ? XS.dbeta[j] : J.betas[j + 1] - J.betas[j]) * des;
-          d[h] = dlt >= 0.0f ||
-                 u24(philox4x32_10(make_uint4(j, i, c, PTAG_EXCH), J.key).x) < __expf(dlt);
-        }
-      }
-      D = (uint64_t)__ballot_sync(0xffffffffu, d[0]) | ((uint64_t)__ballot_sync(0xffffffffu, d[1]) << 32);
-    } else {
-      // Serial semantics: pair j sees ΔE_j plus the carried ΔE_{j-1} when pair
-      // j - 1 swapped (tamc-core/src/pt.rs:138-141).  The draws, Δβ, ΔE_j and
-      // the decisions without a carry do not depend on earlier pairs, so lane
-      // j % 32 computes them for pair j in parallel; the walk over the pairs
-      // then redoes only the decisions whose lower pair swapped, with the same
-      // float operations as a plain sequential loop (same decisions).
-      float des0[2], db[2], u[2];
-      bool d0[2];
-      for (int h = 0; h < 2; ++h) {
-        const uint32_t j = lane + 32u * h;
-        des0[h] = 0.0f;
-        db[h] = 0.0f;
-        u[h] = 1.0f;
-        d0[h] = false;
-        if (j + 1 < nt) {
-          des0[h] = (float)Ec[j + 1] - (float)Ec[j];
-          db[h] = S.xb ? XS.dbeta[j] : J.betas[j + 1] - J.betas[j];
-          u[h] = u24(philox4x32_10(make_uint4(j, i, c, PTAG_EXCH), J.key).x);
-          const float dlt = db[h] * des0[h];
-          d0[h] = dlt >= 0.0f || u[h] < __expf(dlt);
-        }
-      }
-      const uint64_t D0 =
-          (uint64_t)__ballot_sync(0xffffffffu, d0[0]) | ((uint64_t)__ballot_sync(0xffffffffu, d0[1]) << 32);
-      float carry = 0.0f;
-      bool prev = false;
-      for (uint32_t j = 0; j + 1 < nt; ++j) {  // warp-uniform: every lane walks the same values
-        const bool hi = j >= 32u;
-        const float e = __shfl_sync(0xffffffffu, hi ? des0[1] : des0[0], j & 31u);
-        const float b = __shfl_sync(0xffffffffu, hi ? db[1] : db[0], j & 31u);
-        const float uj = __shfl_sync(0xffffffffu, hi ? u[1] : u[0], j & 31u);
-        float des = e;
-        bool dj;
-        if (prev) {
-          des = e + carry;
-          const float dlt = b * des;
-          dj = dlt >= 0.0f || uj < __expf(dlt);
-        } else {
-          dj = (D0 >> j) & 1ull;
-        }
-        if (dj) D |= 1ull << j;
-        prev = dj;
-        carry = des;
-      }
-    }
+    const uint64_t D = exchange_bits(
+        J, c, i, [&](uint32_t j) { return (float)Ec[j]; },
+        [&](uint32_t j) { return S.xb ? XS.dbeta[j] : J.betas[j + 1] - J.betas[j]; });
     // acceptance counts, slot permutation of energies and tags, round trips
     uint32_t* acc = XS.acc + (size_t)c * nt;
     uint8_t* tg = XS.tags + (size_t)c * nt;
@@ -1079,24 +1115,7 @@ __device__ void exchange_decide(const PtJob& J, Smem& S, uint32_t i) {
       tg[k] = t_new[h];
     }
     __syncwarp();
-    if (lane == 0) {  // PTState::update_round_trips (tamc-core/src/pt.rs:54-72)
-      uint8_t lo = tg[0];
-      if (lo == 0) lo = 1;
-      else if (lo == 4) { XS.rtrips[c] += 1; lo = 1; }
-      else if (lo == 2) lo = 3;
-      tg[0] = lo;
-      uint8_t hi = tg[nt - 1];
-      if (hi == 0) hi = 2;
-      else if (hi == 3) { XS.rtrips[c] += 1; hi = 2; }
-      else if (hi == 1) hi = 4;
-      tg[nt - 1] = hi;
-    }
-    __syncwarp();
-    for (uint32_t k = lane; k < nt; k += 32) {
-      const uint8_t v = tg[k];
-      if (v == 1 || v == 3) XS.dhist[((size_t)c * nt + k) * 2] += 1;
-      else if (v == 2 || v == 4) XS.dhist[((size_t)c * nt + k) * 2 + 1] += 1;
-    }
+    exchange_trips(XS, c, nt);
     if (lane == 0) S.Dm[c] = D;
   }
   __syncthreads();
@@ -1624,10 +1643,630 @@ __device__ void run_job(const PtJob& J, char* smem_base) {
   xchg_store(J, S.xb);
 }
 
+// ---- +-J square lattices of even side up to 32 on lattice rows (PtJob::rows)
+// A round of a small run is a chain of short steps, and its time is the steps'
+// latency: 24 us a round at 32 x 32 sites and 2 x 32 replicas, with 40 % of the
+// issue slots in use.  Here the replica words are transposed once a round to a
+// bitmap per slot, and a warp (on 16 or 8 rows half or a quarter of one) takes a
+// slot, the lane of row r its row in a register.  A slot's energies are then
+// popcounts against bitmaps of the couplings' signs, its Houdayer move needs no
+// barrier, no atomics and no list: a step of the growth fills whole runs of a
+// row (an add each way) and looks one row up and down (two shuffles).  The
+// clusters are transposed back, and the sweep keeps no energies at all.
+// With symmetric +-1 couplings, no field and no offset E = 2 n - 2 S with S the
+// satisfied bonds: integers well below 2^24, so the same floats and doubles as
+// the sums of the changes.
+// (32 x 32 sites, 2 x 32 replicas, 512 threads, a round: 24.2 us on the general
+// path, 10.1 here; 8 x 8 sites, 12.1 and 5.1.)
+struct RowsSm {  // byte offsets (from pointers kept in a struct the compiler makes generic loads)
+  uint32_t W, msc, Ec, E, Em, Dm, nb, sw, jw, bits, red, xb, bytes;
+  uint32_t inv;  // ceil(2^16 / L)
+};
+template <typename V>
+__device__ __forceinline__ V* rows_at(uint32_t off) {
+  extern __shared__ uint4 smem_u4[];
+  return reinterpret_cast<V*>(reinterpret_cast<char*>(smem_u4) + off);
+}
+constexpr uint32_t ROWS_STRIDE = 33;  // words between a bitmap's slots: lanes on slots hit different banks
+constexpr uint32_t ROWS_MAP = 32 * ROWS_STRIDE;  // a bitmap of 32 slots
+enum { ROWS_D = 0, ROWS_R = ROWS_MAP, ROWS_C = 2 * ROWS_MAP };  // disagreements and replica 0 by site, clusters by row
+__host__ __device__ inline RowsSm rows_carve(uint32_t n, uint32_t nw, uint32_t wpc, uint32_t C, uint32_t ntp,
+                                             uint32_t L) {
+  uint32_t o = 0;
+  auto take = [&](size_t bytes) {
+    const uint32_t at = o;
+    o = (uint32_t)al16(o + bytes);
+    return at;
+  };
+  RowsSm X;
+  X.W = take((size_t)n * nw * 4);
+  X.msc = take((size_t)nw * MSC_WORDS * 4);
+  X.E = take((size_t)C * ntp * 4);   // energies after the sweep
+  X.Em = take((size_t)C * ntp * 4);  // and after the next round's Houdayer moves
+  X.Ec = take((size_t)C * ntp * 8);  // the former as doubles, for the measurements
+  X.Dm = take((size_t)C * 8);
+  X.nb = take((size_t)n * 8);        // four neighbours a site, 16 bits each: site, top bit J < 0
+  X.sw = take((size_t)nw * 8 * 16);  // a sweep's part of the first two Philox rounds, per (word, call)
+  X.jw = take(64 * 4);               // per row: signs of the bonds to the right, then down
+  X.bits = take((size_t)(C + 1) / 2 * wpc * 3 * ROWS_MAP * 4);  // per pair of words (measurements: n words)
+  X.red = take(16);                  // the round's least energy: energy << 16 | chain and slot
+  X.xb = take(xchg_layout(nullptr, nullptr, C, ntp));
+  X.bytes = o;
+  X.inv = (65536 + L - 1) / L;
+  return X;
+}
+
+// The job and the offsets, in shared memory (they would take 20 registers of the
+// 64, and through a reference parameter their loads would be generic).
+__device__ __forceinline__ PtJob& rows_job() {
+  __shared__ PtJob J;
+  return J;
+}
+__device__ __forceinline__ RowsSm& rows_sm() {
+  __shared__ RowsSm X;
+  return X;
+}
+
+// Row and colour site of file site f (`inv` = ceil(2^16 / L); f < 1024).
+__device__ __forceinline__ uint32_t rows_site(uint32_t f, uint32_t L, uint32_t inv, uint32_t half) {
+  const uint32_t r = (f * inv) >> 16;
+  return ((r + f - r * L) & 1u) * half + (f >> 1);
+}
+
+// The k-th set bit of m (k < popc(m)).
+__device__ __forceinline__ uint32_t nth_bit(uint32_t m, uint32_t k) {
+  uint32_t pos = 0;
+#pragma unroll
+  for (uint32_t z = 16; z; z >>= 1) {
+    const uint32_t c = __popc(m & ((1u << z) - 1u));
+    const bool up = k >= c;
+    k -= up ? c : 0u;
+    m = up ? m >> z : m;
+    pos += up ? z : 0u;
+  }
+  return pos;
+}
+
+// Runs of d's set bits that contain a bit of c (c within d).
+__device__ __forceinline__ uint32_t run_fill(uint32_t c, uint32_t d) {
+  const uint32_t rd = __brev(d), rc = __brev(c);
+  return ((((d + c) ^ d) & d) | c) | __brev((((rd + rc) ^ rd) & rd) | rc);
+}
+
+// Bitmaps by file site, per slot: the disagreements of each pair of words (0 for
+// the last of an odd number of chains) and replica 0.
+__device__ __forceinline__ void rows_bitmaps() {
+  const PtJob& J = rows_job();
+  const RowsSm& X = rows_sm();
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
+  const uint32_t n = J.n, nw = J.nw, L = J.F.cb_L, inv = X.inv, half = n / 2, nch = (n + 31) / 32;
+  const uint32_t* const W = rows_at<const uint32_t>(X.W);
+  for (uint32_t c = 0, g = 0; c < J.C; c += 2)
+    for (uint32_t w = 0; w < J.wpc; ++w, ++g) {
+      const uint32_t o0 = c * J.wpc + w, o1 = c + 1 < J.C ? o0 + J.wpc : o0;
+      uint32_t* const map = rows_at<uint32_t>(X.bits) + g * 3 * ROWS_MAP + lane * ROWS_STRIDE;
+      for (uint32_t ch = warp; ch < nch; ch += nwarp) {
+        const uint32_t f = 32 * ch + lane;
+        uint32_t v0 = 0, v1 = 0;
+        if (f < n) {
+          const uint32_t s = rows_site(f, L, inv, half) * nw;
+          v0 = W[s + o0];
+          v1 = W[s + o1];
+        }
+        map[ROWS_D + ch] = transpose32(v0 ^ v1, lane);
+        map[ROWS_R + ch] = transpose32(v0, lane);
+      }
+    }
+  __syncthreads();
+}
+
+// Every slot's energies, the round's least one, and with `move` the clusters of
+// round i's Houdayer moves and the energies after them: a team of LW lanes per
+// slot (FULL: LW rows).
+template <uint32_t LW, bool FULL>
+__device__ __forceinline__ void rows_slots(uint32_t i, bool move) {
+  const PtJob& J = rows_job();
+  const RowsSm& X = rows_sm();
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
+  const uint32_t L = J.F.cb_L;
+  const uint32_t* const jw = rows_at<const uint32_t>(X.jw);
+  constexpr uint32_t TEAMS = 32 / LW;
+  const uint32_t row = lane % LW, team0 = lane - row, up = L - 1;
+  const bool has = row < L;
+  const uint32_t Lm = has ? (L == 32 ? 0xffffffffu : (1u << L) - 1u) : 0u;
+  constexpr int LOG = LW == 32 ? 5 : LW == 16 ? 4 : 3;
+  // v of the row k below (round the lattice's end)
+  auto from = [&](uint32_t v, int k) -> uint32_t {
+    if (FULL) return __shfl_sync(0xffffffffu, v, (int)row + k, LW);
+    const int r = (int)row + k, n_r = (int)L;
+    return __shfl_sync(0xffffffffu, v, (int)team0 + (r < 0 ? r + n_r : r >= n_r ? r - n_r : r));
+  };
+  const uint32_t wd = (row * L) >> 5, sh = (row * L) & 31u;
+  const uint32_t even = (row & 1u) ? 0xaaaaaaaau : 0x55555555u;  // the row's sites of colour class 0
+  const uint32_t jr = jw[has ? row : 0u], jd = jw[32 + (has ? row : 0u)];
+  auto sum = [&](int v) -> int {
+    if (LW == 32) return __reduce_add_sync(0xffffffffu, v);
+#pragma unroll
+    for (uint32_t o = LW / 2; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+  };
+  for (uint32_t c = 0, g = 0; c < J.C; c += 2)
+    for (uint32_t w = 0; w < J.wpc; ++w, ++g) {
+      uint32_t* const map = rows_at<uint32_t>(X.bits) + g * 3 * ROWS_MAP;
+      const bool pair = c + 1 < J.C;
+      const uint32_t slots = min(J.nt - 32 * w, 32u);
+      for (uint32_t g0 = warp * TEAMS; g0 < slots; g0 += nwarp * TEAMS) {
+        const uint32_t b = g0 + lane / LW, t = 32 * w + b;
+        const bool on = has && b < slots;
+        uint32_t d = 0, r = 0;
+        if (on) {
+          const uint32_t* const m = map + b * ROWS_STRIDE + wd;
+          d = __funnelshift_r(m[ROWS_D], m[ROWS_D + 1], sh) & Lm;
+          r = __funnelshift_r(m[ROWS_R], m[ROWS_R + 1], sh) & Lm;
+        }
+        // satisfied bonds of replica 0, to the right (round the row's end) and
+        // down, and what is different for replica 1
+        auto right = [&](uint32_t v) { return (v >> 1) | ((v & 1u) << up); };
+        const uint32_t d_dn = from(d, 1), r_dn = from(r, 1);
+        const uint32_t ar = (r ^ right(r) ^ jr) & Lm, ad = (r ^ r_dn ^ jd) & Lm;
+        const uint32_t qr = (d ^ right(d)) & Lm, qd = (d ^ d_dn) & Lm;
+        const int S = sum((__popc(ar) + __popc(ad)) | ((__popc(ar ^ qr) + __popc(ad ^ qd)) << 16));
+        const int E0 = 2 * (int)(J.n - (S & 0xffff)), E1 = 2 * (int)(J.n - (S >> 16));
+        const uint32_t x0 = c * J.ntp + t, x1 = x0 + J.ntp;
+        if (on && row == 0) {
+          int* const E = rows_at<int>(X.E);
+          E[x0] = E0;
+          int key = E0 * 65536 + (int)(c * J.nt + t);
+          if (pair) {
+            E[x1] = E1;
+            key = min(key, E1 * 65536 + (int)((c + 1) * J.nt + t));
+          }
+          atomicMin(rows_at<int>(X.red), key);
+        }
+        int dE = 0;
+        const bool in = move && pair && on && t >= J.lo;
+        if (__any_sync(0xffffffffu, in)) {
+          // the seed: the k-th disagreeing site in colour order
+          const uint32_t u = philox4x32_10w(make_uint4(t, i, c / 2, PTAG_ICM), J.key).x;
+          const uint32_t own = in ? __popc(d & even) | (__popc(d & ~even) << 16) : 0u;
+          uint32_t incl = own;
+#pragma unroll
+          for (uint32_t o = 1; o < LW; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o, LW);
+            incl += row >= o ? y : 0u;
+          }
+          const uint32_t tot = __shfl_sync(0xffffffffu, incl, LW - 1, LW);
+          const uint32_t cnt = (tot & 0xffffu) + (tot >> 16);
+          uint32_t cl = 0;
+          if (cnt) {
+            uint32_t k = (uint32_t)(((uint64_t)u * cnt) >> 32);
+            const bool odd = k >= (tot & 0xffffu);
+            k -= odd ? tot & 0xffffu : 0u;
+            const uint32_t mine = odd ? own >> 16 : own & 0xffffu, excl = (odd ? incl >> 16 : incl & 0xffffu) - mine;
+            if (k >= excl && k < excl + mine) cl = 1u << nth_bit(d & (odd ? ~even : even), k - excl);
+          }
+          // growth by whole runs of the columns (log2 LW steps of twice the length
+          // each, both ways at once), then of the rows; a step that is not the last
+          // adds a site, so they end within 32 n.  (On a cluster of the 32 x 32
+          // lattice 4 such steps, where one row up and down at a time took 18.)
+          uint32_t dn[LOG], upw[LOG];  // columns disagreeing from this row over 2^k rows
+          dn[0] = upw[0] = d;
+#pragma unroll
+          for (int k = 1; k < LOG; ++k) {
+            dn[k] = dn[k - 1] & from(dn[k - 1], -(1 << (k - 1)));
+            upw[k] = upw[k - 1] & from(upw[k - 1], 1 << (k - 1));
+          }
+          for (uint32_t step = 0; step < 32u * 1024u; ++step) {
+            const uint32_t before = cl;
+            uint32_t a = cl, b = cl;
+#pragma unroll
+            for (int k = 0; k < LOG; ++k) {
+              a |= dn[k] & from(a, -(1 << k));
+              b |= upw[k] & from(b, 1 << k);
+            }
+            a |= b;
+            cl = run_fill(a | (d & ((a << up) | (a >> up))), d);
+            if (!__any_sync(0xffffffffu, cl != before)) break;
+          }
+          // the bonds across the cluster's boundary change sides
+          const uint32_t c_dn = from(cl, 1);
+          const int now = sum(__popc(ar ^ ((cl ^ right(cl)) & Lm)) + __popc(ad ^ ((cl ^ c_dn) & Lm)));
+          dE = 2 * ((S & 0xffff) - now);
+          if (in) map[ROWS_C + b * ROWS_STRIDE + row] = cl;
+        }
+        if (on && row == 0) {
+          int* const Em = rows_at<int>(X.Em);
+          Em[x0] = E0 + (in ? dE : 0);
+          if (pair) Em[x1] = E1 - (in ? dE : 0);
+        }
+      }
+    }
+  __syncthreads();
+}
+__device__ __forceinline__ void rows_energies(uint32_t i, bool move, PhaseClock& pc) {
+  rows_bitmaps();
+  pc.lap(PHASE_ICM_INIT);
+  const uint32_t L = rows_job().F.cb_L;
+  if (L == 32) rows_slots<32, true>(i, move);
+  else if (L > 16) rows_slots<32, false>(i, move);
+  else if (L == 16) rows_slots<16, true>(i, move);
+  else if (L > 8) rows_slots<16, false>(i, move);
+  else rows_slots<8, false>(i, move);
+  pc.lap(PHASE_ICM_GROW);
+}
+
+__device__ __forceinline__ uint32_t bitperm32(uint32_t v, uint32_t D) {  // bitperm of at most 32 slots
+  const uint32_t S = D & ~(D << 1), E = (D << 1) & ~D;
+  return ((v >> 1) & D) | (((v & S) + D) & E) | (v & ~(D | (D << 1)));
+}
+
+// Flips the clusters in both replicas of their pairs: warps w0 and on.
+__device__ __forceinline__ void rows_flip(uint32_t w0) {
+  const PtJob& J = rows_job();
+  const RowsSm& X = rows_sm();
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
+  const uint32_t n = J.n, nw = J.nw, L = J.F.cb_L, inv = X.inv, half = n / 2, nch = (n + 31) / 32;
+  uint32_t* const W = rows_at<uint32_t>(X.W);
+  for (uint32_t c = 0, g = 0; c + 1 < J.C; c += 2)
+    for (uint32_t w = 0; w < J.wpc; ++w, ++g) {
+      const uint32_t b0 = J.lo > 32 * w ? J.lo - 32 * w : 0u, b1 = min(J.nt - 32 * w, 32u);
+      const uint32_t o0 = c * J.wpc + w, o1 = o0 + J.wpc;
+      const uint32_t* const m = rows_at<const uint32_t>(X.bits) + g * 3 * ROWS_MAP + ROWS_C + lane * ROWS_STRIDE;
+      for (uint32_t ch = warp - w0; ch < nch; ch += nwarp - w0) {
+        uint32_t v = 0;
+        if (lane >= b0 && lane < b1) {
+          if (L == 32) {
+            v = m[ch];
+          } else {
+            for (uint32_t r = (32 * ch * inv) >> 16; r < L && r * L < 32 * ch + 32; ++r) {
+              const int at = (int)(r * L) - (int)(32 * ch);
+              const uint32_t cl = m[r];
+              v |= at >= 0 ? cl << at : cl >> -at;
+            }
+          }
+        }
+        v = transpose32(v, lane);
+        const uint32_t f = 32 * ch + lane;
+        if (f < n && v) {
+          const uint32_t s = rows_site(f, L, inv, half) * nw;
+          W[s + o0] ^= v;
+          W[s + o1] ^= v;
+        }
+      }
+    }
+}
+
+// What a sweep fixes of the first two Philox rounds of its calls' counters
+// (site, i, word << 8 | call, PTAG_MSC): a round multiplies two of the four
+// words, and those of word and call alone are the same for every site.
+__device__ __forceinline__ void rows_sweep_words(const PtJob& J, uint4* sw, uint32_t i) {
+  if (threadIdx.x < J.nw * 8) {
+    const uint64_t a = (uint64_t)0xCD9E8D57u * (((threadIdx.x >> 3) << 8) | (threadIdx.x & 7u));
+    const uint64_t b = (uint64_t)0xD2511F53u * ((uint32_t)(a >> 32) ^ i ^ J.key.x);
+    sw[threadIdx.x] = make_uint4((uint32_t)a ^ (J.key.x + 0x9E3779B9u), (uint32_t)(b >> 32) ^ (J.key.y + 0xBB67AE85u),
+                                 (uint32_t)b, 0u);
+  }
+}
+struct RowsSite {  // and what a site fixes
+  uint32_t b0, b1, b2;
+};
+__device__ __forceinline__ RowsSite rows_site_words(uint32_t s, uint2 key) {
+  const uint64_t a = (uint64_t)0xD2511F53u * s;
+  const uint64_t b = (uint64_t)0xCD9E8D57u * ((uint32_t)(a >> 32) ^ PTAG_MSC ^ key.y);
+  return RowsSite{(uint32_t)(b >> 32), (uint32_t)b, (uint32_t)a};
+}
+__device__ __forceinline__ uint4 rows_random(RowsSite t, uint4 u, uint2 k) {
+  uint4 c = make_uint4(t.b0 ^ u.x, t.b1, t.b2 ^ u.y, u.z);
+#pragma unroll
+  for (int r = 2; r < 10; ++r) {
+    const uint64_t p0 = (uint64_t)0xD2511F53u * c.x, p1 = (uint64_t)0xCD9E8D57u * c.z;
+    c = make_uint4((uint32_t)(p1 >> 32) ^ c.y ^ (k.x + r * 0x9E3779B9u), (uint32_t)p1,
+                   (uint32_t)(p0 >> 32) ^ c.w ^ (k.y + r * 0xBB67AE85u), (uint32_t)p0);
+  }
+  return c;
+}
+
+// The exchange of round i: decisions and bookkeeping by a warp per chain, and
+// the other warps flip the Houdayer clusters meanwhile; then the permutation of
+// the words.  (Energies are not moved: the next are counted.)
+__device__ __forceinline__ void rows_exchange(uint32_t i, PhaseClock& pc) {
+  const PtJob& J = rows_job();
+  const RowsSm& X = rows_sm();
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, nwarp = blockDim.x >> 5;
+  const uint32_t nt = J.nt, beside = nwarp > J.C ? J.C : 0u;  // warps that do not flip
+  if (J.icm && warp >= beside) rows_flip(beside);
+  for (uint32_t c = warp; c < J.C; c += nwarp) {
+    XchgSm XS;
+    xchg_layout(&XS, rows_at<char>(X.xb), J.C, J.ntp);
+    const int* const Em = rows_at<const int>(X.Em) + c * J.ntp;
+    const uint64_t D = exchange_bits(
+        J, c, i, [&](uint32_t j) { return (float)Em[j]; }, [&](uint32_t j) { return XS.dbeta[j]; });
+    if (lane == 0) rows_at<unsigned long long>(X.Dm)[c] = D;
+    uint32_t* acc = XS.acc + (size_t)c * nt;
+    uint8_t* tg = XS.tags + (size_t)c * nt;
+    uint8_t t_new[2];
+    for (int h = 0; h < 2; ++h) {
+      const uint32_t k = lane + 32u * h;
+      if (k >= nt) continue;
+      uint32_t src = k;
+      if ((D >> k) & 1ull) {
+        acc[k] += 1;
+        src = k + 1;
+      } else if (k > 0 && ((D >> (k - 1)) & 1ull)) {
+        const uint64_t nd = ~D & ((1ull << k) - 1ull);
+        src = nd ? (uint32_t)(64 - __clzll((long long)nd)) : 0u;
+      }
+      t_new[h] = tg[src];
+    }
+    __syncwarp();
+    for (int h = 0; h < 2; ++h) {
+      const uint32_t k = lane + 32u * h;
+      if (k < nt) tg[k] = t_new[h];
+    }
+    __syncwarp();
+    exchange_trips(XS, c, nt);
+  }
+  __syncthreads();
+  pc.lap(PHASE_EXCH);
+  rows_sweep_words(J, rows_at<uint4>(X.sw), i);
+  if (tid == 0) *rows_at<int>(X.red) = 0x7fffffff;
+  const unsigned long long* const Dm = rows_at<const unsigned long long>(X.Dm);
+  if (J.nw == 2 && J.wpc == 1) {
+    const uint32_t D0 = (uint32_t)Dm[0], D1 = (uint32_t)Dm[1];
+    uint2* const W = rows_at<uint2>(X.W);
+    for (uint32_t s = tid; s < J.n; s += blockDim.x) {
+      const uint2 v = W[s];
+      W[s] = make_uint2(bitperm32(v.x, D0), bitperm32(v.y, D1));
+    }
+  } else {
+    uint32_t* const W = rows_at<uint32_t>(X.W);
+    for (uint32_t x = tid; x < J.n * J.C; x += blockDim.x) {
+      const uint32_t c = x % J.C;
+      uint32_t* const w = W + x * J.wpc;
+      if (J.wpc == 1) {
+        w[0] = bitperm32(w[0], (uint32_t)Dm[c]);
+      } else {
+        const uint64_t v = bitperm(w[0] | ((uint64_t)w[1] << 32), Dm[c]);
+        w[0] = (uint32_t)v;
+        w[1] = (uint32_t)(v >> 32);
+      }
+    }
+  }
+  __syncthreads();
+  pc.lap(PHASE_ICM_APPLY);
+}
+
+// A word's replicas with no unsatisfied bond (z), those that need random words
+// (und, at none or one), and the word after the flips that need none (S: S0 on
+// entry or another).
+__device__ __forceinline__ void rows_levels(uint32_t S0, const uint32_t* W, const uint32_t* neg, const uint32_t* pl,
+                                            uint32_t& z, uint32_t& und, uint32_t& S) {
+  const uint32_t u0 = ~(S0 ^ W[0] ^ neg[0]), u1 = ~(S0 ^ W[1] ^ neg[1]);
+  const uint32_t u2 = ~(S0 ^ W[2] ^ neg[2]), u3 = ~(S0 ^ W[3] ^ neg[3]);
+  const uint32_t a = u0 ^ u1, ca = u0 & u1, b = u2 ^ u3, cb = u2 & u3;
+  const uint32_t two = ca | cb | (a & b);  // two or more
+  const uint32_t one = (a ^ b) & ~two;
+  z = ~(a | b | two);
+  und = (z & ~(pl[96] | pl[99])) | (one & ~(pl[97] | pl[100]));
+  S = S0 ^ (two | (z & pl[96]) | (one & pl[97]));
+}
+// msc_step4 with fewer operations: the two levels' planes by a select (replicas
+// at neither are decided already), and the group's comparison from its lowest
+// bit up, an operation a bit.
+__device__ __forceinline__ void rows_step4(uint4 r, const uint32_t* pl, uint32_t z, uint32_t kk, uint32_t& und,
+                                           uint32_t& lt) {
+  const uint4 A = *reinterpret_cast<const uint4*>(pl + 28 - 4 * kk);
+  const uint4 B = *reinterpret_cast<const uint4*>(pl + 60 - 4 * kk);
+  const uint32_t t0 = (A.w & z) | (B.w & ~z), t1 = (A.z & z) | (B.z & ~z);
+  const uint32_t t2 = (A.y & z) | (B.y & ~z), t3 = (A.x & z) | (B.x & ~z);
+  uint32_t l = ~r.w & t3;
+  l = (~r.z & t2) | (l & ~(r.z ^ t2));
+  l = (~r.y & t1) | (l & ~(r.y ^ t1));
+  l = (~r.x & t0) | (l & ~(r.x ^ t0));
+  lt |= und & l;
+  und &= ~(r.x ^ t0);
+  und &= ~(r.y ^ t1);
+  und &= ~(r.z ^ t2);
+  und &= ~(r.w ^ t3);
+}
+// The sweep (msc_flip's decisions): a warp on 32 sites of a colour class, a lane
+// per site, PER words at once.  A level group decides 15 of 16 replicas: of the
+// 2048 of a warp's two words some 100 are undecided after one group and 6 after
+// two, so two groups are compared outright, and from the third on a lane takes
+// one of its words at a time.
+template <uint32_t PER>
+__device__ __forceinline__ void rows_sweep(uint32_t i) {
+  const PtJob& J = rows_job();
+  const RowsSm& X = rows_sm();
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, nwarp = blockDim.x >> 5;
+  // words in groups of PER: ng = 1, 2 or 4 groups, of which nwarp is a multiple,
+  // so that a warp keeps its words
+  const uint32_t nw = J.nw, half = J.n / 2, lg = 31 - __clz(nw / PER), tasks = (half + 31) / 32 << lg;
+  uint32_t* const W = rows_at<uint32_t>(X.W);
+  const uint2 key = J.key;
+  const uint2* const nb = rows_at<const uint2>(X.nb);
+  const uint32_t wo = (warp & ((1u << lg) - 1u)) * PER;
+  const uint4* const sw = rows_at<const uint4>(X.sw) + wo * 8;
+  const uint32_t* const pl = rows_at<const uint32_t>(X.msc) + wo * MSC_WORDS;
+  for (uint32_t c = 0; c < 2; ++c) {
+    for (uint32_t task = warp; task < tasks; task += nwarp) {
+      const uint32_t h = (task >> lg) * 32 + lane, s = c * half + h;
+      if (h < half) {
+        const uint2 q = nb[s];
+        const uint32_t j[4] = {q.x & 0x7fffu, (q.x >> 16) & 0x7fffu, q.y & 0x7fffu, (q.y >> 16) & 0x7fffu};
+        const uint32_t neg[4] = {(uint32_t)((int)(q.x << 16) >> 31), (uint32_t)((int)q.x >> 31),
+                                 (uint32_t)((int)(q.y << 16) >> 31), (uint32_t)((int)q.y >> 31)};
+        uint32_t S0[PER], z[PER], und[PER], lt[PER], Wj[PER][4];
+        if (PER == 2) {
+#pragma unroll
+          for (uint32_t m = 0; m < 4; ++m) {
+            const uint2 v = *reinterpret_cast<const uint2*>(W + j[m] * nw + wo);
+            Wj[0][m] = v.x;
+            Wj[PER - 1][m] = v.y;
+          }
+          const uint2 v = *reinterpret_cast<const uint2*>(W + s * nw + wo);
+          S0[0] = v.x;
+          S0[PER - 1] = v.y;
+        } else {
+#pragma unroll
+          for (uint32_t m = 0; m < 4; ++m) Wj[0][m] = W[j[m] * nw + wo];
+          S0[0] = W[s * nw + wo];
+        }
+        const RowsSite t = rows_site_words(s, key);
+#pragma unroll
+        for (uint32_t k = 0; k < PER; ++k)
+          rows_levels(S0[k], Wj[k], neg, pl + k * MSC_WORDS, z[k], und[k], S0[k]);
+#pragma unroll
+        for (uint32_t k = 0; k < PER; ++k) lt[k] = 0;
+#pragma unroll
+        for (uint32_t kk = 0; kk < 2; ++kk)
+#pragma unroll
+          for (uint32_t k = 0; k < PER; ++k)
+            rows_step4(rows_random(t, sw[k * 8 + kk], key), pl + k * MSC_WORDS, z[k], kk, und[k], lt[k]);
+        uint32_t k = und[0] ? 0u : PER - 1, u = und[0] ? und[0] : und[PER - 1], kk = 2, l = 0;
+        while (u) {
+          rows_step4(rows_random(t, sw[k * 8 + kk], key), pl + k * MSC_WORDS, k ? z[PER - 1] : z[0], kk, u, l);
+          if (++kk == 8 || !u) {  // this word is decided
+            const bool first = PER == 2 && k == 0;
+            if (k) lt[PER - 1] |= l;
+            else lt[0] |= l;
+            u = first ? und[PER - 1] : 0u;
+            k = PER - 1;
+            kk = 2;
+            l = 0;
+          }
+        }
+        if (PER == 2) *reinterpret_cast<uint2*>(W + s * nw + wo) = make_uint2(S0[0] ^ lt[0], S0[PER - 1] ^ lt[PER - 1]);
+        else W[s * nw + wo] = S0[0] ^ lt[0];
+      }
+    }
+    __syncthreads();
+  }
+}
+
+// What round i's measurements need: nothing unless its least energy is a new
+// minimum or it is on a sampling schedule.
+__device__ __forceinline__ void rows_measure(uint32_t i, uint32_t& m_cur, uint32_t& s_cur) {
+  const PtJob& J = rows_job();
+  const RowsSm& X = rows_sm();
+  XchgSm XS;
+  xchg_layout(&XS, rows_at<char>(X.xb), J.C, J.ntp);
+  const int key = *rows_at<const int>(X.red);
+  const float e = (float)(key >> 16);
+  const bool lower = !XS.gs->have || e < XS.gs->minE;
+  if (!lower && !sched(J.sample, i, J.meas_init, J.num_sweeps) &&
+      !sched(J.sample_states, i, J.meas_init, J.num_sweeps))
+    return;
+  GsSnap g{0, 0, 0, 0};
+  if (lower) {
+    const uint32_t k = XS.gs->count;
+    if (k < J.log.cap) g = GsSnap{1, k, (key & 0xffff) / J.nt, (key & 0xffff) % J.nt};
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      XS.gs->have = 1;
+      XS.gs->minE = e;
+      if (g.fresh) {
+        J.log.steps[k] = i;
+        J.log.E[k] = e;
+      }
+      XS.gs->count = k + 1;
+    }
+  }
+  Smem S{};
+  S.W = rows_at<uint32_t>(X.W);
+  S.Ec = rows_at<double>(X.Ec);
+  for (uint32_t x = threadIdx.x; x < J.C * J.ntp; x += blockDim.x) S.Ec[x] = rows_at<const int>(X.E)[x];
+  __syncthreads();
+  measure_rest(J, J.F, S, J.F.sus, J.F.iperm, i, m_cur, s_cur, g, rows_at<uint32_t>(X.bits));
+}
+
+// (of rows_job())
+__device__ __forceinline__ void run_rows() {
+  const PtJob& J = rows_job();
+  RowsSm& X = rows_sm();
+  if (threadIdx.x == 0) X = rows_carve(J.n, J.nw, J.wpc, J.C, J.ntp, J.F.cb_L);
+  __syncthreads();
+  const uint32_t tid = threadIdx.x, T = blockDim.x, nwarp = T >> 5, n = J.n, nw = J.nw, L = J.F.cb_L;
+  uint32_t* const W = rows_at<uint32_t>(X.W);
+  msc_fill_planes<4>(J, rows_at<uint32_t>(X.msc));
+  uint2* const nb = rows_at<uint2>(X.nb);
+  for (uint32_t s = tid; s < n; s += T) {
+    uint32_t q[4];
+    for (uint32_t m = 0; m < 4; ++m) {
+      const uint2 ce = J.F.ent[4 * s + m];
+      q[m] = ce.x | (ce.y >> 31 << 15);
+    }
+    nb[s] = make_uint2(q[0] | (q[1] << 16), q[2] | (q[3] << 16));
+  }
+  uint32_t* const jw = rows_at<uint32_t>(X.jw);
+  const uint32_t inv = X.inv;
+  for (uint32_t x = tid; x < 2 * L; x += T) {  // bond signs of row x % L, to the right or down
+    const uint32_t r = x % L, down = x / L;
+    uint32_t v = 0;
+    for (uint32_t k = 0; k < L; ++k) {
+      const uint32_t s = rows_site(r * L + k, L, inv, n / 2);
+      const uint32_t to = rows_site(down ? (r + 1) % L * L + k : r * L + (k + 1) % L, L, inv, n / 2);
+      for (uint32_t m = 0; m < 4; ++m) {
+        const uint2 ce = J.F.ent[4 * s + m];
+        if (ce.x == to) v |= (ce.y >> 31) << k;
+      }
+    }
+    jw[32 * down + r] = v;
+  }
+  if (J.init == 1) {
+    for (uint32_t x = tid; x < n * nw; x += T) {
+      const uint32_t s = x / nw, wo = x % nw, ch = wo / J.wpc, w = wo % J.wpc;
+      uint32_t v = 0;
+      for (uint32_t qq = 0; qq < 8 && 8 * w + qq < J.qpc; ++qq)
+        v |= init_nibble(philox4x32_10(make_uint4(s, 0xffffffffu, ch * 16u + 8 * w + qq, PTAG_INIT), J.key)) << (4 * qq);
+      W[x] = v;
+    }
+  } else {
+    for (uint32_t x = tid; x < n * nw; x += T) W[x] = J.W[x];
+  }
+  for (uint32_t x = tid; x < J.C * J.ntp; x += T) rows_at<int>(X.E)[x] = 0;  // (slots from nt on)
+  xchg_load(J, rows_at<char>(X.xb));
+  // two words at once where that takes fewer steps of the warps
+  const uint32_t ch = (n / 2 + 31) / 32;
+  const bool two = nw % 2 == 0 && (ch * nw / 2 + nwarp - 1) / nwarp < (ch * nw + nwarp - 1) / nwarp;
+  uint32_t m_cur = J.m_base, s_cur = J.s_base;
+  PhaseClock pc;
+  pc.start(J.prof);
+  rows_energies(J.sweep_begin, J.icm && J.sweep_begin < J.sweep_end, pc);
+  for (uint32_t i = J.sweep_begin; i < J.sweep_end; ++i) {
+    rows_exchange(i, pc);
+    if (two) rows_sweep<2>(i);
+    else rows_sweep<1>(i);
+    pc.lap(PHASE_SWEEP);
+    rows_energies(i + 1, J.icm && i + 1 < J.sweep_end, pc);
+    if (i >= J.meas_init) rows_measure(i, m_cur, s_cur);
+    pc.lap(PHASE_MEASURE);
+  }
+  for (uint32_t x = tid; x < n * nw; x += T) J.W[x] = W[x];
+  for (uint32_t x = tid; x < J.C * J.ntp; x += T) J.Ec[x] = J.Er[x] = rows_at<const int>(X.E)[x];
+  xchg_store(J, rows_at<char>(X.xb));
+}
+__device__ __noinline__ void run_rows_call() { run_rows(); }
+
+// A launch of lattice-row jobs only: without the other jobs' code a thread takes
+// half the registers, and an SM twice the CTAs.
+__global__ void __launch_bounds__(1024, 1) k_pt_rows(const PtJob* __restrict__ jobs, uint32_t njobs, uint32_t* ctr) {
+  __shared__ uint32_t s_job;
+  for (;;) {
+    if (threadIdx.x == 0) s_job = atomicAdd(ctr, 1u);
+    __syncthreads();
+    const uint32_t jid = s_job;
+    __syncthreads();
+    if (jid >= njobs) break;
+    load_job(rows_job(), jobs + jid);
+    run_rows();
+  }
+}
+
 __global__ void __launch_bounds__(512, 1) k_pt_fused(const PtJob* __restrict__ jobs, uint32_t njobs, uint32_t* ctr) {
   extern __shared__ uint4 smem_u4[];
   __shared__ uint32_t s_job;
-  __shared__ PtJob s_J;
+  PtJob& s_J = rows_job();
   for (;;) {
     if (threadIdx.x == 0) s_job = atomicAdd(ctr, 1u);
     __syncthreads();
@@ -1635,7 +2274,8 @@ __global__ void __launch_bounds__(512, 1) k_pt_fused(const PtJob* __restrict__ j
     __syncthreads();
     if (jid >= njobs) break;
     load_job(s_J, jobs + jid);
-    if (s_J.self_loops) run_job<true>(s_J, reinterpret_cast<char*>(smem_u4));
+    if (s_J.rows) run_rows_call();
+    else if (s_J.self_loops) run_job<true>(s_J, reinterpret_cast<char*>(smem_u4));
     else run_job<false>(s_J, reinterpret_cast<char*>(smem_u4));
   }
 }
@@ -2801,30 +3441,37 @@ __global__ void k_plain_energy(const PtJob* __restrict__ jp, long long* acc) {
 
 }  // namespace
 
+bool fused_rows(const PtJob& j) {
+  if (const char* e = getenv("TAMC_PT_ROWS"))
+    if (e[0] == '0') return false;
+  return j.msc && j.F.cb_L && j.F.offset == 0.0f;
+}
+
 size_t fused_smem_bytes(const PtJob& j, uint32_t T, bool csr_smem) {
+  if (j.rows) return rows_carve(j.n, j.nw, j.wpc, j.C, j.ntp, j.F.cb_L).bytes;
   if (!j.icm_uf && j.n > 65536) return SIZE_MAX;  // the multi-slot search keeps 16-bit site lists
   return carve_all(nullptr, nullptr, j.n, j.nw, j.C, j.ntp, j.qps, T, j.F.nnz, csr_smem, j.icm_group, j.icm_uf != 0);
 }
 
-// The fused kernel's dynamic shared-memory limit only grows (per device), so
+// The fused kernels' dynamic shared-memory limits only grow (per device), so
 // that a captured launch stays valid whatever smaller launches ran since.
-static void fused_attr(size_t smem) {
+static void fused_attr(size_t smem, bool rows) {
   static std::mutex mu;
-  static std::map<int, size_t> set;
+  static std::map<std::pair<int, bool>, size_t> set;
   int dev = 0;
   TAMC_CUDA(cudaGetDevice(&dev));
   std::lock_guard<std::mutex> lk(mu);
-  size_t& cur = set[dev];
+  size_t& cur = set[{dev, rows}];
   if (smem > cur) {
-    TAMC_CUDA(cudaFuncSetAttribute(k_pt_fused, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    TAMC_CUDA(cudaFuncSetAttribute(rows ? k_pt_rows : k_pt_fused, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     cur = smem;
   }
 }
 
-int fused_blocks_per_sm(uint32_t T, size_t smem) {
-  fused_attr(smem);
+int fused_blocks_per_sm(uint32_t T, size_t smem, bool rows) {
+  fused_attr(smem, rows);
   int nb = 0;
-  TAMC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_pt_fused, (int)T, smem));
+  TAMC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, rows ? k_pt_rows : k_pt_fused, (int)T, smem));
   return nb;
 }
 
@@ -3071,14 +3718,15 @@ void plain_launch_init(cudaStream_t st, const PtJob* d_job, long long* acc, int 
 }
 
 void fused_launch(cudaStream_t st, const PtJob* d_jobs, uint32_t njobs, uint32_t* ctr, uint32_t grid, uint32_t T,
-                  size_t smem) {
-  fused_attr(smem);
-  k_pt_fused<<<grid, T, smem, st>>>(d_jobs, njobs, ctr);
+                  size_t smem, bool rows) {
+  fused_attr(smem, rows);
+  if (rows) k_pt_rows<<<grid, T, smem, st>>>(d_jobs, njobs, ctr);
+  else k_pt_fused<<<grid, T, smem, st>>>(d_jobs, njobs, ctr);
   TAMC_CUDA(cudaGetLastError());
 }
 
 void fused_launch_prio(cudaStream_t st, const PtJob* d_jobs, uint32_t njobs, uint32_t* ctr, uint32_t grid, uint32_t T,
-                       size_t smem, int priority) {
+                       size_t smem, int priority, bool rows) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(T);
@@ -3089,9 +3737,9 @@ void fused_launch_prio(cudaStream_t st, const PtJob* d_jobs, uint32_t njobs, uin
   at[0].val.priority = priority;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  TAMC_CUDA(cudaLaunchKernelEx(&cfg, k_pt_fused, d_jobs, njobs, ctr));
+  TAMC_CUDA(cudaLaunchKernelEx(&cfg, rows ? k_pt_rows : k_pt_fused, d_jobs, njobs, ctr));
 }
 
-void fused_smem_limit(size_t smem) { fused_attr(smem); }
+void fused_smem_limit(size_t smem, bool rows) { fused_attr(smem, rows); }
 
 }  // namespace tamc

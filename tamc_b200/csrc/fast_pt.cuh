@@ -34,7 +34,7 @@ struct PtJob {
   unsigned long long* prof;  // if set: per-phase clock64 cycles (PHASE_* order), off otherwise
   uint64_t cost;       // sweeps * n * R, for longest-first ordering
   int32_t msc;         // multi-spin-coded sweep (+-J instance, nw in {1, 2, 4})
-  int32_t pad_;
+  int32_t rows;        // fused form: Houdayer moves on lattice rows (run_rows; multi-spin-coded checkerboard lattice)
 };
 
 enum { PHASE_ICM_SCAN, PHASE_ICM_INIT, PHASE_ICM_JUMP, PHASE_ICM_GROW, PHASE_ICM_MARK, PHASE_ICM_APPLY, PHASE_EXCH,
@@ -43,19 +43,22 @@ enum { PHASE_ICM_SCAN, PHASE_ICM_INIT, PHASE_ICM_JUMP, PHASE_ICM_GROW, PHASE_ICM
        // levels, flip decisions, energy sums and stores, barrier waits
        PHASE_SW_LEVELS, PHASE_SW_FLIP, PHASE_SW_ENERGY, PHASE_SW_WAIT, PHASE_N };
 
+// Whether the fused kernel runs the job on lattice rows (PtJob::rows).
+bool fused_rows(const PtJob& j);
 // Shared-memory bytes the fused kernel needs for a job with T threads.
 size_t fused_smem_bytes(const PtJob& j, uint32_t T, bool csr_smem);
-// Resident CTAs per SM for the fused kernel at this size.
-int fused_blocks_per_sm(uint32_t T, size_t smem);
+// Resident CTAs per SM for the fused kernel at this size (`rows`, here and
+// below: the kernel of launches whose jobs are all on lattice rows).
+int fused_blocks_per_sm(uint32_t T, size_t smem, bool rows);
 // Launch over `njobs` jobs already on the device; `ctr` is a zeroed counter.
 void fused_launch(cudaStream_t st, const PtJob* d_jobs, uint32_t njobs, uint32_t* ctr, uint32_t grid,
-                  uint32_t T, size_t smem);
+                  uint32_t T, size_t smem, bool rows);
 // A fused launch with a launch priority (cudaLaunchAttributePriority; lower
 // numbers run first); the shared-memory attribute must already cover `smem`
 // (fused_smem_limit).
 void fused_launch_prio(cudaStream_t st, const PtJob* d_jobs, uint32_t njobs, uint32_t* ctr, uint32_t grid, uint32_t T,
-                       size_t smem, int priority);
-void fused_smem_limit(size_t smem);
+                       size_t smem, int priority, bool rows);
+void fused_smem_limit(size_t smem, bool rows);
 
 // Plain form (one instance over the whole GPU, one launch per sweep phase).
 struct PlainCtl {

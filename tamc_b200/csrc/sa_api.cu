@@ -39,6 +39,7 @@ FastInst make_fast_inst(const tamc_inst* d) {
   F.pmj = d->pmj;
   F.lat_L = d->lat_L;
   F.lat_any = d->lat_any;
+  F.cb_L = d->cb_L;
   F.sl_n = d->sl_n;
   F.sl_rows = d->sl_rows;
   F.sl_cls = d->d_sl_cls;
