@@ -141,8 +141,8 @@ thread_local bool g_no_autotune = false;
 thread_local bool g_defer_init = false;
 
 // On lattice rows: 256 threads up to 256 sites, else 512 (microseconds a round,
-// 2 x 32 replicas: 16 x 16 sites 9.1 at 128 threads, 6.5 at 256, 6.3 at 512;
-// 32 x 32 sites 22.2, 13.3, 10.2, and 10.7 at 1024).
+// 2 x 32 replicas: 16 x 16 sites 8.5 at 128 threads, 6.0 at 256, 5.8 at 512;
+// 32 x 32 sites 20.0, 12.1, 9.4).
 static TileChoice rows_tile(const PtJob& j) { return TileChoice{j.n > 256 ? 512u : 256u, false}; }
 
 static TileChoice tune_tile(tamc_gpu* g, const PtJob& j) {
@@ -378,9 +378,10 @@ static std::map<std::tuple<int, uint32_t, uint32_t, uint32_t, uint32_t, int>, bo
 
 // Runs on lattice rows of at most 2048 words take neither the plain nor the
 // ladder form (microseconds a round on rows / in the ladder form, 8 to 32
-// temperatures: 2 chains on 8 x 8 sites 5.0-5.1 / 9.6-10.6, 16 x 16 5.6-6.4 /
-// 10.9-11.9, 32 x 32 8.8-10.1 / 13.8-15.0; 4 chains on 16 x 16 9.3-10.7 /
-// 11.5-12.2; above, 4 chains on 24 x 24 13.9-16.2 / 13.4-14.1).
+// temperatures: 2 chains on 8 x 8 sites 4.5-4.8 / 9.6-10.6, 16 x 16 5.2-6.0 /
+// 10.9-12.2, 32 x 32 8.0-9.3 / 13.8-14.6; 4 chains on 16 x 16 8.7-10.0 /
+// 11.6-12.2; above, 4 chains on 24 x 24 12.5-14.7 / 13.3-14.1, on 32 x 32
+// 14.9-17.1 / 14.4-15.2).
 static bool rows_first(const PtJob& j) { return j.rows && j.n * j.nw <= 2048; }
 
 static bool choose_plain(tamc_pt* pt) {
@@ -989,8 +990,8 @@ struct ChunkRunner {
       // on C3 that measured 27.6 ms per 1000 sweeps against 35.0 ms at the
       // small runs' own autotuned 256 threads (two per SM), which time one
       // run alone on an otherwise idle SM
-      // (all on lattice rows, whose kernel takes half the registers: 256 measured
-      // 11.7 ms against 12.1 at 128, with one class of 512 threads 15.8)
+      // (all on lattice rows, whose kernel takes fewer registers: 256 measured
+      // 11.0 ms against 11.6 at 128)
       std::vector<tamc_pt*> big, small;
       // (`by_size`: runs of at most 512 sites also go to the small class
       // whatever their tile, so that a batch built with heuristic tiles, all

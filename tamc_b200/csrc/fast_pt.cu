@@ -1001,12 +1001,6 @@ __device__ __forceinline__ uint64_t exchange_bits(const PtJob& J, uint32_t c, ui
     }
     D = (uint64_t)__ballot_sync(0xffffffffu, d[0]) | ((uint64_t)__ballot_sync(0xffffffffu, d[1]) << 32);
   } else {
-    // Serial semantics: pair j sees ΔE_j plus the carried ΔE_{j-1} when pair
-    // j - 1 swapped (tamc-core/src/pt.rs:138-141).  The draws, Δβ, ΔE_j and
-    // the decisions without a carry do not depend on earlier pairs, so lane
-    // j % 32 computes them for pair j in parallel; the walk over the pairs
-    // then redoes only the decisions whose lower pair swapped, with the same
-    // float operations as a plain sequential loop (same decisions).
     float des0[2], db[2], u[2];
     bool d0[2];
     for (int h = 0; h < 2; ++h) {
@@ -1023,28 +1017,7 @@ __device__ __forceinline__ uint64_t exchange_bits(const PtJob& J, uint32_t c, ui
         d0[h] = dlt >= 0.0f || u[h] < __expf(dlt);
       }
     }
-    const uint64_t D0 =
-        (uint64_t)__ballot_sync(0xffffffffu, d0[0]) | ((uint64_t)__ballot_sync(0xffffffffu, d0[1]) << 32);
-    float carry = 0.0f;
-    bool prev = false;
-    for (uint32_t j = 0; j + 1 < nt; ++j) {  // warp-uniform: every lane walks the same values
-      const bool hi = j >= 32u;
-      const float e = __shfl_sync(0xffffffffu, hi ? des0[1] : des0[0], j & 31u);
-      const float b = __shfl_sync(0xffffffffu, hi ? db[1] : db[0], j & 31u);
-      const float uj = __shfl_sync(0xffffffffu, hi ? u[1] : u[0], j & 31u);
-      float des = e;
-      bool dj;
-      if (prev) {
-        des = e + carry;
-        const float dlt = b * des;
-        dj = dlt >= 0.0f || uj < __expf(dlt);
-      } else {
-        dj = (D0 >> j) & 1ull;
-      }
-      if (dj) D |= 1ull << j;
-      prev = dj;
-      carry = des;
-    }
+    D = serial_swaps(nt, des0, db, u, d0);
   }
   return D;
 }
@@ -1657,7 +1630,7 @@ __device__ void run_job(const PtJob& J, char* smem_base) {
 // satisfied bonds: integers well below 2^24, so the same floats and doubles as
 // the sums of the changes.
 // (32 x 32 sites, 2 x 32 replicas, 512 threads, a round: 24.2 us on the general
-// path, 10.1 here; 8 x 8 sites, 12.1 and 5.1.)
+// path, 9.4 here; 8 x 8 sites, 12.1 and 4.8.)
 struct RowsSm {  // byte offsets (from pointers kept in a struct the compiler makes generic loads)
   uint32_t W, msc, Ec, E, Em, Dm, nb, sw, jw, bits, red, xb, bytes;
   uint32_t inv;  // ceil(2^16 / L)
@@ -1696,8 +1669,8 @@ __host__ __device__ inline RowsSm rows_carve(uint32_t n, uint32_t nw, uint32_t w
   return X;
 }
 
-// The job and the offsets, in shared memory (they would take 20 registers of the
-// 64, and through a reference parameter their loads would be generic).
+// The job and the offsets, in shared memory (they would take 20 registers,
+// and through a reference parameter their loads would be generic).
 __device__ __forceinline__ PtJob& rows_job() {
   __shared__ PtJob J;
   return J;
@@ -1846,9 +1819,10 @@ __device__ __forceinline__ void rows_slots(uint32_t i, bool move) {
             if (k >= excl && k < excl + mine) cl = 1u << nth_bit(d & (odd ? ~even : even), k - excl);
           }
           // growth by whole runs of the columns (log2 LW steps of twice the length
-          // each, both ways at once), then of the rows; a step that is not the last
-          // adds a site, so they end within 32 n.  (On a cluster of the 32 x 32
-          // lattice 4 such steps, where one row up and down at a time took 18.)
+          // each, both ways at once), then of the rows, until the rows add nothing;
+          // every other step adds a site, so they end within 32 n.  (On a cluster of
+          // the 32 x 32 lattice 4 such steps, where one row up and down at a time
+          // took 18.)
           uint32_t dn[LOG], upw[LOG];  // columns disagreeing from this row over 2^k rows
           dn[0] = upw[0] = d;
 #pragma unroll
@@ -1857,7 +1831,6 @@ __device__ __forceinline__ void rows_slots(uint32_t i, bool move) {
             upw[k] = upw[k - 1] & from(upw[k - 1], 1 << (k - 1));
           }
           for (uint32_t step = 0; step < 32u * 1024u; ++step) {
-            const uint32_t before = cl;
             uint32_t a = cl, b = cl;
 #pragma unroll
             for (int k = 0; k < LOG; ++k) {
@@ -1866,7 +1839,7 @@ __device__ __forceinline__ void rows_slots(uint32_t i, bool move) {
             }
             a |= b;
             cl = run_fill(a | (d & ((a << up) | (a >> up))), d);
-            if (!__any_sync(0xffffffffu, cl != before)) break;
+            if (!__any_sync(0xffffffffu, cl != a)) break;
           }
           // the bonds across the cluster's boundary change sides
           const uint32_t c_dn = from(cl, 1);
@@ -2248,9 +2221,11 @@ __device__ __forceinline__ void run_rows() {
 }
 __device__ __noinline__ void run_rows_call() { run_rows(); }
 
-// A launch of lattice-row jobs only: without the other jobs' code a thread takes
-// half the registers, and an SM twice the CTAs.
-__global__ void __launch_bounds__(1024, 1) k_pt_rows(const PtJob* __restrict__ jobs, uint32_t njobs, uint32_t* ctr) {
+// A launch of lattice-row jobs only.  Without the other jobs' code 80 registers a
+// thread do, so that a run of 512 threads leaves room for one of 256 on its SM
+// (256 uneven runs x 5000 rounds: 58 ms with 64 registers, 55 with 80, 62 with 96
+// and with 128, where it does not).
+__global__ void __launch_bounds__(768, 1) k_pt_rows(const PtJob* __restrict__ jobs, uint32_t njobs, uint32_t* ctr) {
   __shared__ uint32_t s_job;
   for (;;) {
     if (threadIdx.x == 0) s_job = atomicAdd(ctr, 1u);

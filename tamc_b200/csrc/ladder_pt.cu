@@ -103,7 +103,7 @@ struct LadSm {
   uint32_t flat;   // lattices: [nwb + 1] a bitmap in file order
   uint32_t perm, iperm;  // lattices: [n] u16 colour -> file order and back
   uint32_t coff;   // [ncolors + 1] first site of each colour class (sliced rows: first slice)
-  uint32_t ex;     // [3][64] f32 exchange: energy differences, beta differences, uniforms
+  uint32_t ex;     // [2][64] f32 exchange: beta differences, uniforms
   uint32_t E;      // [64][2] f64 the chain's energies at the exchange (cached, energy_ref)
   uint32_t red;    // [32][2] i64
   uint32_t tags;   // [nt] bytes: bookkeeping of the chain (slot 0's CTA)
@@ -139,7 +139,7 @@ __host__ __device__ inline LadSm lad_carve(const LadDims d) {
   S.perm = take(d.lat_rows ? n * 2 : 0);
   S.iperm = take(d.lat_rows ? n * 2 : 0);
   S.coff = take((d.ncolors + 1) * 4);
-  S.ex = take(3 * 64 * 4);
+  S.ex = take(2 * 64 * 4);
   S.E = take(64 * 16);
   S.red = take(32 * 2 * 8);
   S.tags = take(d.nt);
@@ -631,14 +631,19 @@ __device__ __forceinline__ float lad_u24(uint32_t r) { return (float)(r >> 8) * 
 // Exchange decisions of a chain, by one warp: bit j of the result = the
 // replicas of slots j and j + 1 swap.  x = LadSm::ex (beta differences and
 // uniforms already there), pe = published energies of the chain, kept in E.
-__device__ unsigned long long lad_decide(bool threaded, uint32_t nt, float* x, const double* pe, double2* E,
+__device__ unsigned long long lad_decide(bool threaded, uint32_t nt, const float* x, const double* pe, double2* E,
                                          uint32_t lane) {
   bool d0[2];
   double2 e[2];
+  float des0[2] = {0.0f, 0.0f}, db[2] = {0.0f, 0.0f}, u[2] = {1.0f, 1.0f};
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     const uint32_t j = lane + 32u * h;
     e[h] = j < nt ? __ldcg(reinterpret_cast<const double2*>(pe) + j) : make_double2(0.0, 0.0);
+    if (j + 1 < nt) {
+      db[h] = x[j];
+      u[h] = x[64 + j];
+    }
   }
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
@@ -649,45 +654,13 @@ __device__ unsigned long long lad_decide(bool threaded, uint32_t nt, float* x, c
     if (j < nt) E[j] = e[h];
     d0[h] = false;
     if (j + 1 < nt) {
-      const float des = hi - lo;
-      const float dlt = x[64 + j] * des;
-      d0[h] = dlt >= 0.0f || x[128 + j] < __expf(dlt);
-      x[j] = des;
+      des0[h] = hi - lo;
+      const float dlt = db[h] * des0[h];
+      d0[h] = dlt >= 0.0f || u[h] < __expf(dlt);
     }
   }
-  const uint64_t D0 =
-      (uint64_t)__ballot_sync(0xffffffffu, d0[0]) | ((uint64_t)__ballot_sync(0xffffffffu, d0[1]) << 32);
-  __syncwarp();
-  if (threaded) return D0;
-  // serial semantics: a pair above a swap sees the carried energy difference, so
-  // only the pairs after each swap are decided again (every lane walks alike,
-  // the next pair's values loaded ahead)
-  uint64_t D = 0;
-  uint32_t j = 0;
-  while (j + 1 < nt) {
-    const uint64_t rem = D0 >> j;
-    if (!rem) break;
-    j += (uint32_t)__ffsll((long long)rem) - 1u;
-    D |= 1ull << j;
-    float carry = x[j];
-    ++j;
-    float de = x[j], db = x[64 + j], u = x[128 + j];
-    while (j + 1 < nt) {
-      const uint32_t k = min(j + 1, 63u);
-      const float de1 = x[k], db1 = x[64 + k], u1 = x[128 + k];
-      const float des = de + carry;
-      const float dlt = db * des;
-      if (!(dlt >= 0.0f || u < __expf(dlt))) break;
-      D |= 1ull << j;
-      carry = des;
-      ++j;
-      de = de1;
-      db = db1;
-      u = u1;
-    }
-    ++j;
-  }
-  return D;
+  if (!threaded) return serial_swaps(nt, des0, db, u, d0);
+  return (uint64_t)__ballot_sync(0xffffffffu, d0[0]) | ((uint64_t)__ballot_sync(0xffffffffu, d0[1]) << 32);
 }
 
 // The slot whose replica moves to slot t under the swaps D.
@@ -977,7 +950,7 @@ __device__ void lad_run(const LadJob& A) {
     lad_word(s) = (v >> (s & 31u)) << 31;
     if ((s & 31u) == 0) own[s >> 5] = v;
   }
-  for (uint32_t j = tid; j + 1 < nt; j += T) ex[64 + j] = J.betas[j + 1] - J.betas[j];
+  for (uint32_t j = tid; j + 1 < nt; j += T) ex[j] = J.betas[j + 1] - J.betas[j];
   if (tid == 0) {
     s_E[0] = J.Ec[c * J.ntp + t];
     s_E[1] = J.Er[c * J.ntp + t];
@@ -1045,7 +1018,7 @@ __device__ void lad_run(const LadJob& A) {
     // the exchange's uniforms while the stores drain
     if (r < nr && warp == nwarp - 1)
       for (uint32_t j = lane; j + 1 < nt; j += 32)
-        ex[128 + j] = lad_u24(philox4x32_10w(make_uint4(j, i, c, PTAG_EXCH), J.key).x);
+        ex[64 + j] = lad_u24(philox4x32_10w(make_uint4(j, i, c, PTAG_EXCH), J.key).x);
     pc.lap(PHASE_ICM_SCAN);
     if (!lad_barrier(A.bar, (r + 1) * A.ncta, A.polls, A.err, &misc[2])) return;
     pc.lap(PHASE_OTHER);
