@@ -318,7 +318,8 @@ __global__ void __launch_bounds__(1024) k_sa_tab(SaFastArgs a) {
 // words, couplings), else in L2.
 // Bound: the serial chain of loads and sums of a row.  (With k_sa_fast, whose
 // warps wait for their longest row, and here: 251 sites, 100 restarts, 200
-// sweeps 1586 us and 855; 8192 sites, 512 restarts, 100 sweeps 3282 us and 2197.)
+// sweeps 1584 us and 820; 8192 sites, 512 restarts, 100 sweeps 3282 us and 2162.
+// Fetching the next slice's entries ahead made the rows in L2 slower, 2180-3120.)
 struct SaSl {
   uint32_t W, site, soff, bias, colp, J, red, bytes;
 };
@@ -373,18 +374,27 @@ __global__ void __launch_bounds__(1024) k_sa_sl(SaFastArgs a) {
   const uint32_t first = warp / NQ, stride = (T >> 5) / NQ;
   const PhiloxKeys K = philox_schedule(a.key);
   Fx4 acc{0, 0, 0, 0};  // unused: SA energies are computed once at the end
+  const uint32_t* __restrict__ const cls = a.F.sl_cls;
   for (uint32_t sw = 0; sw < a.nbeta; ++sw) {
     const float b = a.betas[sw] * TAMC_2LOG2E;  // 2 beta log2(e)
     const float4 b2 = make_float4(b, b, b, b);
     for (uint32_t c = 0; c < a.F.ncolors; ++c) {
-      const uint32_t g1 = a.F.sl_cls[c + 1];
-      for (uint32_t g = a.F.sl_cls[c] + first; g < g1; g += stride) {
-        const uint32_t s = site[32 * g + lane];
-        if (s == 0xffffu) continue;  // beyond the class's last site
+      const uint32_t g1 = cls[c + 1];
+      for (uint32_t g = cls[c] + first; g < g1; g += stride) {
+        const uint32_t at = site[32 * g + lane];
+        const bool on = at != 0xffffu;  // else beyond the class's last site
+        const uint32_t s = on ? at : 0u;
         uint32_t x = soff[g], w = soff[g + 1] - x;
         x = 32 * x + lane;
         const float h = bias[s];
         float4 f = make_float4(h, h, h, h);
+        auto add = [&](uint32_t j, uint32_t v) {
+          f.x += __uint_as_float(j ^ (v << 31));
+          f.y += __uint_as_float(j ^ ((v << 30) & 0x80000000u));
+          f.z += __uint_as_float(j ^ ((v << 29) & 0x80000000u));
+          f.w += __uint_as_float(j ^ ((v << 28) & 0x80000000u));
+        };
+        auto spin = [&](uint32_t c4) { return *reinterpret_cast<const uint32_t*>(sa_smem + c4) >> shift; };
         auto entries = [&](auto count) {
           constexpr uint32_t N = decltype(count)::value;
           uint32_t c4[N], j[N], v[N];
@@ -400,14 +410,9 @@ __global__ void __launch_bounds__(1024) k_sa_sl(SaFastArgs a) {
             }
           }
 #pragma unroll
-          for (uint32_t m = 0; m < N; ++m) v[m] = *reinterpret_cast<const uint32_t*>(sa_smem + c4[m]) >> shift;
+          for (uint32_t m = 0; m < N; ++m) v[m] = spin(c4[m]);
 #pragma unroll
-          for (uint32_t m = 0; m < N; ++m) {
-            f.x += __uint_as_float(j[m] ^ (v[m] << 31));
-            f.y += __uint_as_float(j[m] ^ ((v[m] << 30) & 0x80000000u));
-            f.z += __uint_as_float(j[m] ^ ((v[m] << 29) & 0x80000000u));
-            f.w += __uint_as_float(j[m] ^ ((v[m] << 28) & 0x80000000u));
-          }
+          for (uint32_t m = 0; m < N; ++m) add(j[m], v[m]);
           x += 32 * N;
         };
 #pragma unroll 1
@@ -415,9 +420,12 @@ __global__ void __launch_bounds__(1024) k_sa_sl(SaFastArgs a) {
         if (w & 4u) entries(std::integral_constant<uint32_t, 4>());
         if (w & 2u) entries(std::integral_constant<uint32_t, 2>());
         const uint4 rnd = philox4x32_10(make_uint4(s, sw, qid, PTAG_SWEEP), K);
-        const uint32_t m = quad_accept<false>(f, W[s] >> shift, b2, rnd, acc);
-        if (NQ == 1) W[s] ^= m;
-        else if (m) atomicXor(&W[s], m << shift);
+        const uint32_t m = on ? quad_accept<false>(f, W[s] >> shift, b2, rnd, acc) : 0u;
+        if (NQ == 1) {
+          if (on) W[s] ^= m;
+        } else if (m) {
+          atomicXor(&W[s], m << shift);
+        }
       }
       __syncthreads();
     }
