@@ -443,7 +443,7 @@ def run_c3(args):
                "gpu_launches": int(launches),
                "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                             "frac": achieved / peak, "traffic": traffic, "peak_kind": f"{kind} burst",
-                            "bytes_per_step": bytes_step, "kernel": "k_pt_fused (one per chunk launch)",
+                            "bytes_per_step": bytes_step, "kernel": "k_pt_rows (one per chunk launch)",
                             "launch_ms_avg": dev_ms / max(1, nlaunch), "launches_per_step": nlaunch / args.steps},
                "issue_roofline": issue,
                "clocks": clocks, "best_energy_jobs_0_3": best}
