@@ -318,10 +318,10 @@ __global__ void __launch_bounds__(1024) k_sa_tab(SaFastArgs a) {
 // words, couplings), else in L2.
 // Bound: the serial chain of loads and sums of a row.  (With k_sa_fast, whose
 // warps wait for their longest row, and here: 251 sites, 100 restarts, 200
-// sweeps 1584 us and 820; 8192 sites, 512 restarts, 100 sweeps 3282 us and 2162.
-// Fetching the next slice's entries ahead made the rows in L2 slower, 2180-3120.)
+// sweeps 1584 us and 820; 8192 sites, 512 restarts, 100 sweeps 3282 us and 2003.
+// Fetching the next slice's entries ahead made the rows in L2 slower, 2120-2280.)
 struct SaSl {
-  uint32_t W, site, soff, bias, colp, J, red, bytes;
+  uint32_t W, site, soff, cls, bias, colp, J, red, bytes;
 };
 __host__ __device__ inline SaSl sa_sl_carve(const FastInst& F, bool cs, uint32_t nq, uint32_t T) {
   uint32_t o = 0;
@@ -335,6 +335,7 @@ __host__ __device__ inline SaSl sa_sl_carve(const FastInst& F, bool cs, uint32_t
   S.site = take(F.sl_n * 64);
   S.soff = take((F.sl_n + 1) * 4);
   S.bias = take(F.n * 4);
+  if (!cs) S.cls = take((F.ncolors + 1) * 4);
   if (cs) {
     S.colp = take(F.sl_rows * 64);
     S.J = take(F.sl_rows * 128);
@@ -359,6 +360,8 @@ __global__ void __launch_bounds__(1024) k_sa_sl(SaFastArgs a) {
   const uint32_t r0 = blockIdx.x * 4 * NQ;
   for (uint32_t x = tid; x < 32 * a.F.sl_n; x += T) site[x] = a.F.sl_site[x];
   for (uint32_t x = tid; x <= a.F.sl_n; x += T) soff[x] = a.F.sl_off[x];
+  if (!CS)
+    for (uint32_t x = tid; x <= a.F.ncolors; x += T) reinterpret_cast<uint32_t*>(sa_smem + S.cls)[x] = a.F.sl_cls[x];
   if (CS)
     for (uint32_t x = tid; x < 32 * a.F.sl_rows; x += T) {
       const uint2 v = ent[x];
@@ -374,13 +377,18 @@ __global__ void __launch_bounds__(1024) k_sa_sl(SaFastArgs a) {
   const uint32_t first = warp / NQ, stride = (T >> 5) / NQ;
   const PhiloxKeys K = philox_schedule(a.key);
   Fx4 acc{0, 0, 0, 0};  // unused: SA energies are computed once at the end
-  const uint32_t* __restrict__ const cls = a.F.sl_cls;
+  // rows from L2 leave nothing else in L1, so that the classes' bounds are in shared
+  // memory with them (8192 sites, 512 restarts, 100 sweeps: 2147 -> 2003 us); with
+  // the rows in shared memory L1 keeps them (251 sites: 819 us, 833 with a copy)
+  const uint32_t* __restrict__ const cls_g = a.F.sl_cls;
+  const uint32_t* const cls_s = reinterpret_cast<const uint32_t*>(sa_smem + S.cls);
+  auto cls = [&](uint32_t c) { return CS ? cls_g[c] : cls_s[c]; };
   for (uint32_t sw = 0; sw < a.nbeta; ++sw) {
     const float b = a.betas[sw] * TAMC_2LOG2E;  // 2 beta log2(e)
     const float4 b2 = make_float4(b, b, b, b);
     for (uint32_t c = 0; c < a.F.ncolors; ++c) {
-      const uint32_t g1 = cls[c + 1];
-      for (uint32_t g = cls[c] + first; g < g1; g += stride) {
+      const uint32_t g1 = cls(c + 1);
+      for (uint32_t g = cls(c) + first; g < g1; g += stride) {
         const uint32_t at = site[32 * g + lane];
         const bool on = at != 0xffffu;  // else beyond the class's last site
         const uint32_t s = on ? at : 0u;
