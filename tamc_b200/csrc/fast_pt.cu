@@ -24,6 +24,8 @@
 //  3. One Metropolis sweep of all replicas in colour order (see fast_common.cuh).
 //  4. Ground-state tracking and, on the reference's schedule, e/q/suscept
 //     measurements and bit-packed state snapshots (src/pt.rs:167-226, 542-583).
+//
+// +-J square lattices run the same rounds on lattice rows (run_rows, k_pt_rows).
 #include "fast_pt.cuh"
 
 #include <cooperative_groups.h>
