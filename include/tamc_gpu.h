@@ -162,7 +162,7 @@ int tamc_gpu_instance_upload_many(tamc_gpu* g, uint32_t count, const tamc_host_i
 int tamc_gpu_instance_destroy(tamc_inst* d);
 
 /* ------------------------------------------------------------------------
- * PT-ICM, plain form: one instance, one launch per sweep phase.
+ * PT-ICM, one instance.
  * Replaces PtIcmRunner::{run, run_parallel, pt_loop, parallel_pt_loop}
  * (src/pt.rs:354-504) below run_parallel_tempering (src/pt.rs:609-655).
  * ---------------------------------------------------------------------- */

@@ -421,7 +421,7 @@ class ThermalSamples:
 
 
 class PtRun:
-    """One PT-ICM run on the device (plain form: tamc_gpu_pt_*)."""
+    """One PT-ICM run on the device (tamc_gpu_pt_*)."""
 
     def __init__(self, dinst: DeviceInstance, params: PtParams, seed: int, mode: int = MODE_FAST):
         self.dinst, self.params, self.mode = dinst, params, mode

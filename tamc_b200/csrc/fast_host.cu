@@ -142,8 +142,12 @@ thread_local bool g_defer_init = false;
 
 // On lattice rows: 256 threads up to 256 sites, else 512 (microseconds a round,
 // 2 x 32 replicas: 16 x 16 sites 8.5 at 128 threads, 6.0 at 256, 5.8 at 512;
-// 32 x 32 sites 20.0, 12.1, 9.4).
-static TileChoice rows_tile(const PtJob& j) { return TileChoice{j.n > 256 ? 512u : 256u, false}; }
+// 32 x 32 sites 20.0, 12.1, 9.4).  A run alone, which shares its SM with no
+// other, takes 512 from 100 sites on.
+static TileChoice rows_tile(const PtJob& j) {
+  const bool alone = !g_defer_init && !g_no_autotune;
+  return TileChoice{j.n > (alone ? 100u : 256u) ? 512u : 256u, false};
+}
 
 static TileChoice tune_tile(tamc_gpu* g, const PtJob& j) {
   if (j.rows) return rows_tile(j);
