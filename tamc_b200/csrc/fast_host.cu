@@ -441,7 +441,6 @@ static bool choose_plain(tamc_pt* pt) {
     scratch.fast = nullptr;
     plain = ms_plain < ms_fused;
   }
-  if (getenv("TAMC_DEBUG")) fprintf(stderr, "[tamc] PT form n=%u nt=%u C=%u: %s\n", j.n, j.nt, j.C, plain ? "plain" : "fused");
   std::lock_guard<std::mutex> lk(g_tune_mu);
   g_form[key] = plain;
   return plain;
@@ -498,9 +497,6 @@ static bool ladder_setup(tamc_pt* pt) {
       F->lad.err = pt->out.err_flag();
       F->d_lad.alloc(1);
       F->ladder = true;
-      if (getenv("TAMC_DEBUG"))
-        fprintf(stderr, "[tamc] PT form n=%u nt=%u C=%u: ladder, %u CTAs of %u threads, rows in smem %d\n", j.n, j.nt,
-                j.C, F->lad.ncta, T, rows);
       return true;
     }
   return false;
@@ -531,6 +527,7 @@ static void ladder_rounds(tamc_pt* pt, uint32_t begin, uint32_t end, int init) {
 static void ladder_leave(tamc_pt* pt) {
   auto* F = pt->fast;
   cudaStream_t st = pt->g->stream;
+  if (getenv("TAMC_DEBUG")) fprintf(stderr, "[tamc] ladder rounds given up: 1 run(s)\n");
   F->ladder = false;
   if (fused_smem_bytes(F->job, 128, false) <= pt->g->smem_optin) {
     fused_setup(pt);
@@ -559,17 +556,20 @@ static void init_state(tamc_pt* pt, int init) {
 void fast_pt_create(tamc_pt* pt, uint64_t seed) {
   pt->fast = new tamc_pt::FastState();
   fill_job(pt, seed, pt->fast);
-  if (ladder_setup(pt)) {  // the initial replicas are drawn with the first rounds
-    pt->fast->init_pending = true;
-    return;
-  }
-  if (choose_plain(pt)) {
+  auto* F = pt->fast;
+  const PtJob& j = F->job;
+  if (ladder_setup(pt)) {
+    F->init_pending = true;  // random initial replicas: drawn by the first launch
+  } else if (choose_plain(pt)) {
     plain_setup(pt);
     plain_init_energies(pt, true);
-    return;
+  } else {
+    fused_setup(pt);
+    F->init_pending = true;
   }
-  fused_setup(pt);
-  pt->fast->init_pending = true;  // random initial replicas: drawn by the first launch
+  if (getenv("TAMC_DEBUG"))
+    fprintf(stderr, "[tamc] PT run n=%u nt=%u C=%u: %s, threads=%u smem=%zu\n", j.n, j.nt, j.C,
+            F->ladder ? "ladder" : F->plain ? "plain" : j.rows ? "rows" : "fused", F->T, F->smem);
 }
 
 // Deferred initial replicas, when something reads or runs the run before its
@@ -1347,6 +1347,8 @@ struct ChunkRunner {
       if (sl.h_counts[x]) pt->out.drain(st);
       else pt->out.pending = 0;
     }
+    if (!again.empty() && getenv("TAMC_DEBUG"))
+      fprintf(stderr, "[tamc] ladder rounds given up: %zu run(s)\n", again.size());
     if (!again.empty() && enqueue(g, slots[0], std::move(again), 0, false, false, false, &again_ends))
       finish(g, slots[0], false, 1);
   }

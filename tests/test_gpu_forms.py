@@ -1,0 +1,121 @@
+"""Which form of a PT-ICM run and which annealing kernel the comparisons of the
+other test files reach, from the lines that TAMC_DEBUG=1 prints: a dispatch rule
+that sent them elsewhere would leave those comparing a kernel with itself."""
+import re
+
+import numpy as np
+import pytest
+
+import test_gpu_ladder as ladder
+import test_gpu_rows as rows
+import test_gpu_sa_kernels as sa
+from tamc_b200 import instances as gi
+
+pytestmark = pytest.mark.gpu
+
+
+def _cases(test):
+    """The parameter sets of a test of another file."""
+    return [m for m in test.pytestmark if m.name == "parametrize"][0].args[1]
+
+
+def _printed(capfd, pattern):
+    return re.findall(pattern, capfd.readouterr().err)
+
+
+def _forms(capfd):
+    return _printed(capfd, r"\[tamc\] PT run .*: (\w+),")
+
+
+@pytest.fixture(autouse=True)
+def _debug(monkeypatch):
+    monkeypatch.setenv("TAMC_DEBUG", "1")
+    monkeypatch.setenv("TAMC_AUTOTUNE", "0")
+
+
+@pytest.mark.parametrize("kind,nt,C,threads,icm,level", _cases(ladder.test_ladder_and_fused_forms_identical))
+def test_form_of_the_ladder_cases(tb, gpu, monkeypatch, capfd, kind, nt, C, threads, icm, level):
+    d = gpu.upload(ladder._host(tb, kind))
+    b = tb.geometric_betas(0.2, 5.0, nt) if nt > 1 else np.array([0.9], np.float32)
+    p = tb.PtParams(60, b, nt // 2, 0.5, icm, C, threads, 7, 9, level)
+    for form in ("fused", "ladder"):
+        monkeypatch.setenv("TAMC_PT_FORM", form)
+        tb.PtRun(d, p, 77)
+    # 64 temperatures on 32 chains: 2048 CTAs of 128 threads are not resident at
+    # once (8 to an SM at 64 registers), so the ladder form does not take them
+    first, second = _forms(capfd)
+    assert first in ("fused", "rows")
+    assert (second == "ladder") == (nt * C <= 1184)
+
+
+@pytest.mark.parametrize("side,kind,nt", _cases(ladder.test_ladder_and_plain_forms_identical_on_large_lattices))
+def test_form_of_the_large_lattices(tb, gpu, monkeypatch, capfd, side, kind, nt):
+    d = gpu.upload(tb.HostInstance.parse(gi.lattice(side, 3, kind, 8)))
+    p = tb.PtParams(24, tb.geometric_betas(0.2, 5.0, nt), nt // 2, 0.5, True, 2, 8, 5, 5, 0)
+    for form in ("plain", "ladder"):
+        monkeypatch.setenv("TAMC_PT_FORM", form)
+        tb.PtRun(d, p, 5)
+    assert _forms(capfd) == ["plain", "ladder"]
+
+
+@pytest.mark.parametrize("side,dim,other", _cases(ladder.test_ladder_rounds_that_are_given_up_run_in_another_form))
+def test_rounds_are_given_up(tb, gpu, monkeypatch, capfd, side, dim, other):
+    d = gpu.upload(tb.HostInstance.parse(gi.lattice(side, dim, "gauss", 2)))
+    p = tb.PtParams(20, tb.geometric_betas(0.2, 5.0, 6), 3, 0.5, True, 2, 8, 5, 5, 0)
+    monkeypatch.setenv("TAMC_PT_FORM", "ladder")
+    monkeypatch.setenv("TAMC_LADDER_POLLS", "0")
+    tb.PtRun(d, p, 3).run().sync()
+    err = capfd.readouterr().err
+    assert re.findall(r"\[tamc\] PT run .*: (\w+),", err) == ["ladder"]
+    assert err.count("[tamc] ladder rounds given up: 1 run(s)") == 1
+
+
+@pytest.mark.parametrize("how", ["serve", "batch"])
+@pytest.mark.parametrize("polls", [None, "0"])
+def test_several_runs_take_the_ladder_form(tb, gpu, monkeypatch, capfd, how, polls):
+    kinds = ["qubo:61", "pm2:12", "gauss3:6", "qubo:300"]
+    monkeypatch.setenv("TAMC_PT_FORM", "ladder")
+    monkeypatch.setenv("TAMC_PT_T", "256")
+    if polls:
+        monkeypatch.setenv("TAMC_LADDER_POLLS", polls)
+    hosts = [ladder._host(tb, k) for k in kinds]
+    params = [tb.PtParams(70, tb.geometric_betas(0.2, 5.0, 12 + k), 5, 0.5, True, 2, 8) for k in range(len(kinds))]
+    if how == "serve":
+        srv = tb.Server(gpu, 8 << 30, 64, 25)
+        for k, (h, p) in enumerate(zip(hosts, params)):
+            srv.submit(h, p, 3 + k)
+        srv.step()
+    else:
+        b = tb.Batch(gpu)
+        for k, (d, p) in enumerate(zip(gpu.upload_many(hosts), params)):
+            b.add(d, p, 3 + k)
+        b.run()
+    err = capfd.readouterr().err
+    plans = re.findall(r"\[tamc\] plan for (\d+) runs: .* (\d+) in the ladder form", err)
+    assert plans[0] == ("4", "4")
+    given_up = re.findall(r"\[tamc\] ladder rounds given up: (\d+) run", err)
+    assert given_up[:1] == (["4"] if polls else [])
+
+
+@pytest.mark.parametrize("L,nt,C,threads,icm,lo,level", _cases(rows.test_rows_and_general_path_identical))
+def test_form_of_the_lattice_rows(tb, gpu, monkeypatch, capfd, L, nt, C, threads, icm, lo, level):
+    d = rows._dev(tb, gpu, L)
+    b = tb.geometric_betas(0.2, 5.0, nt) if nt > 1 else np.array([0.9], np.float32)
+    p = tb.PtParams(60, b, lo, 0.5, icm, C, threads, 7, 9, level)
+    monkeypatch.setenv("TAMC_PT_FORM", "fused")
+    for on in ("0", "1"):
+        monkeypatch.setenv("TAMC_PT_ROWS", on)
+        tb.PtRun(d, p, 11)
+    assert _forms(capfd) == ["fused", "rows"]
+
+
+@pytest.mark.parametrize("kind,size,R", _cases(sa.test_annealing_kernels_identical))
+def test_kernel_of_the_annealing_cases(tb, gpu, capfd, kind, size, R):
+    h = sa._host(tb, kind, size)
+    tb.sa_run(gpu.upload(h), np.array([0.5], np.float32), R, 1, 5)
+    # 0 words, 1 table, 2 slices.  Rows of 4: the table, which at 64 x 64 sites does
+    # not fit; rows of 3: the table where the busiest of 148 SMs has ten warps of
+    # work (32 sites of the largest class x 4 restarts); uneven rows: slices
+    warps = -(-(-(-R // 4)) // 148) * -(-np.bincount(h.coloring()[1]).max() // 32)
+    want = {"gauss2": 0 if size == 64 else 1, "rrg": 1 if warps >= 10 else 0}.get(kind, 2)
+    assert _printed(capfd, r"\[tamc\] SA tile .*: kernel (\d)") == [str(want)]
