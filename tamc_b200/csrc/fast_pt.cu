@@ -3421,7 +3421,7 @@ __global__ void k_plain_energy(const PtJob* __restrict__ jp, long long* acc) {
 bool fused_rows(const PtJob& j) {
   if (const char* e = getenv("TAMC_PT_ROWS"))
     if (e[0] == '0') return false;
-  return j.msc && j.F.cb_L && j.F.offset == 0.0f;
+  return j.msc && !j.icm_uf && j.F.cb_L && j.F.offset == 0.0f;
 }
 
 size_t fused_smem_bytes(const PtJob& j, uint32_t T, bool csr_smem) {

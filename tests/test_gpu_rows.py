@@ -62,3 +62,19 @@ def test_rows_in_a_batch(tb, gpu, monkeypatch, threads, other):
         logs = b.gs_all()
         got.append([x for k in range(len(jobs)) for x in (*b.state(k), b.acceptance(k), *b.round_trips(k), *logs[k])])
     _same(*got)
+
+
+# the rows' cluster growth against the union-find search, which runs on the general path
+@pytest.mark.parametrize("L,nt,C", [(4, 5, 2), (10, 13, 4), (16, 32, 2), (30, 24, 2), (32, 64, 2)])
+def test_rows_and_union_find_identical(tb, gpu, monkeypatch, capfd, L, nt, C):
+    d = _dev(tb, gpu, L)
+    p = tb.PtParams(60, tb.geometric_betas(0.2, 5.0, nt), nt // 3, 0.5, True, C, 8, 7, 9, 0)
+    monkeypatch.setenv("TAMC_PT_FORM", "fused")
+    monkeypatch.setenv("TAMC_AUTOTUNE", "0")
+    monkeypatch.setenv("TAMC_DEBUG", "1")
+    got = [_everything(tb.PtRun(d, p, 11).run())]
+    monkeypatch.setenv("TAMC_ICM", "uf")
+    got.append(_everything(tb.PtRun(d, p, 11).run()))
+    err = capfd.readouterr().err
+    assert [x for x in ("rows", "fused", "plain", "ladder") if f": {x}, threads" in err] == ["rows", "fused"]
+    _same(*got)
