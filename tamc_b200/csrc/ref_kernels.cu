@@ -27,6 +27,9 @@
 // thread per stream with every load from HBM or L2 and the exact expf per site.
 #include "ref_kernels.cuh"
 
+#include <algorithm>
+#include <cstdlib>
+
 namespace tamc {
 namespace refk {
 
@@ -1105,12 +1108,15 @@ void ref_energy_all(cudaStream_t st, const RefInst& I, const int8_t* spins, floa
   refk::k_energy_all<<<R, 128, 0, st>>>(I, spins, energy);
 }
 // Largest dynamic shared memory of the kernels below (they leave room for 8 KB
-// of their own).
+// of their own).  TAMC_REF_SMEM lowers it, so that a small instance takes the
+// kernels for sizes that do not fit.
 static size_t ref_smem_limit() {
   int dev = 0, v = 0;
   TAMC_CUDA(cudaGetDevice(&dev));
   TAMC_CUDA(cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-  return (size_t)v - 8192;
+  const size_t most = (size_t)v - 8192;
+  const char* e = getenv("TAMC_REF_SMEM");
+  return e ? std::min<size_t>(most, strtoull(e, nullptr, 10)) : most;
 }
 template <typename K>
 static void ref_smem_attr(K k, size_t bytes) {
