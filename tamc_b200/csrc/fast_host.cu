@@ -1185,50 +1185,67 @@ struct ChunkRunner {
     const double nr = (double)j.n * j.C * j.ntp;
     return 12 + nr * (j.msc ? 0.16e-3 : j.F.udeg ? 1.2e-3 : j.n > 2048 ? 2.3e-3 : 2e-3);
   }
-  // The ladder launches of runs [k, k1) of `act`: as many runs at a time as have
-  // all their CTAs resident.  The CTA size of a launch is the one with the most
-  // replica rounds per expected time, or the fastest that takes all that remain.
-  static bool ladder_groups(tamc_gpu* g, const std::vector<tamc_pt*>& act, const std::vector<uint32_t>& rounds,
-                            size_t k, size_t k1, Plan& P) {
+  // What the plans of a step need of a run in the ladder form.
+  static constexpr uint32_t LAD_T[3] = {512, 256, 128};
+  struct LadCost {
+    size_t smem = 0;
+    uint32_t ctas = 0;
+    bool takes = false;  // the ladder form takes the run
+    double us[3] = {};   // its expected rounds at LAD_T threads a CTA
+  };
+  static LadCost ladder_cost(const tamc_gpu* g, const PtJob& j, uint32_t rounds) {
+    LadCost c;
+    c.smem = ladder_smem(j, 0);
+    c.ctas = j.C * j.nt;
+    c.takes = !j.icm_uf && c.smem <= g->smem_optin - 512;
+    for (int k = 0; k < 3; ++k) c.us[k] = ladder_us(j, LAD_T[k]) * rounds;
+    return c;
+  }
+  // The ladder launch of runs from k on, before k1: as many as have all their CTAs
+  // resident.  Its CTA size is the one with the most replica rounds per expected time,
+  // or the fastest that takes all that remain.  `reach`: how far the CTA sizes got
+  // (short of k1, the launch would be the same for any later k1).
+  struct LadPick {
+    LadGroup G;
+    double us = 0.0;
+    size_t reach = 0;
+  };
+  static LadPick ladder_group(const tamc_gpu* g, const std::vector<LadCost>& runs, size_t k, size_t k1) {
     const char* t_env = getenv("TAMC_PT_T");
-    while (k < k1) {
-      LadGroup best;
-      double best_us = 0.0, best_rate = 0.0;
-      bool best_all = false;
-      for (uint32_t T : {512u, 256u, 128u}) {
-        if (t_env && (uint32_t)atoi(t_env) != T) continue;
-        LadGroup G;
-        G.first = k;
-        G.T = T;
-        double us = 0.0, work = 0.0;
-        for (size_t x = k; x < k1; ++x) {
-          const PtJob& j = act[x]->fast->job;
-          const size_t own = ladder_smem(j, 0), smem = std::max(G.smem, own);
-          if (j.icm_uf || own > g->smem_optin - 512) return false;
-          if (G.grid + j.C * j.nt > ladder_capacity(g, T, smem)) break;
-          G.smem = smem;
-          G.grid += j.C * j.nt;
-          ++G.count;
-          us = std::max(us, ladder_us(j, T) * rounds[x]);
-          work += (double)j.C * j.nt * ladder_us(j, 512) * rounds[x];
-        }
-        if (!G.count) continue;
-        const bool all = k + G.count == k1;
-        const double rate = work / us;
-        if (!best.count || (all && (!best_all || us < best_us)) || (!all && !best_all && rate > best_rate)) {
-          best = G;
-          best_us = us;
-          best_rate = rate;
-          best_all = all;
-        }
+    LadPick best;
+    double best_rate = 0.0;
+    bool best_all = false;
+    for (int t = 0; t < 3; ++t) {
+      if (t_env && (uint32_t)atoi(t_env) != LAD_T[t]) continue;
+      LadGroup G;
+      G.first = k;
+      G.T = LAD_T[t];
+      double us = 0.0, work = 0.0;
+      uint32_t room = 0;  // CTAs resident at once with G.smem
+      for (size_t x = k; x < k1; ++x) {
+        const LadCost& r = runs[x];
+        if (!r.takes) return LadPick();
+        const size_t smem = std::max(G.smem, r.smem);
+        if (smem != G.smem) room = ladder_capacity(g, G.T, smem);
+        if (G.grid + r.ctas > room) break;
+        G.smem = smem;
+        G.grid += r.ctas;
+        ++G.count;
+        us = std::max(us, r.us[t]);
+        work += r.ctas * r.us[0];
       }
-      if (!best.count) return false;
-      P.groups.push_back(best);
-      P.us += best_us;
-      k += best.count;
+      best.reach = std::max(best.reach, k + G.count);
+      if (!G.count) continue;
+      const bool all = k + G.count == k1;
+      const double rate = work / us;
+      if (!best.G.count || (all && (!best_all || us < best.us)) || (!all && !best_all && rate > best_rate)) {
+        best.G = G;
+        best.us = us;
+        best_rate = rate;
+        best_all = all;
+      }
     }
-    P.ladder = k1;
-    return true;
+    return best;
   }
   // The plan with the least expected time for the runs `act` (by descending
   // size) and their rounds: up to 24 places to split them at.  The ladder form
@@ -1248,14 +1265,29 @@ struct ChunkRunner {
     auto fused_from = [&](size_t x) { return std::max(most[x], sum[x] / g->num_sms); };
     const bool force = f && !strcmp(f, "ladder");
     best.us = force ? 1e30 : 0.9 * fused_from(0);
+    std::vector<LadCost> runs;
+    for (size_t x = 0; x < na; ++x) runs.push_back(ladder_cost(g, act[x]->fast->job, rounds[x]));
+    std::vector<LadPick> picks(na);  // launches from each run on that no place to split at cuts short
     size_t last = 0;
     for (size_t c = 1; c <= 24; ++c) {
-      const size_t k = split && !force ? (na * c + 23) / 24 : na;
-      if (k == last) continue;
-      last = k;
+      const size_t k1 = split && !force ? (na * c + 23) / 24 : na;
+      if (k1 == last) continue;
+      last = k1;
       Plan P;
-      if (!ladder_groups(g, act, rounds, 0, k, P)) break;
-      if (k < na) P.us += fused_from(k);
+      while (P.ladder < k1) {
+        LadPick& known = picks[P.ladder];
+        LadPick p = known;
+        if (!p.G.count) {
+          p = ladder_group(g, runs, P.ladder, k1);
+          if (p.reach < k1) known = p;
+        }
+        if (!p.G.count) break;
+        P.groups.push_back(p.G);
+        P.us += p.us;
+        P.ladder += p.G.count;
+      }
+      if (P.ladder < k1) break;
+      if (k1 < na) P.us += fused_from(k1);
       if (P.us < best.us) best = std::move(P);
     }
     if (getenv("TAMC_DEBUG")) {
@@ -1263,7 +1295,7 @@ struct ChunkRunner {
               best.us, best.ladder);
       for (const LadGroup& G : best.groups)
         fprintf(stderr, " %zu runs, %u CTAs of %u threads, %zu bytes;", G.count, G.grid, G.T, G.smem);
-      fprintf(stderr, "\n");
+      fprintf(stderr, " %llu occupancy queries\n", (unsigned long long)ladder_queries());
     }
     return best;
   }

@@ -145,6 +145,8 @@ size_t ladder_smem(const PtJob& j, int rows);
 void ladder_shape(LadJob& a, int rows, uint32_t cta0);
 // CTAs of T threads and `smem` bytes that are resident at once.
 uint32_t ladder_capacity(const tamc_gpu* g, uint32_t T, size_t smem);
+// How often that had to ask the runtime.
+uint64_t ladder_queries();
 // The three launches of a range of rounds: bitmaps from the words, the rounds
 // (one cooperative launch of `grid` CTAs), results back.  The runs' barrier
 // counters and error flags must be zero.  A run whose error flag is set

@@ -25,9 +25,11 @@
 #include "fast_pt.cuh"
 
 #include <algorithm>
+#include <atomic>
 #include <cstdlib>
 #include <map>
 #include <mutex>
+#include <tuple>
 
 namespace tamc {
 namespace {
@@ -1342,11 +1344,26 @@ static void ladder_attr(size_t smem) {
   }
 }
 
+// Resident CTAs per SM for each CTA size and shared-memory size asked about (at
+// most one entry per 16 bytes of shared memory and CTA size): a server plans every
+// step anew, and asking the runtime for every candidate of a plan cost 0.9 ms a step
+// with 512 requests.
+static std::atomic<uint64_t> g_ladder_queries{0};
+uint64_t ladder_queries() { return g_ladder_queries.load(std::memory_order_relaxed); }
+
 uint32_t ladder_capacity(const tamc_gpu* g, uint32_t T, size_t smem) {
-  ladder_attr(smem);
-  int nb = 0;
-  TAMC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_pt_ladder, (int)T, smem));
-  return (uint32_t)nb * (uint32_t)g->num_sms;
+  static std::mutex mu;
+  static std::map<std::tuple<int, uint32_t, size_t>, int> known;
+  std::lock_guard<std::mutex> lk(mu);
+  auto it = known.find(std::make_tuple(g->device, T, smem));
+  if (it == known.end()) {
+    ladder_attr(smem);
+    int nb = 0;
+    TAMC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_pt_ladder, (int)T, smem));
+    g_ladder_queries.fetch_add(1, std::memory_order_relaxed);
+    it = known.emplace(std::make_tuple(g->device, T, smem), nb).first;
+  }
+  return (uint32_t)it->second * (uint32_t)g->num_sms;
 }
 
 void ladder_launch(cudaStream_t st, const LadJob* d_jobs, const uint32_t* d_cta_job, uint32_t njobs, uint32_t grid,

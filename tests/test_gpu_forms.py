@@ -119,3 +119,16 @@ def test_kernel_of_the_annealing_cases(tb, gpu, capfd, kind, size, R):
     warps = -(-(-(-R // 4)) // 148) * -(-np.bincount(h.coloring()[1]).max() // 32)
     want = {"gauss2": 0 if size == 64 else 1, "rrg": 1 if warps >= 10 else 0}.get(kind, 2)
     assert _printed(capfd, r"\[tamc\] SA tile .*: kernel (\d)") == [str(want)]
+
+
+def test_plans_ask_the_runtime_once(tb, gpu, capfd):
+    # requests of a few sizes, steps of a few rounds: the sizes' occupancies are
+    # known after the first plan
+    srv = tb.Server(gpu, 8 << 30, 64, 5)
+    for k in range(60):
+        h = ladder._host(tb, f"qubo:{61 + 37 * (k % 5)}")
+        srv.submit(h, tb.PtParams(40, tb.geometric_betas(0.2, 5.0, 12 + k % 3), 5, 0.5, True, 2, 8), k)
+    while any(srv.step()):
+        pass
+    asked = [int(x) for x in _printed(capfd, r"\[tamc\] plan for .* (\d+) occupancy queries")]
+    assert len(asked) > 2 and asked[-1] == asked[0]
