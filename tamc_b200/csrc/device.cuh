@@ -193,7 +193,8 @@ struct tamc_gpu {
   int device = 0;
   cudaStream_t stream = nullptr;
   int num_sms = 0;
-  size_t smem_optin = 0;
+  size_t smem_block = 0;  // the most shared memory a CTA can have
+  size_t smem_optin = 0;  // the same less 1 KB for static shared memory
   uint32_t* d_exp = nullptr;  // exception table blob
   tamc::ExpTable exp{};
   std::atomic<uint64_t> launches{0};

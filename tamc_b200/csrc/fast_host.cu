@@ -486,7 +486,7 @@ static bool ladder_setup(tamc_pt* pt) {
   for (uint32_t T = T0; T >= 128; T /= 2)
     for (int rows : {1, 0}) {
       const size_t smem = ladder_smem(j, rows);
-      if (smem > pt->g->smem_optin - 512) continue;  // (the kernel's static shared memory is above 1 KB)
+      if (smem > ladder_smem_limit(pt->g)) continue;
       F->lad.J = j;
       ladder_shape(F->lad, rows, 0);
       if (F->lad.ncta > ladder_capacity(pt->g, T, smem)) continue;
@@ -1197,7 +1197,7 @@ struct ChunkRunner {
     LadCost c;
     c.smem = ladder_smem(j, 0);
     c.ctas = j.C * j.nt;
-    c.takes = !j.icm_uf && c.smem <= g->smem_optin - 512;
+    c.takes = !j.icm_uf && c.smem <= ladder_smem_limit(g);
     for (int k = 0; k < 3; ++k) c.us[k] = ladder_us(j, LAD_T[k]) * rounds;
     return c;
   }

@@ -142,6 +142,8 @@ size_t ladder_bind(LadJob& a, char* base);
 size_t ladder_sync_bytes(const PtJob& j);
 // Shared memory of a CTA (`rows`: rows kept in shared memory).
 size_t ladder_smem(const PtJob& j, int rows);
+// The most that the kernel takes beside its static shared memory.
+size_t ladder_smem_limit(const tamc_gpu* g);
 void ladder_shape(LadJob& a, int rows, uint32_t cta0);
 // CTAs of T threads and `smem` bytes that are resident at once.
 uint32_t ladder_capacity(const tamc_gpu* g, uint32_t T, size_t smem);

@@ -1344,6 +1344,17 @@ static void ladder_attr(size_t smem) {
   }
 }
 
+size_t ladder_smem_limit(const tamc_gpu* g) {
+  static std::atomic<size_t> own{0};  // the kernel's static shared memory
+  size_t b = own.load(std::memory_order_relaxed);
+  if (!b) {
+    cudaFuncAttributes a{};
+    TAMC_CUDA(cudaFuncGetAttributes(&a, k_pt_ladder));
+    own.store(b = a.sharedSizeBytes, std::memory_order_relaxed);
+  }
+  return g->smem_block - b;
+}
+
 // Resident CTAs per SM for each CTA size and shared-memory size asked about (at
 // most one entry per 16 bytes of shared memory and CTA size): a server plans every
 // step anew, and asking the runtime for every candidate of a plan cost 0.9 ms a step

@@ -132,3 +132,27 @@ def test_plans_ask_the_runtime_once(tb, gpu, capfd):
         pass
     asked = [int(x) for x in _printed(capfd, r"\[tamc\] plan for .* (\d+) occupancy queries")]
     assert len(asked) > 2 and asked[-1] == asked[0]
+
+
+def test_most_shared_memory_of_the_ladder_form(tb, gpu, monkeypatch, capfd):
+    # the longest even ring whose rows (26 bytes a site with everything else) a CTA
+    # keeps in shared memory; the next ones keep 10 bytes a site there
+    p = tb.PtParams(3, np.array([0.5, 1.0], np.float32), 1, 0.5, True, 2, 8)
+
+    def run(n, form):
+        x = np.arange(n)
+        rows = np.sort(np.stack([(x - 1) % n, (x + 1) % n], 1), 1)
+        h = tb.HostInstance.from_csr(2 * np.arange(n + 1), rows.ravel(), np.ones(2 * n), np.zeros(n))
+        monkeypatch.setenv("TAMC_PT_FORM", form)
+        return tb.PtRun(gpu.upload(h), p, 3)
+
+    lo, hi = 6000, 14000
+    while hi - lo > 2:
+        mid = (lo + hi) // 4 * 2
+        run(mid, "ladder")
+        form, smem = _printed(capfd, r"\[tamc\] PT run .*: (\w+), threads=\d+ smem=(\d+)")[0]
+        assert form == "ladder"
+        lo, hi = (mid, hi) if int(smem) > 20 * mid else (lo, mid)
+    assert lo > 6000 and hi < 14000
+    a, b = run(lo, "ladder").run().sync(), run(lo, "plain").run().sync()
+    assert a.state()[0].tobytes() == b.state()[0].tobytes() and a.state()[1].tobytes() == b.state()[1].tobytes()
