@@ -168,7 +168,10 @@ void* dev_alloc(size_t bytes) {
   bytes = std::max<size_t>(bytes, 1);
   void* p = nullptr;
   if (bytes > kCacheMaxBlock) {
-    if (cudaMalloc(&p, bytes) != cudaSuccess) fail(TAMC_E_NOMEM, "device allocation failed");
+    if (cudaMalloc(&p, bytes) != cudaSuccess) {
+      cudaGetLastError();
+      fail(TAMC_E_NOMEM, "device allocation failed");
+    }
     return p;
   }
   int dev = 0;
@@ -203,7 +206,10 @@ void* dev_alloc(size_t bytes) {
       cudaDeviceSynchronize();
       free_all_locked(g_cache[dev]);
     }
-    if (cudaMalloc(&p, c) != cudaSuccess) fail(TAMC_E_NOMEM, "device allocation failed");
+    if (cudaMalloc(&p, c) != cudaSuccess) {
+      cudaGetLastError();
+      fail(TAMC_E_NOMEM, "device allocation failed");
+    }
   }
   return p;
 }

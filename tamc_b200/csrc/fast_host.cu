@@ -40,6 +40,7 @@ struct tamc_pt::FastState {
   std::map<uint32_t, cudaGraphExec_t> graphs;  // captured chunks of K rounds
   // ladder form (one run over many CTAs, ladder_pt.cu)
   bool ladder = false;
+  bool no_ladder = false;  // its scratch could not be had
   tamc::LadJob lad{};
   tamc::DBuf<char> lad_mem;
   tamc::DBuf<tamc::LadJob> d_lad;
@@ -464,6 +465,25 @@ static bool other_forms_take(const tamc_gpu* g, const PtJob& j) {
   return plain_head_bytes(j, false) <= g->smem_optin && plain_icm_bytes(j) <= g->smem_optin;
 }
 
+// Memory that only the ladder form needs: false where it cannot be had (the run
+// then takes another form).  TAMC_LADDER_SCRATCH: bytes a run may have.
+template <class T>
+static bool ladder_alloc(DBuf<T>& b, size_t count) {
+  if (b.p && b.n >= count) return true;
+  try {
+    b.alloc(count);
+  } catch (const Error& e) {
+    if (e.code != TAMC_E_NOMEM) throw;
+    return false;
+  }
+  return true;
+}
+static bool ladder_scratch(tamc_pt::FastState* F) {
+  const size_t bytes = ladder_scratch_bytes(F->job);
+  const char* e = getenv("TAMC_LADDER_SCRATCH");
+  return !(e && bytes > strtoull(e, nullptr, 10)) && ladder_alloc(F->lad_mem, bytes);
+}
+
 // Sets the run up in the ladder form if it takes it: all its CTAs, one per
 // replica, are resident at once; rows in shared memory where they fit.
 // A single run takes it whenever it can and is not on lattice rows: over square and cubic lattices, random
@@ -490,12 +510,11 @@ static bool ladder_setup(tamc_pt* pt) {
       F->lad.J = j;
       ladder_shape(F->lad, rows, 0);
       if (F->lad.ncta > ladder_capacity(pt->g, T, smem)) continue;
+      if (!ladder_scratch(F) || !ladder_alloc(F->d_lad, 1)) return false;
       F->T = T;
       F->smem = smem;
-      F->lad_mem.alloc(ladder_scratch_bytes(j));
       ladder_bind(F->lad, F->lad_mem.p);
       F->lad.err = pt->out.err_flag();
-      F->d_lad.alloc(1);
       F->ladder = true;
       return true;
     }
@@ -1193,11 +1212,12 @@ struct ChunkRunner {
     bool takes = false;  // the ladder form takes the run
     double us[3] = {};   // its expected rounds at LAD_T threads a CTA
   };
-  static LadCost ladder_cost(const tamc_gpu* g, const PtJob& j, uint32_t rounds) {
+  static LadCost ladder_cost(const tamc_gpu* g, const tamc_pt* pt, uint32_t rounds) {
+    const PtJob& j = pt->fast->job;
     LadCost c;
     c.smem = ladder_smem(j, 0);
     c.ctas = j.C * j.nt;
-    c.takes = !j.icm_uf && c.smem <= ladder_smem_limit(g);
+    c.takes = !j.icm_uf && !pt->fast->no_ladder && c.smem <= ladder_smem_limit(g);
     for (int k = 0; k < 3; ++k) c.us[k] = ladder_us(j, LAD_T[k]) * rounds;
     return c;
   }
@@ -1247,8 +1267,15 @@ struct ChunkRunner {
     }
     return best;
   }
-  // The plan with the least expected time for the runs `act` (by descending
-  // size) and their rounds: up to 24 places to split them at.  The ladder form
+  // Runs that cannot take the ladder form last, else by descending size.
+  static void plan_order(std::vector<tamc_pt*>& act) {
+    std::stable_sort(act.begin(), act.end(), [](tamc_pt* x, tamc_pt* y) {
+      const bool a = x->fast->no_ladder, b = y->fast->no_ladder;
+      return a != b ? b : x->fast->job.n > y->fast->job.n;
+    });
+  }
+  // The plan with the least expected time for the runs `act` (in plan_order)
+  // and their rounds: up to 24 places to split them at.  The ladder form
   // has to promise a tenth less than the fused one.
   static Plan make_plan(tamc_gpu* g, const std::vector<tamc_pt*>& act, const std::vector<uint32_t>& rounds,
                         bool split = true) {
@@ -1266,7 +1293,7 @@ struct ChunkRunner {
     const bool force = f && !strcmp(f, "ladder");
     best.us = force ? 1e30 : 0.9 * fused_from(0);
     std::vector<LadCost> runs;
-    for (size_t x = 0; x < na; ++x) runs.push_back(ladder_cost(g, act[x]->fast->job, rounds[x]));
+    for (size_t x = 0; x < na; ++x) runs.push_back(ladder_cost(g, act[x], rounds[x]));
     std::vector<LadPick> picks(na);  // launches from each run on that no place to split at cuts short
     size_t last = 0;
     for (size_t c = 1; c <= 24; ++c) {
@@ -1300,23 +1327,30 @@ struct ChunkRunner {
     return best;
   }
   // Advances the runs act[0 .. plan.ladder) to `ends` in the plan's launches and
-  // waits.  Runs whose rounds were given up take theirs in the fused form.
-  void run_ladder(tamc_gpu* g, const std::vector<tamc_pt*>& all, const std::vector<uint32_t>& ends, const Plan& plan) {
+  // waits; false where their scratch could not be had and nothing was done.  Runs
+  // whose rounds were given up take theirs in the fused form.
+  bool run_ladder(tamc_gpu* g, const std::vector<tamc_pt*>& all, const std::vector<uint32_t>& ends, const Plan& plan) {
     cudaStream_t st = g->stream;
     const std::vector<LadGroup>& groups = plan.groups;
     const std::vector<tamc_pt*> act(all.begin(), all.begin() + plan.ladder);
     const size_t na = act.size();
-    reserve((uint32_t)na);
-    if (d_lad.n < na) d_lad.alloc(na);
     std::vector<LadJob> lad(na);
     std::vector<uint32_t> map;
     std::vector<size_t> sync_off(na);
-    size_t sync = 0;
-    for (size_t x = 0; x < na; ++x) {
+    size_t sync = 0, ctas = 0;
+    bool room = true;
+    for (size_t x = 0; x < na && room; ++x) {
       sync_off[x] = sync;
       sync += (ladder_sync_bytes(act[x]->fast->job) + 15) & ~(size_t)15;
+      ctas += (size_t)act[x]->fast->job.C * act[x]->fast->job.nt;
+      room = ladder_scratch(act[x]->fast);
+      act[x]->fast->no_ladder = !room;
     }
-    if (d_sync.n < sync) d_sync.alloc(sync);
+    if (!room || !ladder_alloc(d_lad, na) || !ladder_alloc(d_map, ctas) || !ladder_alloc(d_sync, sync)) {
+      if (getenv("TAMC_DEBUG")) fprintf(stderr, "[tamc] no memory for the planned ladder form\n");
+      return false;
+    }
+    reserve((uint32_t)na);
     TAMC_CUDA(cudaMemsetAsync(d_sync.p, 0, sync, st));
     for (const LadGroup& G : groups) {
       uint32_t cta0 = 0;
@@ -1324,7 +1358,6 @@ struct ChunkRunner {
         const size_t x = G.first + k;
         tamc_pt* pt = act[x];
         auto* F = pt->fast;
-        if (!F->lad_mem.p) F->lad_mem.alloc(ladder_scratch_bytes(F->job));
         LadJob& L = lad[x];
         L.J = F->job;
         L.J.init = F->init_pending ? 1 : 0;
@@ -1342,7 +1375,6 @@ struct ChunkRunner {
         map.insert(map.end(), L.ncta, (uint32_t)k);
       }
     }
-    if (d_map.n < map.size()) d_map.alloc(map.size());
     TAMC_CUDA(tamc::copy_async(d_lad.p, lad.data(), na * sizeof(LadJob), cudaMemcpyHostToDevice, st));
     TAMC_CUDA(tamc::copy_async(d_map.p, map.data(), map.size() * 4, cudaMemcpyHostToDevice, st));
     size_t m0 = 0;
@@ -1383,6 +1415,7 @@ struct ChunkRunner {
       fprintf(stderr, "[tamc] ladder rounds given up: %zu run(s)\n", again.size());
     if (!again.empty() && enqueue(g, slots[0], std::move(again), 0, false, false, false, &again_ends))
       finish(g, slots[0], false, 1);
+    return true;
   }
 
   // Advances every run in `act` by up to `chunk` rounds (one chunk) and waits.
@@ -1393,7 +1426,7 @@ struct ChunkRunner {
 
   bool run_all_ladder(tamc_gpu* g, const std::vector<tamc_pt*>& jobs) {
     std::vector<tamc_pt*> act(jobs);
-    std::stable_sort(act.begin(), act.end(), [](tamc_pt* x, tamc_pt* y) { return x->fast->job.n > y->fast->job.n; });
+    plan_order(act);
     if (act.empty()) return false;
     for (bool first = true;; first = false) {
       act.erase(std::remove_if(act.begin(), act.end(), [](tamc_pt* p) { return p->next_sweep >= p->cfg.num_sweeps; }),
@@ -1404,7 +1437,7 @@ struct ChunkRunner {
       for (size_t x = 0; x < act.size(); ++x) rounds.push_back(ends[x] - act[x]->next_sweep);
       const Plan plan = make_plan(g, act, rounds, false);
       if (plan.ladder != act.size() || (first && plan.groups.size() != 1)) return false;
-      run_ladder(g, act, ends, plan);
+      if (!run_ladder(g, act, ends, plan)) return false;
     }
   }
 
@@ -1433,13 +1466,12 @@ void chunk_run(ChunkRunner* r, tamc_gpu* g, std::vector<tamc_pt*>& act, uint32_t
   for (auto* pt : act)
     if (pt->next_sweep < pt->cfg.num_sweeps) by_size.push_back(pt);
   if (by_size.empty()) return;
-  std::stable_sort(by_size.begin(), by_size.end(),
-                   [](tamc_pt* x, tamc_pt* y) { return x->fast->job.n > y->fast->job.n; });
+  ChunkRunner::plan_order(by_size);
   const std::vector<uint32_t> ends = ChunkRunner::chunk_ends(by_size, chunk, true);
   std::vector<uint32_t> rounds;
   for (size_t x = 0; x < by_size.size(); ++x) rounds.push_back(ends[x] - by_size[x]->next_sweep);
-  const ChunkRunner::Plan plan = ChunkRunner::make_plan(g, by_size, rounds);
-  if (plan.ladder) r->run_ladder(g, by_size, ends, plan);
+  ChunkRunner::Plan plan = ChunkRunner::make_plan(g, by_size, rounds);
+  if (plan.ladder && !r->run_ladder(g, by_size, ends, plan)) plan = ChunkRunner::Plan();
   if (plan.ladder < by_size.size()) {
     const std::vector<tamc_pt*> rest(by_size.begin() + plan.ladder, by_size.end());
     const std::vector<uint32_t> rest_ends(ends.begin() + plan.ladder, ends.end());

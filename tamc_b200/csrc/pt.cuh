@@ -22,8 +22,9 @@ struct DBuf {  // owning device buffer, or a view into another buffer's block
   void alloc(size_t count) {
     release();
     own = true;
-    n = count;
+    n = 0;  // (nothing is held if the allocation fails)
     p = static_cast<T*>(dev_alloc(std::max<size_t>(count, 1) * sizeof(T)));
+    n = count;
   }
   // `count` elements at `q`, inside a block that another DBuf owns and frees
   void view(void* q, size_t count) {

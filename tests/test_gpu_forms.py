@@ -156,3 +156,36 @@ def test_most_shared_memory_of_the_ladder_form(tb, gpu, monkeypatch, capfd):
     assert lo > 6000 and hi < 14000
     a, b = run(lo, "ladder").run().sync(), run(lo, "plain").run().sync()
     assert a.state()[0].tobytes() == b.state()[0].tobytes() and a.state()[1].tobytes() == b.state()[1].tobytes()
+
+
+# scratch that cannot be had: the run, the batch and the server's step take another form
+@pytest.mark.parametrize("how", ["run", "serve", "batch"])
+def test_ladder_scratch_that_cannot_be_had(tb, gpu, monkeypatch, capfd, how):
+    hosts = [ladder._host(tb, k) for k in ("qubo:300", "gauss2:9", "gauss3:6", "qubo:61")]
+    p = tb.PtParams(70, tb.geometric_betas(0.2, 5.0, 12), 5, 0.5, True, 2, 8)
+    monkeypatch.setenv("TAMC_PT_FORM", "ladder")
+    got = []
+    for scratch in (None, "0"):
+        if scratch:
+            monkeypatch.setenv("TAMC_LADDER_SCRATCH", scratch)
+        if how == "run":
+            got.append([x for h in hosts for x in ladder._everything(tb.PtRun(gpu.upload(h), p, 3).run())])
+        elif how == "serve":
+            srv = tb.Server(gpu, 8 << 30, 64, 25)
+            ids = [srv.submit(h, p, 3) for h in hosts]
+            while any(srv.step()):
+                pass
+            got.append([x for i in ids for x in (*srv.state(i), np.float32(srv.result(i)[1]))])
+        else:
+            b = tb.Batch(gpu)
+            for d in gpu.upload_many(hosts):
+                b.add(d, p, 3)
+            b.run()
+            got.append([x for k in range(4) for x in (*b.state(k), b.acceptance(k))])
+        err = capfd.readouterr().err
+        if how == "run":
+            assert set(re.findall(r"\[tamc\] PT run .*: (\w+),", err)) == {"fused" if scratch else "ladder"}
+        else:
+            assert "ladder form: 4 runs" in err  # planned, and with no scratch not taken
+            assert ("[tamc] no memory for the planned ladder form" in err) == bool(scratch)
+    ladder._same(*got)
