@@ -465,10 +465,9 @@ static bool other_forms_take(const tamc_gpu* g, const PtJob& j) {
   return plain_head_bytes(j, false) <= g->smem_optin && plain_icm_bytes(j) <= g->smem_optin;
 }
 
-// Memory that only the ladder form needs: false where it cannot be had (the run
-// then takes another form).  TAMC_LADDER_SCRATCH: bytes a run may have.
+// Room for `count` elements: false where the memory cannot be had.
 template <class T>
-static bool ladder_alloc(DBuf<T>& b, size_t count) {
+static bool may_alloc(DBuf<T>& b, size_t count) {
   if (b.p && b.n >= count) return true;
   try {
     b.alloc(count);
@@ -478,10 +477,12 @@ static bool ladder_alloc(DBuf<T>& b, size_t count) {
   }
   return true;
 }
+// Memory that only the ladder form needs; without it the run takes another form.
+// TAMC_LADDER_SCRATCH: bytes a run may have.
 static bool ladder_scratch(tamc_pt::FastState* F) {
   const size_t bytes = ladder_scratch_bytes(F->job);
   const char* e = getenv("TAMC_LADDER_SCRATCH");
-  return !(e && bytes > strtoull(e, nullptr, 10)) && ladder_alloc(F->lad_mem, bytes);
+  return !(e && bytes > strtoull(e, nullptr, 10)) && may_alloc(F->lad_mem, bytes);
 }
 
 // Sets the run up in the ladder form if it takes it: all its CTAs, one per
@@ -510,7 +511,7 @@ static bool ladder_setup(tamc_pt* pt) {
       F->lad.J = j;
       ladder_shape(F->lad, rows, 0);
       if (F->lad.ncta > ladder_capacity(pt->g, T, smem)) continue;
-      if (!ladder_scratch(F) || !ladder_alloc(F->d_lad, 1)) return false;
+      if (!ladder_scratch(F) || !may_alloc(F->d_lad, 1)) return false;
       F->T = T;
       F->smem = smem;
       ladder_bind(F->lad, F->lad_mem.p);
@@ -668,19 +669,27 @@ void fast_pt_get_state(tamc_pt* pt, int8_t* spins, float* energies) {
   cudaStream_t st = pt->g->stream;
   std::vector<double> Ec((size_t)j.C * j.ntp);
   if (energies) TAMC_CUDA(tamc::copy_async(Ec.data(), F->Ec.p, Ec.size() * 8, cudaMemcpyDeviceToHost, st));
-  if (spins) {
-    DBuf<int8_t> d((size_t)j.C * j.nt * j.n);
+  DBuf<int8_t> d;
+  std::vector<uint32_t> W;
+  if (spins && may_alloc(d, (size_t)j.C * j.nt * j.n)) {
     const uint64_t warps = (uint64_t)((j.n + 127) / 128) * j.nw;
     k_unpack_states<<<(unsigned)((warps + 7) / 8), 256, 0, st>>>(F->W.p, j.F.iperm, j.n, j.nw, j.wpc, j.nt, d.p);
     TAMC_CUDA(cudaGetLastError());
     pt->g->count();
     TAMC_CUDA(tamc::copy_async(spins, d.p, d.n, cudaMemcpyDeviceToHost, st));
-    TAMC_CUDA(cudaStreamSynchronize(st));  // before the buffer goes back
+  } else if (spins) {  // no device memory for them: unpacked here
+    W.resize((size_t)j.n * j.nw);
+    TAMC_CUDA(tamc::copy_async(W.data(), F->W.p, W.size() * 4, cudaMemcpyDeviceToHost, st));
   }
   TAMC_CUDA(cudaStreamSynchronize(st));
   if (energies)
     for (uint32_t ch = 0; ch < j.C; ++ch)
       for (uint32_t t = 0; t < j.nt; ++t) energies[(size_t)ch * j.nt + t] = (float)Ec[(size_t)ch * j.ntp + t];
+  for (uint32_t r = 0; r < (W.empty() ? 0u : j.C * j.nt); ++r) {
+    const uint32_t o = r / j.nt * j.wpc + r % j.nt / 32, b = r % j.nt % 32;
+    for (uint32_t s = 0; s < j.n; ++s)
+      spins[(size_t)r * j.n + pt->inst->h_perm[s]] = ((W[(size_t)s * j.nw + o] >> b) & 1u) ? -1 : 1;
+  }
 }
 
 void fast_pt_set_state(tamc_pt* pt, const int8_t* spins) {
@@ -1346,7 +1355,7 @@ struct ChunkRunner {
       room = ladder_scratch(act[x]->fast);
       act[x]->fast->no_ladder = !room;
     }
-    if (!room || !ladder_alloc(d_lad, na) || !ladder_alloc(d_map, ctas) || !ladder_alloc(d_sync, sync)) {
+    if (!room || !may_alloc(d_lad, na) || !may_alloc(d_map, ctas) || !may_alloc(d_sync, sync)) {
       if (getenv("TAMC_DEBUG")) fprintf(stderr, "[tamc] no memory for the planned ladder form\n");
       return false;
     }

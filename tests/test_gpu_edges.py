@@ -92,3 +92,20 @@ def test_instance_without_sites_is_refused(tb, gpu):
     with pytest.raises(tb.TamcError) as e:
         gpu.upload(h)
     assert e.value.code == -1
+
+
+def test_states_are_read_without_free_device_memory(tb, gpu):
+    """Reading 2048 replicas of 16384 sites while 24 MiB of device memory are free."""
+    torch = pytest.importorskip("torch")
+    d = gpu.upload(tb.HostInstance.parse(gi.lattice(128, 2, "gauss", 1)))
+    p = tb.PtParams(2, tb.geometric_betas(0.2, 5.0, 64), 32, 0.5, True, 32, 8)
+    r = tb.PtRun(d, p, 4).run().sync()
+    S, E = r.state()
+    torch.cuda.empty_cache()
+    held = torch.empty(torch.cuda.mem_get_info()[0] - (24 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        S1, E1 = r.state()
+    finally:
+        del held
+        torch.cuda.empty_cache()
+    assert S.tobytes() == S1.tobytes() and E.tobytes() == E1.tobytes()
