@@ -2,6 +2,7 @@
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
+#include <functional>
 #include <map>
 #include <mutex>
 #include <string>
@@ -65,8 +66,8 @@ static T* dmalloc_copy(const T* h, size_t count) {
   return d;
 }
 
-// The arrays of one instance upload, packed at 256-byte offsets into one host
-// staging buffer, then one device allocation and one copy.
+// Arrays of an instance upload, packed at 256-byte offsets into one host staging
+// buffer, for one device allocation and one copy.
 struct UploadPack {
   std::vector<char> host;
   std::vector<std::pair<void**, size_t>> slots;
@@ -77,12 +78,6 @@ struct UploadPack {
     host.resize(off + bytes, 0);
     if (count) memcpy(host.data() + off, h, count * sizeof(T));
     slots.emplace_back(reinterpret_cast<void**>(slot), off);
-  }
-  void commit(void*& arena, size_t& bytes) {
-    bytes = host.size();
-    arena = dev_alloc(bytes);
-    TAMC_CUDA(copy_sync(arena, host.data(), bytes, cudaMemcpyHostToDevice));
-    bind(arena);
   }
   // the arrays' device addresses inside `arena`
   void bind(void* arena) {
@@ -265,7 +260,8 @@ void tamc_inst_release(tamc_inst* d) {
   if (d->refs.fetch_sub(1) != 1) return;
   tamc_gpu* g = d->g;
   cudaSetDevice(g->device);
-  if (d->arena) dev_free(d->arena, d->arena_bytes);  // holds every array of the instance
+  if (d->arena) dev_free(d->arena, d->arena_bytes);
+  if (d->sl_arena) dev_free(d->sl_arena, d->sl_bytes);
   d->sa_scratch.release();
   delete d;
   tamc_gpu_release(g);
@@ -275,6 +271,10 @@ void tamc_inst_release(tamc_inst* d) {
 // by descending row length (a counting sort), 32 to a slice as long as its
 // longest row (made even).  On rows of uneven length the lanes of a warp then run loops of
 // about the same length and read consecutive entries.
+static bool wants_slices(uint32_t n, uint32_t udeg, bool self_loops) {
+  return n <= 65535 && (self_loops || (udeg != 3 && udeg != 4 && udeg != 6));
+}
+static bool slices_padded(uint64_t entries, uint64_t nnz) { return entries > std::max<uint64_t>(2 * nnz, 65536); }
 static void slice_rows(tamc_inst* d, const std::vector<uint32_t>& frp, const std::vector<uint2>& fent,
                        UploadPack& pack) {
   const uint32_t n = d->n, len_max = d->max_deg;
@@ -299,7 +299,7 @@ static void slice_rows(tamc_inst* d, const std::vector<uint32_t>& frp, const std
     cls[c + 1] = (uint32_t)(site.size() / 32);
   }
   // positions are 16 bits; many small classes of long rows would be mostly padding
-  if (site.size() > 65535 || (uint64_t)off.back() * 32 > std::max<uint64_t>(2 * fent.size(), 65536)) return;
+  if (site.size() > 65535 || slices_padded((uint64_t)off.back() * 32, fent.size())) return;
   d->sl_n = (uint32_t)off.size() - 1;
   d->sl_rows = off.back();
   std::vector<uint2> ent((size_t)d->sl_rows * 32);
@@ -319,11 +319,41 @@ static void slice_rows(tamc_inst* d, const std::vector<uint32_t>& frp, const std
   pack.add(&d->d_sl_ent, ent.data(), ent.size());
 }
 
+namespace tamc {
+void inst_drop_slices(tamc_inst* d) {
+  if (d->sl_arena) dev_free(d->sl_arena, d->sl_bytes);
+  d->sl_arena = nullptr;
+  d->sl_bytes = 0;
+  d->sl_n = d->sl_rows = 0;
+  d->d_sl_cls = d->d_sl_off = nullptr;
+  d->d_sl_site = d->d_sl_pos = nullptr;
+  d->d_sl_ent = nullptr;
+}
+
+// Without the colouring.  Its classes are at most as many as rows x, by descending
+// length, with more than x entries (or two); a class's first slice is as long as its
+// longest row, and 32 times the length of every other slice is at most what the 32
+// rows before it hold; lengths are made even.  (QUBOs of 61 to 8192 sites: 1.4 to 3.8
+// times what they take.)
+uint64_t slices_bytes(const HostInstance& h) {
+  const uint64_t n = h.n, nnz = h.col.size();
+  std::vector<uint32_t> len(h.n);
+  for (uint32_t i = 0; i < h.n; ++i) len[i] = h.row_ptr[i + 1] - h.row_ptr[i];
+  std::sort(len.begin(), len.end(), std::greater<uint32_t>());
+  if (!n || !wants_slices(h.n, len.front() == len.back() ? len.front() : 0u, h.has_self_loops())) return 0;
+  uint64_t classes = 2, most = nnz + n;
+  while (classes < n && len[classes] >= classes) ++classes;
+  for (uint64_t c = 0; c < std::min(classes, n); ++c) most += 32 * (len[c] + 1);
+  const uint64_t entries = std::min<uint64_t>(most, std::max<uint64_t>(2 * nnz, 65536));
+  return entries * 8 + (n + 32 * classes) * 2 + n * 2 + (classes + 1) * 4 + (n / 32 + classes + 1) * 4 + 5 * 256;
+}
+}  // namespace tamc
+
 // Host side of an upload: every array of the instance (reference order, ICM
-// graph, colour order, lattice layouts) into `pack`, and the host fields of
-// `d`.  Touches no device state, so uploads of several instances prepare in
-// parallel.
-static void inst_prepare(tamc_inst* d, const HostInstance& h, UploadPack& pack) {
+// graph, colour order, lattice layouts) into `pack`, its sliced rows into `slices`
+// (unless null), and the host fields of `d`.  Touches no device state, so uploads
+// of several instances prepare in parallel.
+static void inst_prepare(tamc_inst* d, const HostInstance& h, UploadPack& pack, UploadPack* slices) {
   d->host = h;
   d->n = h.n;
   d->nnz = h.col.size();
@@ -420,8 +450,7 @@ static void inst_prepare(tamc_inst* d, const HostInstance& h, UploadPack& pack) 
     pack.add(&d->d_fJt, fJt.data(), fJt.size());
     pack.add(&d->d_fcolt, fcolt.data(), fcolt.size());
   }
-  if (h.n <= 65535 && (d->self_loops || (d->udeg != 3 && d->udeg != 4 && d->udeg != 6)))
-    slice_rows(d, frp, fent, pack);
+  if (slices && wants_slices(h.n, d->udeg, d->self_loops)) slice_rows(d, frp, fent, *slices);
   pack.add(&d->d_fbias, fbias.data(), fbias.size());
   pack.add(&d->d_fkd, fkd.data(), fkd.size());
   pack.add(&d->d_fsus, fsus.data(), fsus.size());
@@ -497,8 +526,26 @@ void tamc_copy_bytes(uint64_t* h2d, uint64_t* d2h) {
 void* tamc_gpu_stream(tamc_gpu* g) { return g ? (void*)g->stream : nullptr; }
 uint64_t tamc_gpu_launch_count(tamc_gpu* g) { return g ? g->launches.load() : 0; }
 
-int tamc_gpu_instance_upload(tamc_gpu* g, const tamc_host_instance* hi, tamc_inst** out) {
-  TAMC_API_BEGIN
+}  // extern "C"
+
+namespace tamc {
+// The device memory of an upload part: false where the sliced rows' cannot be had
+// (the instance then goes without).
+static bool part_alloc(tamc_inst* d, size_t bytes, bool slices) {
+  void*& arena = slices ? d->sl_arena : d->arena;
+  size_t& size = slices ? d->sl_bytes : d->arena_bytes;
+  size = bytes;
+  try {
+    arena = dev_alloc(bytes);
+  } catch (const Error& e) {
+    if (!slices || e.code != TAMC_E_NOMEM) throw;
+    inst_drop_slices(d);
+    return false;
+  }
+  return true;
+}
+
+void upload_instance(tamc_gpu* g, const tamc_host_instance* hi, bool slices, tamc_inst** out) {
   TraceRange tr("tamc upload");
   if (!g || !hi || !out) fail(TAMC_E_INVAL, "null argument");
   // an instance without sites has nothing to sample; refused here rather than
@@ -509,27 +556,31 @@ int tamc_gpu_instance_upload(tamc_gpu* g, const tamc_host_instance* hi, tamc_ins
   d->g = g;
   tamc_gpu_retain(g);
   try {
-    UploadPack pack;
-    inst_prepare(d, hi->h, pack);
-    pack.commit(d->arena, d->arena_bytes);
+    UploadPack packs[2];
+    inst_prepare(d, hi->h, packs[0], slices ? &packs[1] : nullptr);
+    for (int k = 0; k < 2; ++k) {
+      const size_t bytes = packs[k].host.size();
+      if (!bytes || !part_alloc(d, bytes, k == 1)) continue;
+      void* const arena = k ? d->sl_arena : d->arena;
+      TAMC_CUDA(copy_sync(arena, packs[k].host.data(), bytes, cudaMemcpyHostToDevice));
+      packs[k].bind(arena);
+    }
   } catch (...) {
     tamc_gpu_instance_destroy(d);
     throw;
   }
   *out = d;
-  TAMC_API_END
 }
 
-int tamc_gpu_instance_upload_many(tamc_gpu* g, uint32_t count, const tamc_host_instance* const* his,
-                                  tamc_inst** outs) {
-  TAMC_API_BEGIN
+void upload_instances(tamc_gpu* g, uint32_t count, const tamc_host_instance* const* his, const uint8_t* slices,
+                      tamc_inst** outs) {
   TraceRange tr("tamc upload_many");
   if (!g || (count && (!his || !outs))) fail(TAMC_E_INVAL, "null argument");
   for (uint32_t k = 0; k < count; ++k) {
     if (!his[k]) fail(TAMC_E_INVAL, "null instance at index " + std::to_string(k));
     if (his[k]->h.n == 0) fail(TAMC_E_INVAL, "instance at index " + std::to_string(k) + " has no sites");
   }
-  if (count == 0) return TAMC_OK;
+  if (count == 0) return;
   TAMC_CUDA(cudaSetDevice(g->device));
   std::vector<tamc_inst*> ds(count, nullptr);
   auto drop_all = [&] {
@@ -545,9 +596,11 @@ int tamc_gpu_instance_upload_many(tamc_gpu* g, uint32_t count, const tamc_host_i
     }
     // on up to 16 threads: host preparation of every instance, then (after
     // the staging offsets are known) its copy into the pinned staging block
-    std::vector<UploadPack> packs(count);
-    std::vector<size_t> off(count + 1, 0);
-    std::vector<std::exception_ptr> errs(count);
+    // (packs 2 k and 2 k + 1: the arrays of instance k, its sliced rows)
+    const uint32_t parts = 2 * count;
+    std::vector<UploadPack> packs(parts);
+    std::vector<size_t> off(parts + 1, 0);
+    std::vector<std::exception_ptr> errs(parts);
     const uint32_t hw = std::max(1u, std::thread::hardware_concurrency());
     auto parallel = [&](uint32_t k0, uint32_t k1, auto&& f) {
       std::atomic<uint32_t> next{k0};
@@ -573,19 +626,21 @@ int tamc_gpu_instance_upload_many(tamc_gpu* g, uint32_t count, const tamc_host_i
       for (uint32_t k = k0; k < k1; ++k)
         if (errs[k]) std::rethrow_exception(errs[k]);
     };
-    parallel(0, count, [&](uint32_t k) { inst_prepare(ds[k], his[k]->h, packs[k]); });
-    for (uint32_t k = 0; k < count; ++k) off[k + 1] = off[k] + ((packs[k].host.size() + 255) & ~(size_t)255);
-    // staged in rounds of at most `cap` bytes (one instance at least): fill
-    // the block, one device allocation and one asynchronous copy per instance
+    parallel(0, count, [&](uint32_t k) {
+      inst_prepare(ds[k], his[k]->h, packs[2 * k], !slices || slices[k] ? &packs[2 * k + 1] : nullptr);
+    });
+    for (uint32_t k = 0; k < parts; ++k) off[k + 1] = off[k] + ((packs[k].host.size() + 255) & ~(size_t)255);
+    // staged in rounds of at most `cap` bytes (one pack at least): fill
+    // the block, one device allocation and one asynchronous copy per pack
     // on the upload stream, one wait; the instances are complete on return,
     // as after tamc_gpu_instance_upload
     size_t cap = (size_t)256 << 20;
     if (const char* e = getenv("TAMC_UPLOAD_STAGE_BYTES")) cap = std::max<size_t>(256, strtoull(e, nullptr, 10));
     std::lock_guard<std::mutex> lk(g->up_mu);
     if (!g->up_stream) TAMC_CUDA(cudaStreamCreateWithFlags(&g->up_stream, cudaStreamNonBlocking));
-    for (uint32_t k0 = 0, k1; k0 < count; k0 = k1) {
+    for (uint32_t k0 = 0, k1; k0 < parts; k0 = k1) {
       k1 = k0 + 1;
-      while (k1 < count && off[k1 + 1] - off[k0] <= cap) ++k1;
+      while (k1 < parts && off[k1 + 1] - off[k0] <= cap) ++k1;
       const size_t bytes = off[k1] - off[k0];
       if (bytes > g->up_pin_bytes) {
         if (g->up_pin) TAMC_CUDA(cudaFreeHost(g->up_pin));
@@ -598,10 +653,11 @@ int tamc_gpu_instance_upload_many(tamc_gpu* g, uint32_t count, const tamc_host_i
       auto pin = [&](uint32_t k) { return g->up_pin + (off[k] - off[k0]); };
       parallel(k0, k1, [&](uint32_t k) { memcpy(pin(k), packs[k].host.data(), packs[k].host.size()); });
       for (uint32_t k = k0; k < k1; ++k) {
-        ds[k]->arena_bytes = packs[k].host.size();
-        ds[k]->arena = dev_alloc(ds[k]->arena_bytes);
-        TAMC_CUDA(copy_async(ds[k]->arena, pin(k), ds[k]->arena_bytes, cudaMemcpyHostToDevice, g->up_stream));
-        packs[k].bind(ds[k]->arena);
+        const size_t part = packs[k].host.size();
+        if (!part || !part_alloc(ds[k / 2], part, k % 2)) continue;
+        void* const arena = k % 2 ? ds[k / 2]->sl_arena : ds[k / 2]->arena;
+        TAMC_CUDA(copy_async(arena, pin(k), part, cudaMemcpyHostToDevice, g->up_stream));
+        packs[k].bind(arena);
       }
       TAMC_CUDA(cudaStreamSynchronize(g->up_stream));
     }
@@ -610,6 +666,22 @@ int tamc_gpu_instance_upload_many(tamc_gpu* g, uint32_t count, const tamc_host_i
     throw;
   }
   for (uint32_t k = 0; k < count; ++k) outs[k] = ds[k];
+}
+
+}  // namespace tamc
+
+extern "C" {
+
+int tamc_gpu_instance_upload(tamc_gpu* g, const tamc_host_instance* hi, tamc_inst** out) {
+  TAMC_API_BEGIN
+  upload_instance(g, hi, true, out);
+  TAMC_API_END
+}
+
+int tamc_gpu_instance_upload_many(tamc_gpu* g, uint32_t count, const tamc_host_instance* const* his,
+                                  tamc_inst** outs) {
+  TAMC_API_BEGIN
+  upload_instances(g, count, his, nullptr, outs);
   TAMC_API_END
 }
 

@@ -296,8 +296,10 @@ struct tamc_inst {
   uint16_t *d_sl_site = nullptr, *d_sl_pos = nullptr;
   uint2* d_sl_ent = nullptr;
   float* d_fbias = nullptr;          // n
-  void* arena = nullptr;             // one allocation holding every array above
+  void* arena = nullptr;             // one allocation holding every array but the sliced rows
   size_t arena_bytes = 0;
+  void* sl_arena = nullptr;          // one holding those: kernels that want them are left out without
+  size_t sl_bytes = 0;
   float* d_fkd = nullptr;            // n: self-loop coefficient (0 if none)
   double* d_fsus = nullptr;          // [nchi][n] colour order
   // host copies used by drivers
@@ -305,5 +307,16 @@ struct tamc_inst {
   std::vector<uint32_t> h_perm;
   SaScratch sa_scratch;
 };
+namespace tamc {
+// Uploads of instances, each with its sliced rows unless `slices` says 0 for it
+// (null: all with them).
+void upload_instance(tamc_gpu* g, const tamc_host_instance* h, bool slices, tamc_inst** out);
+void upload_instances(tamc_gpu* g, uint32_t count, const tamc_host_instance* const* hs, const uint8_t* slices,
+                      tamc_inst** outs);
+// Gives the sliced rows back (nothing that uses the instance may be in flight).
+void inst_drop_slices(tamc_inst* d);
+// The most that the sliced rows of an instance take.
+uint64_t slices_bytes(const HostInstance& h);
+}  // namespace tamc
 void tamc_inst_retain(tamc_inst* d);
 void tamc_inst_release(tamc_inst* d);

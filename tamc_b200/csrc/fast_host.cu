@@ -40,7 +40,7 @@ struct tamc_pt::FastState {
   std::map<uint32_t, cudaGraphExec_t> graphs;  // captured chunks of K rounds
   // ladder form (one run over many CTAs, ladder_pt.cu)
   bool ladder = false;
-  bool no_ladder = false;  // its scratch could not be had
+  bool no_ladder = false;  // its scratch could not be had, or is not to be
   tamc::LadJob lad{};
   tamc::DBuf<char> lad_mem;
   tamc::DBuf<tamc::LadJob> d_lad;
@@ -483,6 +483,12 @@ static bool ladder_scratch(tamc_pt::FastState* F) {
   const size_t bytes = ladder_scratch_bytes(F->job);
   const char* e = getenv("TAMC_LADDER_SCRATCH");
   return !(e && bytes > strtoull(e, nullptr, 10)) && may_alloc(F->lad_mem, bytes);
+}
+
+void fast_pt_no_ladder(tamc_pt* pt) {
+  pt->fast->no_ladder = true;
+  pt->fast->lad_mem.release();
+  pt->fast->job.F = make_fast_inst(pt->inst);
 }
 
 // Sets the run up in the ladder form if it takes it: all its CTAs, one per

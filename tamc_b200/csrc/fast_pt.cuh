@@ -156,6 +156,10 @@ uint64_t ladder_queries();
 void ladder_launch(cudaStream_t st, const LadJob* d_jobs, const uint32_t* d_cta_job, uint32_t njobs, uint32_t grid,
                    uint32_t T, size_t smem, uint32_t open_grid);
 
+// Keeps a run out of the ladder form for good and gives its scratch for it back
+// (nothing of the run may be in flight; its instance may have dropped its sliced rows).
+void fast_pt_no_ladder(tamc_pt* pt);
+
 // tamc_pt glue (single-instance handle in fast mode)
 void fast_pt_create(tamc_pt* pt, uint64_t seed);
 void fast_pt_run(tamc_pt* pt, uint32_t sweep_end);

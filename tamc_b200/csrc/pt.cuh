@@ -18,11 +18,11 @@ struct DBuf {  // owning device buffer, or a view into another buffer's block
   void release() {
     if (p && own) dev_free(p, std::max<size_t>(n, 1) * sizeof(T));
     p = nullptr;
+    n = 0;
   }
   void alloc(size_t count) {
-    release();
+    release();  // (nothing is held if the allocation fails)
     own = true;
-    n = 0;  // (nothing is held if the allocation fails)
     p = static_cast<T*>(dev_alloc(std::max<size_t>(count, 1) * sizeof(T)));
     n = count;
   }

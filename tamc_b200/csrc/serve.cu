@@ -2,7 +2,9 @@
 //
 // Requests (instance + PT-ICM method) arrive at any time.  A scheduling step
 // admits queued requests while the number of active requests stays under
-// `max_active` and their estimated HBM footprint stays under the budget, runs
+// `max_active` and their estimated HBM footprint stays under the budget (what only
+// the ladder form needs comes on top where the budget leaves room, and is given back
+// when a request could not be admitted beside it), runs
 // one chunk of PT rounds for every active request -- in one fused launch, in
 // launches of the ladder form, or the largest in those and the others in that,
 // whichever promises to take least time -- (each request's replica state stays
@@ -40,6 +42,9 @@ struct Request {
   uint64_t seed = 0;
   float target = NAN;
   uint64_t footprint = 0;
+  uint64_t extra = 0;     // what the ladder form needs on top: sliced rows and scratch
+  uint64_t slices = 0;    // (the rows' part, as estimated)
+  bool spread = false;    // it has that
   tamc_inst* dinst = nullptr;
   tamc_pt* pt = nullptr;
   int state = 0;  // TAMC_REQ_QUEUED / _ACTIVE / _DONE / _CANCELLED / _FAILED
@@ -63,6 +68,14 @@ uint64_t footprint_bytes(const HostInstance& h, const tamc_pt_params& p) {
   b += nt * M * C * 4 + nt * M * (C / 2) * 4 * (1 + nchi) + nt * S * C * ((n + 7) / 8);
   b += 1024ull * (8 + ((n + 63) / 64) * 8);  // ground-state log
   return b;
+}
+
+uint64_t scratch_bytes(const HostInstance& h, const tamc_pt_params& p) {
+  PtJob j{};
+  j.n = h.n;
+  j.nt = p.num_beta;
+  j.C = p.num_replica_chains;
+  return ladder_scratch_bytes(j);
 }
 }  // namespace
 
@@ -104,7 +117,25 @@ static void retire(tamc_server* s, Request* r, int state = TAMC_REQ_DONE) {
   r->dinst = nullptr;
   r->state = state;
   r->t_done = Clock::now();
-  s->used -= r->footprint;
+  s->used -= r->footprint + (r->spread ? r->extra : 0);
+}
+
+// Room for a request of `need` bytes: where the budget is used up, active requests
+// (the last admitted first) give back what only the ladder form needs and go on
+// without it, so that requests are admitted by their footprint alone.
+static bool make_room(tamc_server* s, uint64_t need) {
+  uint64_t back = 0;
+  for (const Request* r : s->active) back += r->spread ? r->extra : 0;
+  if (s->used + need > s->budget + back) return false;
+  for (size_t k = s->active.size(); k-- > 0 && s->used + need > s->budget;) {
+    Request* r = s->active[k];
+    if (!r->spread) continue;
+    inst_drop_slices(r->dinst);
+    fast_pt_no_ladder(r->pt);
+    r->spread = false;
+    s->used -= r->extra;
+  }
+  return true;
 }
 
 extern "C" {
@@ -139,6 +170,8 @@ int tamc_serve_submit(tamc_server* s, const tamc_host_instance* inst, const tamc
   r->seed = seed;
   r->target = target_energy;
   r->footprint = footprint_bytes(inst->h, *p);
+  r->slices = slices_bytes(inst->h);
+  r->extra = r->slices + scratch_bytes(inst->h, *p);
   if (r->footprint > s->budget) {
     delete r->h;
     delete r;
@@ -166,20 +199,38 @@ int tamc_serve_step(tamc_server* s, uint32_t* active, uint32_t* queued) {
     more = false;
     std::vector<Request*> in;
     while (!s->queue.empty() && s->active.size() + in.size() < s->max_active &&
-           s->used + s->queue.front()->footprint <= s->budget) {
+           make_room(s, s->queue.front()->footprint)) {
       in.push_back(s->queue.front());
       s->queue.pop_front();
       s->used += in.back()->footprint;
     }
+    std::vector<const tamc_host_instance*> hs;
+    std::vector<uint8_t> spread;
+    for (auto* r : in) {
+      r->spread = s->used + r->extra <= s->budget;
+      if (r->spread) s->used += r->extra;
+      hs.push_back(r->h);
+      spread.push_back(r->spread);
+    }
     if (in.size() >= 4) {  // (fewer are not worth the threads: 24 QUBOs of 64-8192 sites 11 -> 4 ms)
-      std::vector<const tamc_host_instance*> hs;
-      for (auto* r : in) hs.push_back(r->h);
       std::vector<tamc_inst*> ds(in.size(), nullptr);
-      if (tamc_gpu_instance_upload_many(s->g, (uint32_t)in.size(), hs.data(), ds.data()) == TAMC_OK)
+      try {
+        upload_instances(s->g, (uint32_t)in.size(), hs.data(), spread.data(), ds.data());
         for (size_t k = 0; k < in.size(); ++k) in[k]->dinst = ds[k];
+      } catch (const std::exception&) {  // one by one below
+      }
     }
     for (Request* r : in) {
-      int rc = r->dinst ? TAMC_OK : tamc_gpu_instance_upload(s->g, r->h, &r->dinst);
+      int rc = TAMC_OK;
+      try {
+        if (!r->dinst) upload_instance(s->g, r->h, r->spread, &r->dinst);
+      } catch (const Error& e) {
+        rc = e.code;
+        set_error(e.what());
+      } catch (const std::bad_alloc&) {
+        rc = TAMC_E_NOMEM;
+        set_error("host allocation failed");
+      }
       if (rc == TAMC_OK) {
         g_no_autotune = true;
         g_defer_init = true;  // its first rounds draw the initial replicas
@@ -199,9 +250,16 @@ int tamc_serve_step(tamc_server* s, uint32_t* active, uint32_t* queued) {
         r->dinst = nullptr;
         r->state = TAMC_REQ_FAILED;
         r->t_done = Clock::now();
-        s->used -= r->footprint;
+        s->used -= r->footprint + (r->spread ? r->extra : 0);
         more = true;
         continue;
+      }
+      if (r->spread) {  // the rows' size is known now
+        const uint64_t less = r->slices - std::min<uint64_t>(r->slices, r->dinst->sl_bytes);
+        r->extra -= less;
+        s->used -= less;
+      } else {
+        fast_pt_no_ladder(r->pt);
       }
       r->state = TAMC_REQ_ACTIVE;
       s->active.push_back(r);

@@ -189,3 +189,61 @@ def test_ladder_scratch_that_cannot_be_had(tb, gpu, monkeypatch, capfd, how):
             assert "ladder form: 4 runs" in err  # planned, and with no scratch not taken
             assert ("[tamc] no memory for the planned ladder form" in err) == bool(scratch)
     ladder._same(*got)
+
+
+def _serve(tb, gpu, budget, reqs, steps_between=0):
+    """The server and the ids of the requests, each submitted `steps_between` steps after the last."""
+    srv = tb.Server(gpu, budget, 64, 10)
+    ids = []
+    for k, (h, p) in enumerate(reqs):
+        for _ in range(steps_between if k else 0):
+            srv.step()
+        ids.append(srv.submit(h, p, 3 + k))
+    return srv, ids
+
+
+def _footprint(tb, gpu, h, p):
+    """The smallest budget that a request is accepted with."""
+    lo, hi = 0, 1 << 28
+    while hi - lo > 1:
+        mid = (lo + hi) // 2
+        try:
+            tb.Server(gpu, mid, 4, 10).submit(h, p, 1)
+            hi = mid
+        except tb.TamcError as e:
+            assert e.code == -9
+            lo = mid
+    return hi
+
+
+# rows of uneven length (sliced rows and scratch) and of one length (scratch alone)
+@pytest.mark.parametrize("kind", ["qubo:700", "gauss3:8"])
+def test_server_budget_covers_the_ladder_form(tb, gpu, monkeypatch, capfd, kind):
+    monkeypatch.setenv("TAMC_PT_FORM", "ladder")
+    h = ladder._host(tb, kind)
+    p = tb.PtParams(60, tb.geometric_betas(0.2, 5.0, 16), 5, 0.5, True, 2, 8)
+    own = _footprint(tb, gpu, h, p)
+
+    def planned():
+        """(runs, those in the ladder form) of the last step's plan."""
+        found = _printed(capfd, r"\[tamc\] plan for (\d+) runs: .* (\d+) in the ladder form")
+        return tuple(int(x) for x in found[-1])
+
+    def results(srv, ids):
+        while any(srv.step()):
+            pass
+        return [x for i in ids for x in (*srv.state(i), np.float32(srv.result(i)[1]))]
+
+    # room for nothing but the footprint: fused, and the second request waits
+    srv, ids = _serve(tb, gpu, own, [(h, p), (h, p)])
+    assert srv.step() == (1, 1) and planned() == (1, 0)
+    got = results(srv, ids)
+    # room for both with all they need
+    srv, ids = _serve(tb, gpu, 4 * own, [(h, p), (h, p)])
+    assert srv.step() == (2, 0) and planned() == (2, 2)
+    ladder._same(results(srv, ids), got)
+    # room for two footprints: the first request has more until the second needs it
+    srv, ids = _serve(tb, gpu, 2 * own, [(h, p), (h, p)], steps_between=2)
+    assert planned() == (1, 1)
+    assert srv.step() == (2, 0) and planned() == (2, 0)
+    ladder._same(results(srv, ids), got)
