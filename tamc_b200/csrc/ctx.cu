@@ -468,8 +468,10 @@ int tamc_gpu_open(int device, tamc_gpu** out) {
   cudaDeviceProp prop;
   TAMC_CUDA(cudaGetDeviceProperties(&prop, device));
   if (prop.major < 10) fail(TAMC_E_UNSUPPORTED, "this library is built for sm_100a (B200)");
+  static std::atomic<uint32_t> busy[64];  // per device (those past the last share one)
   auto* g = new tamc_gpu();
   g->device = device;
+  g->contexts_busy = &busy[std::min(device, 63)];
   g->num_sms = prop.multiProcessorCount;
   // dynamic shared memory a launch may ask for: the opt-in limit less 1 KB for
   // the kernels' static shared memory (job descriptor copies, counters)

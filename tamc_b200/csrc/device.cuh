@@ -208,11 +208,27 @@ struct tamc_gpu {
   cudaStream_t up_stream = nullptr;
   char* up_pin = nullptr;
   size_t up_pin_bytes = 0;
+  // PT runs and batches of this context in progress and its servers with active
+  // requests (they follow one another on its stream), and the contexts of the device
+  // with any.
+  std::atomic<uint32_t> calls{0};
+  std::atomic<uint32_t>* contexts_busy = nullptr;
   void count(uint64_t k = 1) { launches.fetch_add(k, std::memory_order_relaxed); }
 };
 void tamc_gpu_retain(tamc_gpu* g);
 void tamc_gpu_release(tamc_gpu* g);
 namespace tamc {
+struct InProgress {  // one of tamc_gpu::calls
+  tamc_gpu* g;
+  explicit InProgress(tamc_gpu* g_) : g(g_) {
+    if (g->calls.fetch_add(1) == 0) g->contexts_busy->fetch_add(1);
+  }
+  ~InProgress() {
+    if (g->calls.fetch_sub(1) == 1) g->contexts_busy->fetch_sub(1);
+  }
+  InProgress(const InProgress&) = delete;
+  InProgress& operator=(const InProgress&) = delete;
+};
 // Frees the batch chunk runners kept for reuse on this context.
 void runner_pool_release(tamc_gpu* g);
 }  // namespace tamc

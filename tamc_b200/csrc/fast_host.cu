@@ -41,6 +41,9 @@ struct tamc_pt::FastState {
   // ladder form (one run over many CTAs, ladder_pt.cu)
   bool ladder = false;
   bool no_ladder = false;  // its scratch could not be had, or is not to be
+  uint32_t lad_T = 0;
+  size_t lad_smem = 0;
+  bool beside = false;     // the fused form is set up too, for rounds beside other runs
   tamc::LadJob lad{};
   tamc::DBuf<char> lad_mem;
   tamc::DBuf<tamc::LadJob> d_lad;
@@ -518,14 +521,69 @@ static bool ladder_setup(tamc_pt* pt) {
       ladder_shape(F->lad, rows, 0);
       if (F->lad.ncta > ladder_capacity(pt->g, T, smem)) continue;
       if (!ladder_scratch(F) || !may_alloc(F->d_lad, 1)) return false;
-      F->T = T;
-      F->smem = smem;
+      F->lad_T = T;
+      F->lad_smem = smem;
       ladder_bind(F->lad, F->lad_mem.p);
       F->lad.err = pt->out.err_flag();
       F->ladder = true;
       return true;
     }
   return false;
+}
+
+// Expected microseconds per round.  Ladder, in a launch that fills the GPU with
+// CTAs of T threads (48 replicas a run; rows of a QUBO / 3-D Gaussian and 2-D
+// +-J lattices): 512 threads 200 sites 20, 700 38, 2000 45, 6000 80 / 12^3 19,
+// 32^2 14; 256: 30, 35, 57, 95 / 27, 18; 128: 32, 43, 78, 152 / 38, 20.
+// Fused, one run to an SM: QUBO 30, 80, 195, 670; 12^3 Gaussian 113; 32^2 +-J 22.
+static double ladder_us(const PtJob& j, uint32_t T) {
+  const double n = j.n;
+  if (j.F.lat_any) return T >= 512 ? 11 + 0.0045 * n : T >= 256 ? 13 + 0.008 * n : 16 + 0.013 * n;
+  return T >= 512 ? 25 + 0.0092 * n : T >= 256 ? 26 + 0.0125 * n : 27 + 0.022 * n;
+}
+// (on lattice rows, pairs of words: 8^2 sites 5, 32^2 10; two pairs 7, 17)
+static double fused_us(const PtJob& j) {
+  if (j.rows)
+    return 3 + 1.8 * ((j.C + 1) / 2 * j.wpc) + 2e-3 * j.n * j.nw + 2.4e-5 * ((double)j.n * j.C * j.ntp);
+  const double nr = (double)j.n * j.C * j.ntp;
+  return 12 + nr * (j.msc ? 0.16e-3 : j.F.udeg ? 1.2e-3 : j.n > 2048 ? 2.3e-3 : 2e-3);
+}
+
+// Other contexts with something in progress, for one that has (TAMC_PT_BESIDE: so many).
+static uint32_t contexts_beside(const tamc_gpu* g) {
+  if (const char* e = getenv("TAMC_PT_BESIDE")) return (uint32_t)strtoul(e, nullptr, 10);
+  return std::max(g->contexts_busy->load(), 1u) - 1u;
+}
+
+// Whether a run in the ladder form takes its next rounds in the fused form, on one
+// SM, because k - 1 other contexts run something: where k such runs, each taking its
+// CTAs' share of the GPU, are expected to need a seventh more for a round of all of
+// them than side by side on an SM each, 23 at a time (the streams share the device's
+// queues).  Measured, us a round of all, ladder / fused: 2039-site QUBO, 21 temperatures 8 runs 89 / 197, 24 238 / 246, 64 641 / 501,
+// 128 1285 / 682; 300 sites, 24 temperatures 62 / 75 at 24, 164 / 127 at 64; 32 x 32
+// Gaussian 31 / 50 at 8, 95 / 72 at 24, 254 / 150 at 64; 10^3 Gaussian 63 / 108 at 24,
+// 169 / 203 at 64.  (Beside one batch, whatever its size, the ladder form gets its turn
+// between two chunks: 2039-site QUBO 31 / 112.)
+static bool better_fused(tamc_pt* pt) {
+  auto* F = pt->fast;
+  const PtJob& j = F->job;
+  const uint32_t others = contexts_beside(pt->g);
+  const char* f = getenv("TAMC_PT_FORM");
+  if (!others || (f && !strcmp(f, "ladder")) || fused_smem_bytes(j, 128, false) > pt->g->smem_optin) return false;
+  const double k = others + 1.0;
+  const double share = (double)F->lad.ncta / ladder_capacity(pt->g, F->lad_T, F->lad_smem);
+  // (rows of 4 in shared memory take half of what fused_us says)
+  const double alone = fused_us(j) * (j.F.udeg == 4 && !j.msc && j.n <= 1100 ? 0.5 : 1.0);
+  if (std::max(1.0, k * share) * ladder_us(j, std::min(F->lad_T, 512u)) < 1.15 * std::max(1.0, k / 23) * alone)
+    return false;
+  if (!F->beside) {
+    const TileChoice t = heuristic_tile(pt->g, j);
+    F->T = t.T;
+    F->job.csr_smem = t.csr;
+    F->smem = fused_smem_bytes(j, t.T, t.csr);
+    F->beside = true;
+  }
+  return F->smem <= pt->g->smem_optin;
 }
 
 // Rounds [begin, end) (none: only the initial state, init != 0).
@@ -543,7 +601,7 @@ static void ladder_rounds(tamc_pt* pt, uint32_t begin, uint32_t end, int init) {
   TAMC_CUDA(tamc::copy_async(F->d_lad.p, &F->lad, sizeof(LadJob), cudaMemcpyHostToDevice, st));
   TAMC_CUDA(cudaMemsetAsync(F->lad.bar, 0, ladder_sync_bytes(j), st));
   const uint32_t blocks = (uint32_t)(((uint64_t)((j.n + 31) / 32) * j.nw + 7) / 8);
-  ladder_launch(st, F->d_lad.p, nullptr, 1, F->lad.ncta, F->T, F->smem, std::min(blocks, 592u));
+  ladder_launch(st, F->d_lad.p, nullptr, 1, F->lad.ncta, F->lad_T, F->lad_smem, std::min(blocks, 592u));
   pt->g->count(3);
 }
 
@@ -595,7 +653,8 @@ void fast_pt_create(tamc_pt* pt, uint64_t seed) {
   }
   if (getenv("TAMC_DEBUG"))
     fprintf(stderr, "[tamc] PT run n=%u nt=%u C=%u: %s, threads=%u smem=%zu\n", j.n, j.nt, j.C,
-            F->ladder ? "ladder" : F->plain ? "plain" : j.rows ? "rows" : "fused", F->T, F->smem);
+            F->ladder ? "ladder" : F->plain ? "plain" : j.rows ? "rows" : "fused", F->ladder ? F->lad_T : F->T,
+            F->ladder ? F->lad_smem : F->smem);
 }
 
 // Deferred initial replicas, when something reads or runs the run before its
@@ -608,12 +667,17 @@ static void ensure_init(tamc_pt* pt) {
 }
 
 void fast_pt_run(tamc_pt* pt, uint32_t sweep_end) {
+  const InProgress busy(pt->g);
   if (pt->fast->plain) ensure_init(pt);
   const PtCfg& c = pt->cfg;
   while (pt->next_sweep < sweep_end) {
     const uint32_t b = pt->next_sweep;
     const uint32_t e = std::min(sweep_end, b + pt->out.cap);
-    if (pt->fast->ladder) {
+    const bool spread = pt->fast->ladder && !better_fused(pt);
+    if (pt->fast->ladder && !spread && getenv("TAMC_DEBUG"))
+      fprintf(stderr, "[tamc] rounds %u to %u in the fused form beside %u contexts\n", b, e,
+              contexts_beside(pt->g));
+    if (spread) {
       ladder_rounds(pt, b, e, pt->fast->init_pending ? 1 : 0);
       pt->out.dirty = true;
       pt->out.drain(pt->g->stream);
@@ -633,7 +697,7 @@ void fast_pt_run(tamc_pt* pt, uint32_t sweep_end) {
     pt->m_next += count_sched(c.sample, c.meas_init, c.num_sweeps, b, e);
     pt->s_next += count_sched(c.sample_states, c.meas_init, c.num_sweeps, b, e);
     pt->next_sweep = e;
-    if (pt->fast->ladder) pt->out.dirty = false;  // drained above
+    if (spread) pt->out.dirty = false;  // drained above
     else pt->out.drain(pt->g->stream);
   }
 }
@@ -1202,23 +1266,6 @@ struct ChunkRunner {
     size_t ladder = 0;
     double us = 0.0;
   };
-  // Expected microseconds per round.  Ladder, in a launch that fills the GPU with
-  // CTAs of T threads (48 replicas a run; rows of a QUBO / 3-D Gaussian and 2-D
-  // +-J lattices): 512 threads 200 sites 20, 700 38, 2000 45, 6000 80 / 12^3 19,
-  // 32^2 14; 256: 30, 35, 57, 95 / 27, 18; 128: 32, 43, 78, 152 / 38, 20.
-  // Fused, one run to an SM: QUBO 30, 80, 195, 670; 12^3 Gaussian 113; 32^2 +-J 22.
-  static double ladder_us(const PtJob& j, uint32_t T) {
-    const double n = j.n;
-    if (j.F.lat_any) return T >= 512 ? 11 + 0.0045 * n : T >= 256 ? 13 + 0.008 * n : 16 + 0.013 * n;
-    return T >= 512 ? 25 + 0.0092 * n : T >= 256 ? 26 + 0.0125 * n : 27 + 0.022 * n;
-  }
-  // (on lattice rows, pairs of words: 8^2 sites 5, 32^2 10; two pairs 7, 17)
-  static double fused_us(const PtJob& j) {
-    if (j.rows)
-      return 3 + 1.8 * ((j.C + 1) / 2 * j.wpc) + 2e-3 * j.n * j.nw + 2.4e-5 * ((double)j.n * j.C * j.ntp);
-    const double nr = (double)j.n * j.C * j.ntp;
-    return 12 + nr * (j.msc ? 0.16e-3 : j.F.udeg ? 1.2e-3 : j.n > 2048 ? 2.3e-3 : 2e-3);
-  }
   // What the plans of a step need of a run in the ladder form.
   static constexpr uint32_t LAD_T[3] = {512, 256, 128};
   struct LadCost {
@@ -1243,6 +1290,7 @@ struct ChunkRunner {
   struct LadPick {
     LadGroup G;
     double us = 0.0;
+    double fill = 0.0;  // the part of the GPU that its CTAs take
     size_t reach = 0;
   };
   static LadPick ladder_group(const tamc_gpu* g, const std::vector<LadCost>& runs, size_t k, size_t k1) {
@@ -1276,6 +1324,7 @@ struct ChunkRunner {
       if (!best.G.count || (all && (!best_all || us < best.us)) || (!all && !best_all && rate > best_rate)) {
         best.G = G;
         best.us = us;
+        best.fill = (double)G.grid / room;
         best_rate = rate;
         best_all = all;
       }
@@ -1304,7 +1353,13 @@ struct ChunkRunner {
       most[x] = std::max(most[x + 1], us);
       sum[x] = sum[x + 1] + us;
     }
-    auto fused_from = [&](size_t x) { return std::max(most[x], sum[x] / g->num_sms); };
+    // other contexts' runs are taken to be about as many and as large as these (ms,
+    // ladder / fused: batches of 8 QUBOs of 600 sites 38 / 79, four at once 147 / 80,
+    // 16 584 / 333; servers of 24 QUBOs 56 / 223, four 206 / 226, eight 521 / 413)
+    const double crowd = 1.0 + contexts_beside(g);
+    // (a step in two parts waits for the other contexts' twice)
+    split = split && crowd == 1.0;
+    auto fused_from = [&](size_t x) { return std::max(most[x], crowd * sum[x] / g->num_sms); };
     const bool force = f && !strcmp(f, "ladder");
     best.us = force ? 1e30 : 0.9 * fused_from(0);
     std::vector<LadCost> runs;
@@ -1325,7 +1380,7 @@ struct ChunkRunner {
         }
         if (!p.G.count) break;
         P.groups.push_back(p.G);
-        P.us += p.us;
+        P.us += p.us * std::max(1.0, p.fill * crowd);
         P.ladder += p.G.count;
       }
       if (P.ladder < k1) break;
@@ -1614,7 +1669,10 @@ int tamc_gpu_batch_run(tamc_batch* b) {
   TraceRange tr("tamc batch run");
   if (!b) fail(TAMC_E_INVAL, "null batch");
   TAMC_CUDA(cudaSetDevice(b->g->device));
-  b->runner->run_all(b->g, b->jobs, b->chunk);
+  {
+    const InProgress busy(b->g);
+    b->runner->run_all(b->g, b->jobs, b->chunk);
+  }
   b->logs_pending = true;  // drained, all runs at once, by the first log read
   b->acc_pending = true;
   TAMC_API_END

@@ -18,6 +18,7 @@
 #include <cstring>
 #include <deque>
 #include <map>
+#include <memory>
 #include <string>
 
 #include "fast_pt.cuh"
@@ -88,6 +89,11 @@ struct tamc_server {
   std::vector<Request*> active;
   std::map<uint64_t, Request*> all;
   ChunkRunner* runner = nullptr;
+  std::unique_ptr<InProgress> busy;  // while requests are active
+  void mark() {
+    if (active.empty()) busy.reset();
+    else if (!busy) busy = std::make_unique<InProgress>(g);
+  }
   ~tamc_server() {
     for (auto& kv : all) {
       Request* r = kv.second;
@@ -265,6 +271,7 @@ int tamc_serve_step(tamc_server* s, uint32_t* active, uint32_t* queued) {
       s->active.push_back(r);
     }
   }
+  s->mark();
   if (!s->active.empty()) {
     std::vector<tamc_pt*> pts;
     for (auto* r : s->active) pts.push_back(r->pt);
@@ -278,6 +285,7 @@ int tamc_serve_step(tamc_server* s, uint32_t* active, uint32_t* queued) {
       else keep.push_back(r);
     }
     s->active.swap(keep);
+    s->mark();
   }
   if (active) *active = (uint32_t)s->active.size();
   if (queued) *queued = (uint32_t)s->queue.size();
@@ -323,6 +331,7 @@ int tamc_serve_cancel(tamc_server* s, uint64_t request_id) {
     // steps run synchronously: between calls no launch of this request is in flight
     TAMC_CUDA(cudaSetDevice(s->g->device));
     s->active.erase(std::find(s->active.begin(), s->active.end(), r));
+    s->mark();
     retire(s, r, TAMC_REQ_CANCELLED);
   } else {
     fail(TAMC_E_INVAL, "request already ended");

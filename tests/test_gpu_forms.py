@@ -2,6 +2,7 @@
 other test files reach, from the lines that TAMC_DEBUG=1 prints: a dispatch rule
 that sent them elsewhere would leave those comparing a kernel with itself."""
 import re
+import threading
 
 import numpy as np
 import pytest
@@ -247,3 +248,62 @@ def test_server_budget_covers_the_ladder_form(tb, gpu, monkeypatch, capfd, kind)
     assert planned() == (1, 1)
     assert srv.step() == (2, 0) and planned() == (2, 0)
     ladder._same(results(srv, ids), got)
+
+
+# rounds in the ladder form, then beside many other runs in the fused form, then in the ladder form again
+@pytest.mark.parametrize("kind,nt", [("qubo:300", 24), ("gauss2:17", 32), ("pm3:10", 32)])
+def test_rounds_beside_other_runs(tb, gpu, monkeypatch, capfd, kind, nt):
+    d = gpu.upload(ladder._host(tb, kind))
+    p = tb.PtParams(60, tb.geometric_betas(0.2, 5.0, nt), nt // 3, 0.2, True, 2, 8, 7, 9, 0)
+    r = tb.PtRun(d, p, 11).run(20)
+    monkeypatch.setenv("TAMC_PT_BESIDE", "1000")
+    r.run(45)
+    monkeypatch.delenv("TAMC_PT_BESIDE")
+    got = ladder._everything(r.run())
+    err = capfd.readouterr().err
+    assert re.findall(r"\[tamc\] PT run .*: (\w+),", err) == ["ladder"]
+    assert re.findall(r"\[tamc\] rounds (\d+) to (\d+) in the fused form beside 1000 contexts", err) == [("20", "45")]
+    monkeypatch.setenv("TAMC_PT_FORM", "fused")
+    ladder._same(ladder._everything(tb.PtRun(d, p, 11).run()), got)
+
+
+def test_several_contexts_at_once(tb, gpu):
+    """Single runs in the ladder form, a batch and a server on contexts of their own,
+    each in a thread, against the same work one after another."""
+    kinds = ["qubo:300", "gauss3:8", "rrg:130", "gauss2:17"]
+    p = tb.PtParams(300, tb.geometric_betas(0.2, 5.0, 16), 5, 0.5, True, 2, 8)
+
+    def single(kind):
+        def work(g):
+            return ladder._everything(tb.PtRun(g.upload(ladder._host(tb, kind)), p, 3).run())
+        return work
+
+    def batch(g):
+        b = tb.Batch(g)
+        for d in g.upload_many([ladder._host(tb, k) for k in kinds + ["pm2:16", "pm2:12"]]):
+            b.add(d, p, 3)
+        b.run()
+        return [x for k in range(6) for x in b.state(k)]
+
+    def serve(g):
+        srv = tb.Server(g, 8 << 30, 64, 60)
+        ids = [srv.submit(ladder._host(tb, k), p, 3) for k in kinds]
+        while any(srv.step()):
+            pass
+        return [x for i in ids for x in srv.state(i)]
+
+    work = [single(k) for k in kinds] * 2 + [batch, serve]
+    want = [w(gpu) for w in work]
+    got = [None] * len(work)
+
+    def thread(k, g):
+        got[k] = work[k](g)
+
+    contexts = [tb.Gpu(0) for _ in work]
+    threads = [threading.Thread(target=thread, args=(k, g)) for k, g in enumerate(contexts)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for a, b in zip(want, got):
+        ladder._same(a, b)
