@@ -125,7 +125,7 @@ static float time_tile(tamc_gpu* g, const PtJob& proto, TileChoice t, uint32_t r
     TAMC_CUDA(tamc::copy_async(dj.p, &j, sizeof(PtJob), cudaMemcpyHostToDevice, st));
     ctr.zero(st);
     TAMC_CUDA(cudaEventRecord(e0, st));
-    fused_launch(st, dj.p, 1, ctr.p, 1, t.T, smem, j.rows);
+    fused_launch(st, dj.p, 1, ctr.p, 1, t.T, smem, j.rows ? FUSED_ROWS : FUSED_GENERAL);
     TAMC_CUDA(cudaEventRecord(e1, st));
     g->count();
     TAMC_CUDA(cudaEventSynchronize(e1));  // also keeps the host copy of j unchanged until it is read
@@ -300,7 +300,7 @@ static void launch_one(tamc_pt* pt, uint32_t begin, uint32_t end, int init) {
   j.s_base = pt->s_next;
   TAMC_CUDA(tamc::copy_async(F->d_job.p, &j, sizeof(PtJob), cudaMemcpyHostToDevice, st));
   F->ctr.zero(st);
-  fused_launch(st, F->d_job.p, 1, F->ctr.p, 1, F->T, F->smem, F->job.rows);
+  fused_launch(st, F->d_job.p, 1, F->ctr.p, 1, F->T, F->smem, F->job.rows ? FUSED_ROWS : FUSED_GENERAL);
   pt->g->count();
   // the job struct is read by the kernel; keep the host copy alive until done
   TAMC_CUDA(cudaStreamSynchronize(st));
@@ -1004,7 +1004,7 @@ struct ChunkRunner {
     uint32_t T = 0, grid = 0;
     size_t smem = 0;
     int per_sm = 0;
-    bool rows = true;  // every run is on lattice rows
+    FusedKind kind = FUSED_GENERAL;
   };
   static Launch shape(tamc_gpu* g, std::vector<tamc_pt*>& grp, uint32_t T) {
     const char* csr_env = getenv("TAMC_PT_CSR");
@@ -1029,8 +1029,10 @@ struct ChunkRunner {
     Launch L;
     L.T = T;
     L.smem = smem;
-    for (auto* pt : grp) L.rows = L.rows && pt->fast->job.rows;
-    L.per_sm = fused_blocks_per_sm(T, smem, L.rows);
+    size_t on_rows = 0;
+    for (auto* pt : grp) on_rows += pt->fast->job.rows != 0;
+    L.kind = on_rows == grp.size() ? FUSED_ROWS : on_rows ? FUSED_MIXED : FUSED_GENERAL;
+    L.per_sm = fused_blocks_per_sm(T, smem, L.kind);
     L.grid = std::min<uint32_t>((uint32_t)grp.size(), (uint32_t)(g->num_sms * std::max(L.per_sm, 1)));
     return L;
   }
@@ -1163,20 +1165,21 @@ struct ChunkRunner {
     // the kernel launches of one chunk (both classes, or one launch)
     auto launch_all = [&]() {
       if (!split) {
-        fused_launch(st, d_jobs.p, na, ctr.p, A.grid, A.T, A.smem, A.rows);
+        fused_launch(st, d_jobs.p, na, ctr.p, A.grid, A.T, A.smem, A.kind);
         return;
       }
-      fused_smem_limit(std::max(A.smem, B.smem), A.rows);
-      if (B.rows != A.rows) fused_smem_limit(B.smem, B.rows);
+      fused_smem_limit(std::max(A.smem, B.smem), A.kind);
+      if (B.kind != A.kind) fused_smem_limit(B.smem, B.kind);
       TAMC_CUDA(cudaEventRecord(fork, st));
       TAMC_CUDA(cudaStreamWaitEvent(aux, fork, 0));
-      fused_launch_prio(st, d_jobs.p, nb, ctr.p, A.grid, A.T, A.smem, prio_hi, A.rows);
-      fused_launch_prio(aux, d_jobs.p + nb, na - nb, ctr.p + 1, B.grid, B.T, B.smem, prio_lo, B.rows);
+      fused_launch_prio(st, d_jobs.p, nb, ctr.p, A.grid, A.T, A.smem, prio_hi, A.kind);
+      fused_launch_prio(aux, d_jobs.p + nb, na - nb, ctr.p + 1, B.grid, B.T, B.smem, prio_lo, B.kind);
       TAMC_CUDA(cudaEventRecord(join, aux));
       TAMC_CUDA(cudaStreamWaitEvent(st, join, 0));
     };
     if (use_graph) {
-      const uint32_t key[8] = {na, nb, A.grid, 2 * A.T + A.rows, (uint32_t)A.smem, B.grid, 2 * B.T + B.rows, (uint32_t)B.smem};
+      const uint32_t key[8] = {na, nb, A.grid, 4 * A.T + A.kind, (uint32_t)A.smem,
+                               B.grid, 4 * B.T + B.kind, (uint32_t)B.smem};
       if (!sl.exec || memcmp(key, sl.key, sizeof(key)) != 0) {
         if (sl.exec) cudaGraphExecDestroy(sl.exec);
         if (sl.graph) cudaGraphDestroy(sl.graph);

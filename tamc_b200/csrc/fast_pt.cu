@@ -2240,6 +2240,9 @@ __global__ void __launch_bounds__(768, 1) k_pt_rows(const PtJob* __restrict__ jo
   }
 }
 
+// (The call costs the general path registers even where no job takes it: 128 fully
+// connected sites, 4 x 3 replicas 455 us a round without it, 503 with it.)
+template <bool MIXED>
 __global__ void __launch_bounds__(512, 1) k_pt_fused(const PtJob* __restrict__ jobs, uint32_t njobs, uint32_t* ctr) {
   extern __shared__ uint4 smem_u4[];
   __shared__ uint32_t s_job;
@@ -2251,7 +2254,7 @@ __global__ void __launch_bounds__(512, 1) k_pt_fused(const PtJob* __restrict__ j
     __syncthreads();
     if (jid >= njobs) break;
     load_job(s_J, jobs + jid);
-    if (s_J.rows) run_rows_call();
+    if (MIXED && s_J.rows) run_rows_call();
     else if (s_J.self_loops) run_job<true>(s_J, reinterpret_cast<char*>(smem_u4));
     else run_job<false>(s_J, reinterpret_cast<char*>(smem_u4));
   }
@@ -3432,23 +3435,27 @@ size_t fused_smem_bytes(const PtJob& j, uint32_t T, bool csr_smem) {
 
 // The fused kernels' dynamic shared-memory limits only grow (per device), so
 // that a captured launch stays valid whatever smaller launches ran since.
-static void fused_attr(size_t smem, bool rows) {
+using FusedFn = void (*)(const PtJob*, uint32_t, uint32_t*);
+static FusedFn fused_fn(FusedKind kind) {
+  return kind == FUSED_ROWS ? k_pt_rows : kind == FUSED_MIXED ? k_pt_fused<true> : k_pt_fused<false>;
+}
+static void fused_attr(size_t smem, FusedKind kind) {
   static std::mutex mu;
-  static std::map<std::pair<int, bool>, size_t> set;
+  static std::map<std::pair<int, FusedKind>, size_t> set;
   int dev = 0;
   TAMC_CUDA(cudaGetDevice(&dev));
   std::lock_guard<std::mutex> lk(mu);
-  size_t& cur = set[{dev, rows}];
+  size_t& cur = set[{dev, kind}];
   if (smem > cur) {
-    TAMC_CUDA(cudaFuncSetAttribute(rows ? k_pt_rows : k_pt_fused, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    TAMC_CUDA(cudaFuncSetAttribute(fused_fn(kind), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     cur = smem;
   }
 }
 
-int fused_blocks_per_sm(uint32_t T, size_t smem, bool rows) {
-  fused_attr(smem, rows);
+int fused_blocks_per_sm(uint32_t T, size_t smem, FusedKind kind) {
+  fused_attr(smem, kind);
   int nb = 0;
-  TAMC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, rows ? k_pt_rows : k_pt_fused, (int)T, smem));
+  TAMC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fused_fn(kind), (int)T, smem));
   return nb;
 }
 
@@ -3695,15 +3702,14 @@ void plain_launch_init(cudaStream_t st, const PtJob* d_job, long long* acc, int 
 }
 
 void fused_launch(cudaStream_t st, const PtJob* d_jobs, uint32_t njobs, uint32_t* ctr, uint32_t grid, uint32_t T,
-                  size_t smem, bool rows) {
-  fused_attr(smem, rows);
-  if (rows) k_pt_rows<<<grid, T, smem, st>>>(d_jobs, njobs, ctr);
-  else k_pt_fused<<<grid, T, smem, st>>>(d_jobs, njobs, ctr);
+                  size_t smem, FusedKind kind) {
+  fused_attr(smem, kind);
+  fused_fn(kind)<<<grid, T, smem, st>>>(d_jobs, njobs, ctr);
   TAMC_CUDA(cudaGetLastError());
 }
 
 void fused_launch_prio(cudaStream_t st, const PtJob* d_jobs, uint32_t njobs, uint32_t* ctr, uint32_t grid, uint32_t T,
-                       size_t smem, int priority, bool rows) {
+                       size_t smem, int priority, FusedKind kind) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(T);
@@ -3714,9 +3720,9 @@ void fused_launch_prio(cudaStream_t st, const PtJob* d_jobs, uint32_t njobs, uin
   at[0].val.priority = priority;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  TAMC_CUDA(cudaLaunchKernelEx(&cfg, rows ? k_pt_rows : k_pt_fused, d_jobs, njobs, ctr));
+  TAMC_CUDA(cudaLaunchKernelEx(&cfg, fused_fn(kind), d_jobs, njobs, ctr));
 }
 
-void fused_smem_limit(size_t smem, bool rows) { fused_attr(smem, rows); }
+void fused_smem_limit(size_t smem, FusedKind kind) { fused_attr(smem, kind); }
 
 }  // namespace tamc

@@ -45,20 +45,21 @@ enum { PHASE_ICM_SCAN, PHASE_ICM_INIT, PHASE_ICM_JUMP, PHASE_ICM_GROW, PHASE_ICM
 
 // Whether the fused kernel runs the job on lattice rows (PtJob::rows).
 bool fused_rows(const PtJob& j);
+// The kernel of a fused launch, by its jobs: none, all or some of them on lattice rows.
+enum FusedKind { FUSED_GENERAL = 0, FUSED_ROWS, FUSED_MIXED };
 // Shared-memory bytes the fused kernel needs for a job with T threads.
 size_t fused_smem_bytes(const PtJob& j, uint32_t T, bool csr_smem);
-// Resident CTAs per SM for the fused kernel at this size (`rows`, here and
-// below: the kernel of launches whose jobs are all on lattice rows).
-int fused_blocks_per_sm(uint32_t T, size_t smem, bool rows);
+// Resident CTAs per SM for the fused kernel at this size.
+int fused_blocks_per_sm(uint32_t T, size_t smem, FusedKind kind);
 // Launch over `njobs` jobs already on the device; `ctr` is a zeroed counter.
 void fused_launch(cudaStream_t st, const PtJob* d_jobs, uint32_t njobs, uint32_t* ctr, uint32_t grid,
-                  uint32_t T, size_t smem, bool rows);
+                  uint32_t T, size_t smem, FusedKind kind);
 // A fused launch with a launch priority (cudaLaunchAttributePriority; lower
 // numbers run first); the shared-memory attribute must already cover `smem`
 // (fused_smem_limit).
 void fused_launch_prio(cudaStream_t st, const PtJob* d_jobs, uint32_t njobs, uint32_t* ctr, uint32_t grid, uint32_t T,
-                       size_t smem, int priority, bool rows);
-void fused_smem_limit(size_t smem, bool rows);
+                       size_t smem, int priority, FusedKind kind);
+void fused_smem_limit(size_t smem, FusedKind kind);
 
 // Plain form (one instance over the whole GPU, one launch per sweep phase).
 struct PlainCtl {
