@@ -250,6 +250,32 @@ __device__ __forceinline__ uint64_t serial_swaps(uint32_t nt, const float* des0,
   return (uint64_t)__ballot_sync(0xffffffffu, d[0]) | ((uint64_t)__ballot_sync(0xffffffffu, d[1]) << 32);
 }
 
+// The same pair by pair (D0: the decisions without a carry): as many steps as pairs,
+// but each of less latency than one above.
+__device__ __forceinline__ uint64_t serial_walk(uint32_t nt, const float* des0, const float* db, const float* u,
+                                                uint64_t D0) {
+  uint64_t D = 0;
+  float carry = 0.0f;
+  bool prev = false;
+  for (uint32_t j = 0; j + 1 < nt; ++j) {  // warp-uniform: every lane walks the same values
+    const bool hi = j >= 32u;
+    const float e = __shfl_sync(0xffffffffu, hi ? des0[1] : des0[0], j & 31u);
+    const float b = __shfl_sync(0xffffffffu, hi ? db[1] : db[0], j & 31u);
+    const float uj = __shfl_sync(0xffffffffu, hi ? u[1] : u[0], j & 31u);
+    float des = e;
+    bool dj = (D0 >> j) & 1ull;
+    if (prev) {
+      des = e + carry;
+      const float dlt = b * des;
+      dj = dlt >= 0.0f || uj < __expf(dlt);
+    }
+    if (dj) D |= 1ull << j;
+    prev = dj;
+    carry = des;
+  }
+  return D;
+}
+
 // ------------------------------------------------- multi-spin coding ----
 // For +-J instances (every J = +-1, no field, rows of DEG = 4 or 6 entries) a
 // site update acts on the 32 replicas of one word at once.  Bond (s, j) is

@@ -143,3 +143,17 @@ def test_several_runs_in_the_ladder_form_equal_the_fused_form(tb, gpu, monkeypat
     if polls:
         monkeypatch.setenv("TAMC_LADDER_POLLS", polls)
     _same(want, run())
+
+
+# serial exchange with few and with most pairs swapping: the fused form walks the
+# pairs in the second, the ladder form never does
+@pytest.mark.parametrize("nt", [2, 6, 7, 8, 32, 33, 34, 64])
+@pytest.mark.parametrize("hi", [0.02, 0.5, 5.0])
+def test_serial_exchange_of_ladder_and_fused_forms_identical(tb, gpu, monkeypatch, nt, hi):
+    d = gpu.upload(_host(tb, "qubo:61"))
+    p = tb.PtParams(80, tb.geometric_betas(0.01, hi, nt), nt // 2, 0.0, True, 2, 1, 7, 9, 0)
+    got = {}
+    for form in ("fused", "ladder"):
+        monkeypatch.setenv("TAMC_PT_FORM", form)
+        got[form] = _everything(tb.PtRun(d, p, 5).run())
+    _same(got["fused"], got["ladder"])
