@@ -544,25 +544,40 @@ static bool sa_rule(const tamc_gpu* g, const FastInst& F, uint32_t R, uint32_t l
 
 // Heuristic tile.  Rows of 3 or 4 entries take the table kernel where its table
 // fits (the one with the site's own spin in it first), rows of uneven length the
-// sliced one.  3-regular instances stay with the words where SMs have few warps
-// of work, whose latency the table does not shorten (300 sites, 100 restarts:
-// 393 us against 407), and above 2600 sites, where only the smaller table fits
-// (2700 sites, 800 restarts: 1141 us against 1359).  For the words: 256
-// threads and the smallest replica group (quads per CTA) that gives no SM more
-// than two CTAs.
+// sliced one, but for these, where k_sa_fast took less time (that / the other; QUBOs
+// of 6 entries a row and 3-regular instances, 30 to 100 sweeps):
+// * 3-regular instances where SMs have few warps of work, whose latency the table does
+//   not shorten (300 sites, 100 restarts: 393 us / 407), above 2600 sites, where only
+//   the smaller table fits (2700 sites, 800 restarts: 1141 / 1359), where the CTAs
+//   that an SM needs do not fit beside one another (2600 sites, 600 restarts: 609 /
+//   665, 2048 restarts 762 / 888), and with five to eight quads on an SM (4096
+//   restarts of 300, 1000 and 2000 sites: 352 / 376, 651 / 698, 787 / 897);
+// * more than four quads on an SM, where issue and not latency bounds, and many lanes
+//   without work: classes well below 32 sites (rows of 3 or 4, 16384 restarts: 64 sites
+//   in classes of 16 295 / 380, 16 in classes of 8 154 / 229; 64 in classes of 32 297 /
+//   248), slices padded to more than 1.6 times the entries (8192 restarts: 30 sites 426
+//   / 638, 251 sites 967 / 1176, a star of 300 1130 / 1829; 700 sites, padded to 1.44
+//   times, 1277 / 1303, 2000 sites 2121 / 1909).
+// For the words: 256 threads and the smallest replica group (quads per CTA) that gives
+// no SM more than two CTAs.
 static SaTile heuristic(const tamc_gpu* g, const FastInst& F, uint32_t R, uint32_t largest_class) {
   SaTile t;
-  const uint32_t Q = (R + 3) / 4, sms = (uint32_t)g->num_sms;
-  const uint32_t warps = (Q + sms - 1) / sms * ((largest_class + 31) / 32);  // of 32 sites x a quad, busiest SM
+  const uint32_t Q = (R + 3) / 4, sms = (uint32_t)g->num_sms, per = (largest_class + 31) / 32 * 32;
+  const uint32_t quads = (Q + sms - 1) / sms;  // of the busiest SM
   const char* env = getenv("TAMC_SA_KERNEL");  // "words": k_sa_fast whatever the rows (tests, profiling)
   const bool words = env && !strcmp(env, "words");
-  if (!words && (F.udeg == 4 || (F.udeg == 3 && warps >= 10))) {
+  const bool many = quads > 4;
+  if (words) {
+  } else if (F.udeg == 4 || (F.udeg == 3 && quads * (per / 32) >= 10)) {
     t.kind = SA_TABLE;
+    const bool idle = many && (uint64_t)F.ncolors * per * 2 > 3ull * F.n;
     for (bool half : {false, true}) {
       t.smem_csr = half;
-      if (!(half && F.udeg == 3) && sa_rule(g, F, R, largest_class, t)) return t;
+      if (idle || (half && F.udeg == 3) || !sa_rule(g, F, R, largest_class, t)) continue;
+      const uint32_t beside = t.nq * (uint32_t)std::max<size_t>(1, std::min<size_t>(g->smem_optin / t.smem, 1024 / t.T));
+      if (F.udeg == 4 || (many ? quads > 8 && beside >= 4 : quads <= beside)) return t;
     }
-  } else if (!words && F.sl_ent) {
+  } else if (F.sl_ent && !(many && 32ull * F.sl_rows * 5 > 8 * F.nnz)) {
     t.kind = SA_SLICED;
     for (bool rows : {true, false}) {
       t.smem_csr = rows;

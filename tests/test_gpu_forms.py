@@ -307,3 +307,16 @@ def test_several_contexts_at_once(tb, gpu):
         t.join()
     for a, b in zip(want, got):
         ladder._same(a, b)
+
+
+# many restarts on an SM and few sites a class or padded slices, 3-regular instances
+# whose CTAs do not fit beside one another: words (0), else table (1) and slices (2)
+@pytest.mark.parametrize("kind,size,R,kernel", [
+    ("gauss2", 4, 2368, 1), ("gauss2", 4, 2372, 0), ("gauss2", 8, 16384, 1), ("rrg", 2000, 2048, 1),
+    ("rrg", 2000, 4096, 0), ("rrg", 2000, 16384, 1), ("rrg", 2400, 1024, 1), ("rrg", 2400, 2048, 0),
+    ("rrg", 2600, 592, 1), ("rrg", 2600, 600, 0), ("qubo", 30, 2368, 2), ("qubo", 30, 2372, 0),
+    ("qubo", 1000, 8192, 2),
+])
+def test_annealing_kernel_for_many_restarts(tb, gpu, capfd, kind, size, R, kernel):
+    tb.sa_run(gpu.upload(sa._host(tb, kind, size)), np.linspace(0.1, 2.0, 8).astype(np.float32), R, 1, 5)
+    assert _printed(capfd, r"\[tamc\] SA tile .*: kernel (\d)") == [str(kernel)]
