@@ -546,6 +546,9 @@ static bool sa_rule(const tamc_gpu* g, const FastInst& F, uint32_t R, uint32_t l
 // fits (the one with the site's own spin in it first), rows of uneven length the
 // sliced one, but for these, where k_sa_fast took less time (that / the other; QUBOs
 // of 6 entries a row and 3-regular instances, 30 to 100 sweeps):
+// * fewer than four sweeps, which do not pay for the tables or the larger code (a sweep
+//   of 30 sites, 4 restarts 58 us / 71, of 251 sites 58 / 70, of 2000 sites, 700
+//   restarts 110 / 117; five sweeps 76 / 82, 93 / 84, 151 / 154);
 // * 3-regular instances where SMs have few warps of work, whose latency the table does
 //   not shorten (300 sites, 100 restarts: 393 us / 407), above 2600 sites, where only
 //   the smaller table fits (2700 sites, 800 restarts: 1141 / 1359), where the CTAs
@@ -560,12 +563,12 @@ static bool sa_rule(const tamc_gpu* g, const FastInst& F, uint32_t R, uint32_t l
 //   times, 1277 / 1303, 2000 sites 2121 / 1909).
 // For the words: 256 threads and the smallest replica group (quads per CTA) that gives
 // no SM more than two CTAs.
-static SaTile heuristic(const tamc_gpu* g, const FastInst& F, uint32_t R, uint32_t largest_class) {
+static SaTile heuristic(const tamc_gpu* g, const FastInst& F, uint32_t R, uint32_t largest_class, uint32_t nbeta) {
   SaTile t;
   const uint32_t Q = (R + 3) / 4, sms = (uint32_t)g->num_sms, per = (largest_class + 31) / 32 * 32;
   const uint32_t quads = (Q + sms - 1) / sms;  // of the busiest SM
   const char* env = getenv("TAMC_SA_KERNEL");  // "words": k_sa_fast whatever the rows (tests, profiling)
-  const bool words = env && !strcmp(env, "words");
+  const bool words = (env && !strcmp(env, "words")) || nbeta < 4;
   const bool many = quads > 4;
   if (words) {
   } else if (F.udeg == 4 || (F.udeg == 3 && quads * (per / 32) >= 10)) {
@@ -608,8 +611,8 @@ static SaTile heuristic(const tamc_gpu* g, const FastInst& F, uint32_t R, uint32
 static std::mutex g_sa_mu;
 static std::map<std::tuple<int, uint32_t, uint32_t, uint32_t>, SaTile> g_sa_tune;
 
-SaTile sa_fast_choose(tamc_gpu* g, const FastInst& F, uint32_t R, uint32_t largest_class) {
-  SaTile best = heuristic(g, F, R, largest_class);
+SaTile sa_fast_choose(tamc_gpu* g, const FastInst& F, uint32_t R, uint32_t largest_class, uint32_t nbeta) {
+  SaTile best = heuristic(g, F, R, largest_class, nbeta);
   const auto key = std::make_tuple(g->device, F.n, F.nnz, R);
   if (best.kind == SA_WORDS) {
     std::lock_guard<std::mutex> lk(g_sa_mu);
@@ -740,8 +743,8 @@ void sa_fast_launch(cudaStream_t st, const SaFastArgs& a, const SaTile& t) {
   }
 }
 
-SaTile sa_fast_peek(const tamc_gpu* g, const FastInst& F, uint32_t R, uint32_t largest_class) {
-  const SaTile t = heuristic(g, F, R, largest_class);
+SaTile sa_fast_peek(const tamc_gpu* g, const FastInst& F, uint32_t R, uint32_t largest_class, uint32_t nbeta) {
+  const SaTile t = heuristic(g, F, R, largest_class, nbeta);
   if (t.kind == SA_WORDS) {
     std::lock_guard<std::mutex> lk(g_sa_mu);
     auto it = g_sa_tune.find(std::make_tuple(g->device, F.n, F.nnz, R));

@@ -27,13 +27,13 @@ struct SaTile {
 };
 
 // (`largest_class`: sites of the largest colour class)
-SaTile sa_fast_choose(tamc_gpu* g, const FastInst& F, uint32_t R, uint32_t largest_class);
+SaTile sa_fast_choose(tamc_gpu* g, const FastInst& F, uint32_t R, uint32_t largest_class, uint32_t nbeta);
 // Device-side conversion of SA words to the reference's packed byte layout.
 void sa_pack_states(cudaStream_t st, const uint32_t* words, uint32_t n, uint32_t R, uint8_t* out);
 void sa_fast_launch(cudaStream_t st, const SaFastArgs& a, const SaTile& t);
 // The tile sa_fast_choose has cached for this shape, else the heuristic tile;
 // never times candidates, so it launches and allocates nothing.
-SaTile sa_fast_peek(const tamc_gpu* g, const FastInst& F, uint32_t R, uint32_t largest_class);
+SaTile sa_fast_peek(const tamc_gpu* g, const FastInst& F, uint32_t R, uint32_t largest_class, uint32_t nbeta);
 // Sites of the instance's largest colour class.
 inline uint32_t largest_class(const tamc_inst* d) {
   uint32_t m = 1;

@@ -101,7 +101,7 @@ int tamc_gpu_sa_run(tamc_inst* inst, const float* betas, uint32_t nbeta, uint32_
     a.init_words = nullptr;
     a.words_out = sc.words;
     a.energies_out = sc.energies;
-    const SaTile t = sa_fast_choose(g, a.F, R, largest_class(inst));
+    const SaTile t = sa_fast_choose(g, a.F, R, largest_class(inst), nbeta);
     sa_fast_launch(st, a, t);
     sa_pack_states(st, sc.words, n, R, sc.packed);
     g->count(2);
@@ -174,7 +174,7 @@ int tamc_gpu_sa_run_device(tamc_inst* inst, const float* d_betas, uint32_t nbeta
   a.init_words = nullptr;
   a.words_out = d_words;
   a.energies_out = d_energies;
-  const SaTile t = sa_fast_choose(g, a.F, R, largest_class(inst));
+  const SaTile t = sa_fast_choose(g, a.F, R, largest_class(inst), nbeta);
   sa_fast_launch(st, a, t);
   g->count();
   TAMC_API_END

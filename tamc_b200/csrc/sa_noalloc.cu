@@ -59,7 +59,7 @@ int tamc_gpu_sa_run_noalloc(tamc_inst* inst, const float* d_betas, uint32_t nbet
   SaFastArgs a;
   a.F = make_fast_inst(inst);
   // the shared-memory check sa_fast_choose makes, before anything is queued
-  const SaTile tile = sa_fast_peek(g, a.F, R, largest_class(inst));
+  const SaTile tile = sa_fast_peek(g, a.F, R, largest_class(inst), nbeta);
   if (tile.smem > g->smem_optin) fail(TAMC_E_UNSUPPORTED, "instance too large for the fast SA kernel");
   TAMC_CUDA(cudaSetDevice(g->device));
   uint32_t* words = words_on(g->device);

@@ -113,7 +113,7 @@ def test_form_of_the_lattice_rows(tb, gpu, monkeypatch, capfd, L, nt, C, threads
 @pytest.mark.parametrize("kind,size,R", _cases(sa.test_annealing_kernels_identical))
 def test_kernel_of_the_annealing_cases(tb, gpu, capfd, kind, size, R):
     h = sa._host(tb, kind, size)
-    tb.sa_run(gpu.upload(h), np.array([0.5], np.float32), R, 1, 5)
+    tb.sa_run(gpu.upload(h), np.linspace(0.1, 6.0, 23).astype(np.float32), R, 1, 5)
     # 0 words, 1 table, 2 slices.  Rows of 4: the table, which at 64 x 64 sites does
     # not fit; rows of 3: the table where the busiest of 148 SMs has ten warps of
     # work (32 sites of the largest class x 4 restarts); uneven rows: slices
@@ -320,3 +320,16 @@ def test_several_contexts_at_once(tb, gpu):
 def test_annealing_kernel_for_many_restarts(tb, gpu, capfd, kind, size, R, kernel):
     tb.sa_run(gpu.upload(sa._host(tb, kind, size)), np.linspace(0.1, 2.0, 8).astype(np.float32), R, 1, 5)
     assert _printed(capfd, r"\[tamc\] SA tile .*: kernel (\d)") == [str(kernel)]
+
+
+@pytest.mark.parametrize("kind,kernel", [("gauss2", 1), ("qubo", 2)])
+def test_annealing_kernel_of_few_sweeps(tb, gpu, monkeypatch, capfd, kind, kernel):
+    d = gpu.upload(sa._host(tb, kind, 30))
+    got = []
+    for nbeta in (0, 3, 4, 4):
+        if len(got) == 3:
+            monkeypatch.setenv("TAMC_SA_KERNEL", "words")
+        got.append(tb.sa_run(d, np.linspace(0.1, 6.0, nbeta).astype(np.float32), 40, 1, 5))
+    # (the words kernel's tile is printed when it is chosen, at the first call)
+    assert _printed(capfd, r"\[tamc\] SA tile .*: kernel (\d)") == ["0", str(kernel)]
+    assert got[2][0].tobytes() == got[3][0].tobytes() and got[2][1].tobytes() == got[3][1].tobytes()
