@@ -2,7 +2,6 @@
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
-#include <functional>
 #include <map>
 #include <mutex>
 #include <string>
@@ -337,13 +336,18 @@ void inst_drop_slices(tamc_inst* d) {
 // times what they take.)
 uint64_t slices_bytes(const HostInstance& h) {
   const uint64_t n = h.n, nnz = h.col.size();
-  std::vector<uint32_t> len(h.n);
-  for (uint32_t i = 0; i < h.n; ++i) len[i] = h.row_ptr[i + 1] - h.row_ptr[i];
-  std::sort(len.begin(), len.end(), std::greater<uint32_t>());
-  if (!n || !wants_slices(h.n, len.front() == len.back() ? len.front() : 0u, h.has_self_loops())) return 0;
-  uint64_t classes = 2, most = nnz + n;
-  while (classes < n && len[classes] >= classes) ++classes;
-  for (uint64_t c = 0; c < std::min(classes, n); ++c) most += 32 * (len[c] + 1);
+  std::vector<uint32_t> of;  // rows of each length
+  for (uint32_t i = 0; i < h.n; ++i) {
+    const uint32_t len = h.row_ptr[i + 1] - h.row_ptr[i];
+    if (len >= of.size()) of.resize(len + 1, 0);
+    ++of[len];
+  }
+  const uint64_t longest = of.size() - 1;
+  if (!n || !wants_slices(h.n, of.back() == n ? (uint32_t)longest : 0u, h.has_self_loops())) return 0;
+  uint64_t classes = 0, most = nnz + n;
+  for (uint64_t len = longest + 1; len-- > 0;)
+    for (uint64_t k = 0; k < of[len] && classes < n && (classes < 2 || len >= classes); ++k, ++classes)
+      most += 32 * (len + 1);
   const uint64_t entries = std::min<uint64_t>(most, std::max<uint64_t>(2 * nnz, 65536));
   return entries * 8 + (n + 32 * classes) * 2 + n * 2 + (classes + 1) * 4 + (n / 32 + classes + 1) * 4 + 5 * 256;
 }
@@ -599,10 +603,9 @@ void upload_instances(tamc_gpu* g, uint32_t count, const tamc_host_instance* con
     // on up to 16 threads: host preparation of every instance, then (after
     // the staging offsets are known) its copy into the pinned staging block
     // (packs 2 k and 2 k + 1: the arrays of instance k, its sliced rows)
-    const uint32_t parts = 2 * count;
-    std::vector<UploadPack> packs(parts);
-    std::vector<size_t> off(parts + 1, 0);
-    std::vector<std::exception_ptr> errs(parts);
+    std::vector<UploadPack> packs(2 * count);
+    std::vector<size_t> off(count + 1, 0);
+    std::vector<std::exception_ptr> errs(count);
     const uint32_t hw = std::max(1u, std::thread::hardware_concurrency());
     auto parallel = [&](uint32_t k0, uint32_t k1, auto&& f) {
       std::atomic<uint32_t> next{k0};
@@ -631,8 +634,10 @@ void upload_instances(tamc_gpu* g, uint32_t count, const tamc_host_instance* con
     parallel(0, count, [&](uint32_t k) {
       inst_prepare(ds[k], his[k]->h, packs[2 * k], !slices || slices[k] ? &packs[2 * k + 1] : nullptr);
     });
-    for (uint32_t k = 0; k < parts; ++k) off[k + 1] = off[k] + ((packs[k].host.size() + 255) & ~(size_t)255);
-    // staged in rounds of at most `cap` bytes (one pack at least): fill
+    auto up256 = [](size_t b) { return (b + 255) & ~(size_t)255; };
+    for (uint32_t k = 0; k < count; ++k)
+      off[k + 1] = off[k] + up256(packs[2 * k].host.size()) + up256(packs[2 * k + 1].host.size());
+    // staged in rounds of at most `cap` bytes (one instance at least): fill
     // the block, one device allocation and one asynchronous copy per pack
     // on the upload stream, one wait; the instances are complete on return,
     // as after tamc_gpu_instance_upload
@@ -640,9 +645,9 @@ void upload_instances(tamc_gpu* g, uint32_t count, const tamc_host_instance* con
     if (const char* e = getenv("TAMC_UPLOAD_STAGE_BYTES")) cap = std::max<size_t>(256, strtoull(e, nullptr, 10));
     std::lock_guard<std::mutex> lk(g->up_mu);
     if (!g->up_stream) TAMC_CUDA(cudaStreamCreateWithFlags(&g->up_stream, cudaStreamNonBlocking));
-    for (uint32_t k0 = 0, k1; k0 < parts; k0 = k1) {
+    for (uint32_t k0 = 0, k1; k0 < count; k0 = k1) {
       k1 = k0 + 1;
-      while (k1 < parts && off[k1 + 1] - off[k0] <= cap) ++k1;
+      while (k1 < count && off[k1 + 1] - off[k0] <= cap) ++k1;
       const size_t bytes = off[k1] - off[k0];
       if (bytes > g->up_pin_bytes) {
         if (g->up_pin) TAMC_CUDA(cudaFreeHost(g->up_pin));
@@ -652,14 +657,20 @@ void upload_instances(tamc_gpu* g, uint32_t count, const tamc_host_instance* con
         TAMC_CUDA(cudaHostAlloc((void**)&g->up_pin, want, cudaHostAllocDefault));
         g->up_pin_bytes = want;
       }
-      auto pin = [&](uint32_t k) { return g->up_pin + (off[k] - off[k0]); };
-      parallel(k0, k1, [&](uint32_t k) { memcpy(pin(k), packs[k].host.data(), packs[k].host.size()); });
-      for (uint32_t k = k0; k < k1; ++k) {
-        const size_t part = packs[k].host.size();
-        if (!part || !part_alloc(ds[k / 2], part, k % 2)) continue;
-        void* const arena = k % 2 ? ds[k / 2]->sl_arena : ds[k / 2]->arena;
-        TAMC_CUDA(copy_async(arena, pin(k), part, cudaMemcpyHostToDevice, g->up_stream));
-        packs[k].bind(arena);
+      // (pack p of instance p / 2)
+      auto pin = [&](uint32_t p) {
+        return g->up_pin + (off[p / 2] - off[k0]) + (p % 2 ? up256(packs[p - 1].host.size()) : 0);
+      };
+      parallel(k0, k1, [&](uint32_t k) {
+        for (uint32_t p : {2 * k, 2 * k + 1}) std::copy(packs[p].host.begin(), packs[p].host.end(), pin(p));
+      });
+      for (uint32_t p = 2 * k0; p < 2 * k1; ++p) {
+        tamc_inst* const d = ds[p / 2];
+        const size_t part = packs[p].host.size();
+        if (!part || !part_alloc(d, part, p % 2)) continue;
+        void* const arena = p % 2 ? d->sl_arena : d->arena;
+        TAMC_CUDA(copy_async(arena, pin(p), part, cudaMemcpyHostToDevice, g->up_stream));
+        packs[p].bind(arena);
       }
       TAMC_CUDA(cudaStreamSynchronize(g->up_stream));
     }
