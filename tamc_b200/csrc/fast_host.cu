@@ -1491,12 +1491,6 @@ struct ChunkRunner {
     return true;
   }
 
-  // Advances every run in `act` by up to `chunk` rounds (one chunk) and waits.
-  void run(tamc_gpu* g, std::vector<tamc_pt*> act, uint32_t chunk, bool use_graph, bool balance = false,
-           bool lazy_logs = false) {
-    if (enqueue(g, slots[0], std::move(act), chunk, use_graph, balance)) finish(g, slots[0], lazy_logs, 1);
-  }
-
   bool run_all_ladder(tamc_gpu* g, const std::vector<tamc_pt*>& jobs) {
     std::vector<tamc_pt*> act(jobs);
     plan_order(act);

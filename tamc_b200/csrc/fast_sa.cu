@@ -317,8 +317,8 @@ __global__ void __launch_bounds__(1024) k_sa_tab(SaFastArgs a) {
 // sums.  With CS the rows are in shared memory (16-bit byte offsets of the
 // words, couplings), else in L2.
 // Bound: the serial chain of loads and sums of a row.  (With k_sa_fast, whose
-// warps wait for their longest row, and here: 251 sites, 100 restarts, 200
-// sweeps 1584 us and 820; 8192 sites, 512 restarts, 100 sweeps 3282 us and 2003.
+// warps wait for their longest row, and here, whole calls: 251 sites, 100 restarts,
+// 200 sweeps 1.47 ms and 0.77; 8192 sites, 512 restarts, 100 sweeps 3.04 and 1.90.
 // Fetching the next slice's entries ahead made the rows in L2 slower, 2120-2280.)
 struct SaSl {
   uint32_t W, site, soff, cls, bias, colp, J, red, bytes;

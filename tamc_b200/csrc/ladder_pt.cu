@@ -1312,7 +1312,8 @@ size_t ladder_smem(const PtJob& j, int rows) {
   const int m = lad_mode(j);
   const uint32_t deg = lad_deg(m);
   if (rows && j.n > 16383) return SIZE_MAX;  // 16-bit byte offsets
-  // (the layout below counts in 32 bits; nothing near a megabyte fits anyway)
+  // (the layout below counts in 32 bits; rows of more than a megabyte, which could be
+  // read from L2, were not measured in this form)
   if (j.n > 65535 || (uint64_t)j.F.sl_rows * 192 > (1u << 20)) return SIZE_MAX;
   if (!deg && !j.F.sl_ent) return SIZE_MAX;
   return lad_carve(lad_dims(j, rows, deg, m == LAD_MSC4 || m == LAD_MSC6)).bytes;
