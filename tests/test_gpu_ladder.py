@@ -157,3 +157,22 @@ def test_serial_exchange_of_ladder_and_fused_forms_identical(tb, gpu, monkeypatc
         monkeypatch.setenv("TAMC_PT_FORM", form)
         got[form] = _everything(tb.PtRun(d, p, 5).run())
     _same(got["fused"], got["ladder"])
+
+
+# couplings beyond the fixed point's range (2^31): sums of them wrap, in every form alike
+@pytest.mark.parametrize("value", [3e9, 3e30, np.inf, np.nan])
+@pytest.mark.parametrize("kind", ["gauss2:9", "gauss3:6", "rrg:100", "qubo:300"])
+@pytest.mark.parametrize("threads,C", [(8, 2), (1, 4)])
+def test_ladder_and_other_forms_identical_on_huge_couplings(tb, gpu, monkeypatch, kind, value, threads, C):
+    h = _host(tb, kind)
+    row_ptr, col, J, bias = h.csr()
+    J = np.array(J, np.float32)
+    J[np.random.default_rng(2).integers(0, len(J), len(J) // 30 + 1)] = value
+    d = gpu.upload(tb.HostInstance.from_csr(row_ptr, col, J, bias))
+    p = tb.PtParams(40, tb.geometric_betas(0.01, 2.0, 12), 3, 0.3, True, C, threads, 7, 9, 0)
+    got = {}
+    for form in ("fused", "plain", "ladder"):
+        monkeypatch.setenv("TAMC_PT_FORM", form)
+        got[form] = _everything(tb.PtRun(d, p, 9).run())
+    _same(got["fused"], got["plain"])
+    _same(got["fused"], got["ladder"])
