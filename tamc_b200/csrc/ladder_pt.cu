@@ -490,13 +490,14 @@ __device__ uint32_t lad_bfs(const PtJob& J, const LadSm S, uint32_t seed, uint32
 // boundary terms in fixed point).  `mate`: the other replica's spin bits.  The
 // terms are summed for the pair's first replica and the second's change is the
 // negative sum, as there: every neighbour outside the cluster has the same spin in
-// both replicas and every cluster site opposite ones, so in the second's CTA (`odd`)
-// the own spins are turned.  (Its own sum would be the negative one too, but not
-// where a term is beyond the fixed point's range: that ends at -2^63 and 2^63 - 1.)
+// both replicas and every cluster site opposite ones, so in the second's CTA the
+// own spins are turned (misc[7]: 2^31 there; in a register it cost the search on
+// lattices 1 to 2 % of a round).  (Its own sum would be the negative one too, but
+// not where a term is beyond the fixed point's range: -2^63 to 2^63 - 1.)
 // Returns whether the slot had a q<0 site; *dE: the energy change (thread 0).
 template <int MODE, bool RS>
 __device__ __noinline__ bool lad_icm(const PtJob& J, const LadSm S, const uint32_t* mate, uint32_t t, uint32_t p,
-                                     bool odd, uint32_t i, uint32_t* misc, long long* dE, LadClock& pc) {
+                                     uint32_t i, uint32_t* misc, long long* dE, LadClock& pc) {
   const LadRows<MODE, RS> R(J, S);
   const uint32_t tid = threadIdx.x, T = blockDim.x, lane = tid & 31u, warp = tid >> 5, nwarp = T >> 5;
   const uint32_t n = J.n, nwb = (n + 31) / 32;
@@ -608,14 +609,13 @@ __device__ __noinline__ bool lad_icm(const PtJob& J, const LadSm S, const uint32
   }
   // boundary terms -2 s (h + sum over neighbours outside the cluster)
   long long a0 = 0;
-  const uint32_t turn = odd ? 0x80000000u : 0u;
   for (uint32_t x = tid; x < nlist; x += T) {
     const uint32_t s = list[x];
     float f = R.bias(s);
     R.each(s, [&](uint32_t c4, float j) {
       if (!bm_bit(Cb, c4 >> 2)) f += __uint_as_float(__float_as_uint(j) ^ lad_sign(c4));
     });
-    a0 += to_fx(-2.0f * __uint_as_float(__float_as_uint(f) ^ lad_word(s) ^ turn));
+    a0 += to_fx(-2.0f * __uint_as_float(__float_as_uint(f) ^ lad_word(s) ^ misc[7]));
   }
   a0 = lad_warp_sum(a0);
   if (lane == 0) red[2 * warp] = a0;
@@ -624,7 +624,7 @@ __device__ __noinline__ bool lad_icm(const PtJob& J, const LadSm S, const uint32
   for (uint32_t w = tid; w < nwb; w += T) own[w] ^= Cb[w];
   if (warp == 0) {
     const long long a = lad_warp_sum(lane < nwarp ? red[2 * lane] : 0ll);
-    if (tid == 0) *dE = odd ? -a : a;
+    if (tid == 0) *dE = misc[7] ? -a : a;
   }
   pc.lap(PHASE_ICM_APPLY);
   return true;
@@ -886,7 +886,7 @@ __device__ void lad_run(const LadJob& A) {
   const PtJob& J = A.J;
   constexpr uint32_t DEG = LadMode<MODE>::DEG;
   constexpr bool MSC = LadMode<MODE>::MSC;
-  __shared__ uint32_t misc[8];      // q<0 count, seed, waits' result, list length, [3] search counters
+  __shared__ uint32_t misc[8];      // q<0 count, seed, waits' result, list length, [3] search counters, second replica
   __shared__ unsigned long long s_D; // exchange: swapped slot pairs of the chain
   __shared__ double s_E[2];         // this replica's Ec, Er
   __shared__ float s_be;            // the round's lowest energy, and its slot
@@ -957,6 +957,7 @@ __device__ void lad_run(const LadJob& A) {
   }
   for (uint32_t j = tid; j + 1 < nt; j += T) ex[j] = J.betas[j + 1] - J.betas[j];
   if (tid == 0) {
+    misc[7] = c << 31;
     s_E[0] = J.Ec[c * J.ntp + t];
     s_E[1] = J.Er[c * J.ntp + t];
     if (MSC) {
@@ -1005,7 +1006,7 @@ __device__ void lad_run(const LadJob& A) {
       pc.lap(PHASE_ICM_SCAN);
       long long dE = 0;
       const uint32_t* mb = r ? A.post + (size_t)mate * nwb : A.bits + bstride + (size_t)mate * nwb;
-      if (lad_icm<MODE, RS>(J, S, mb, t, p, c & 1u, i, misc, &dE, pc) && tid == 0) {
+      if (lad_icm<MODE, RS>(J, S, mb, t, p, i, misc, &dE, pc) && tid == 0) {
         // the reference invalidates both caches; the next energy() is energy_ref
         s_E[1] += (double)dE * TAMC_FX_INV;
         s_E[0] = s_E[1];
