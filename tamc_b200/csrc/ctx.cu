@@ -158,6 +158,15 @@ uint32_t checkerboard_side(uint32_t L, const std::vector<uint32_t>& perm, const 
 }
 }  // namespace
 
+std::shared_mutex& capture_lock() {
+  static std::shared_mutex m;
+  return m;
+}
+static cudaError_t device_sync() {
+  std::unique_lock<std::shared_mutex> lk(capture_lock());
+  return cudaDeviceSynchronize();
+}
+
 void* dev_alloc(size_t bytes) {
   bytes = std::max<size_t>(bytes, 1);
   void* p = nullptr;
@@ -184,7 +193,7 @@ void* dev_alloc(size_t bytes) {
       }
       if (attempt == 0 && !C.pending.empty()) {
         // freed blocks become reusable once nothing in flight can still read them
-        TAMC_CUDA(cudaDeviceSynchronize());
+        TAMC_CUDA(device_sync());
         for (auto& kv : C.pending) {
           auto& r = C.ready[kv.first];
           r.insert(r.end(), kv.second.begin(), kv.second.end());
@@ -197,7 +206,7 @@ void* dev_alloc(size_t bytes) {
     cudaGetLastError();
     {
       std::lock_guard<std::mutex> lk(g_cache_mu);
-      cudaDeviceSynchronize();
+      device_sync();
       free_all_locked(g_cache[dev]);
     }
     if (cudaMalloc(&p, c) != cudaSuccess) {
@@ -232,7 +241,7 @@ void dev_cache_release(int device) {
   std::lock_guard<std::mutex> lk(g_cache_mu);
   auto it = g_cache.find(device);
   if (it == g_cache.end()) return;
-  cudaDeviceSynchronize();
+  device_sync();
   free_all_locked(it->second);
   g_cache.erase(it);
 }

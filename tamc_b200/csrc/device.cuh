@@ -5,6 +5,7 @@
 
 #include <atomic>
 #include <mutex>
+#include <shared_mutex>
 #include <string>
 #include <type_traits>
 #include <vector>
@@ -59,6 +60,9 @@ struct TraceRange {
 // destroying many small runs then costs no cudaMalloc / cudaFree each.
 void* dev_alloc(size_t bytes);
 void dev_free(void* p, size_t bytes);
+// While a stream captures, a device synchronisation in any thread fails and spoils the
+// capture: captures hold this lock shared, device synchronisations alone.
+std::shared_mutex& capture_lock();
 // Returns the cached blocks of `device` to the driver.
 void dev_cache_release(int device);
 

@@ -333,9 +333,12 @@ static void plain_run_chunk(tamc_pt* pt, uint32_t K) {
   auto it = F->graphs.find(K);
   if (it == F->graphs.end()) {
     cudaGraph_t graph;
-    TAMC_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-    plain_enqueue_rounds(pt, K);
-    TAMC_CUDA(cudaStreamEndCapture(st, &graph));
+    {
+      std::shared_lock<std::shared_mutex> capturing(capture_lock());
+      TAMC_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
+      plain_enqueue_rounds(pt, K);
+      TAMC_CUDA(cudaStreamEndCapture(st, &graph));
+    }
     cudaGraphExec_t exec;
     TAMC_CUDA(cudaGraphInstantiate(&exec, graph, 0));
     cudaGraphDestroy(graph);
@@ -1185,6 +1188,7 @@ struct ChunkRunner {
         if (sl.graph) cudaGraphDestroy(sl.graph);
         sl.exec = nullptr;
         sl.graph = nullptr;
+        std::shared_lock<std::shared_mutex> capturing(capture_lock());
         TAMC_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
         // the graph's two copies are counted at every replay below
         cudaMemcpyAsync(d_jobs.p, h_jobs, na * sizeof(PtJob), cudaMemcpyHostToDevice, st);
@@ -1192,6 +1196,7 @@ struct ChunkRunner {
         launch_all();
         cudaMemcpyAsync(sl.h_counts, counts.p, na * 4, cudaMemcpyDeviceToHost, st);
         TAMC_CUDA(cudaStreamEndCapture(st, &sl.graph));
+        capturing.unlock();
         TAMC_CUDA(cudaGraphInstantiate(&sl.exec, sl.graph, 0));
         memcpy(sl.key, key, sizeof(key));
       }

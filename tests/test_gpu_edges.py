@@ -3,6 +3,8 @@ chains with a single temperature, a single sweep, the largest and the first
 too-large fast-mode shapes, and an instance without sites.  Reference-order
 results must equal the oracle's bit for bit; fast-mode energies must match an
 FP64 recomputation."""
+import threading
+
 import numpy as np
 import pytest
 
@@ -109,3 +111,34 @@ def test_states_are_read_without_free_device_memory(tb, gpu):
         del held
         torch.cuda.empty_cache()
     assert S.tobytes() == S1.tobytes() and E.tobytes() == E1.tobytes()
+
+
+def test_captures_beside_allocations_of_another_thread(tb, gpu):
+    """A batch captures a graph for every number of runs it holds while another
+    thread creates and destroys runs, whose blocks are synchronised for reuse."""
+    h = tb.HostInstance.parse(gi.lattice(12, 2, "pm", 1))
+    p = tb.PtParams(40, tb.geometric_betas(0.2, 5.0, 8), 4, 0.5, True, 2, 8)
+    other = tb.Gpu(0)
+    stop, errors = threading.Event(), []
+
+    def churn():
+        try:
+            d = other.upload(h)
+            while not stop.is_set():
+                tb.PtRun(d, p, 1).state()
+        except Exception as e:
+            errors.append(e)
+
+    d = gpu.upload(h)
+    t = threading.Thread(target=churn)
+    t.start()
+    try:
+        for k in range(120):
+            b = tb.Batch(gpu)
+            for j in range(20 + k % 40):
+                b.add(d, p, j)
+            b.run()
+    finally:
+        stop.set()
+        t.join()
+    assert not errors
