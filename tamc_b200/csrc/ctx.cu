@@ -57,11 +57,12 @@ void xo_jump(Xo& x) {
 }
 
 template <class T>
-static T* dmalloc_copy(const T* h, size_t count) {
+static T* dmalloc_copy(const T* h, size_t count, cudaStream_t st) {
   T* d = nullptr;
   const size_t bytes = std::max<size_t>(count, 1) * sizeof(T);
   TAMC_CUDA(cudaMalloc((void**)&d, bytes));
-  if (count) TAMC_CUDA(copy_sync(d, h, count * sizeof(T), cudaMemcpyHostToDevice));
+  if (count) TAMC_CUDA(copy_async(d, h, count * sizeof(T), cudaMemcpyHostToDevice, st));
+  TAMC_CUDA(cudaStreamSynchronize(st));
   return d;
 }
 
@@ -499,7 +500,7 @@ int tamc_gpu_open(int device, tamc_gpu** out) {
     if (hdr[0] != 0x54505845u || hdr[1] != TAMC_EXPF_NUM_BUCKETS ||
         blob != 12 + 4 * ((size_t)hdr[1] + 1 + 2 * (size_t)hdr[2]))
       fail(TAMC_E_INVAL, "corrupt expf table in the library");
-    g->d_exp = dmalloc_copy((const uint32_t*)(tamc_expf_blob_begin + 12), (blob - 12) / 4);
+    g->d_exp = dmalloc_copy((const uint32_t*)(tamc_expf_blob_begin + 12), (blob - 12) / 4, g->stream);
     g->exp.off = g->d_exp;
     g->exp.keys = g->d_exp + hdr[1] + 1;
     g->exp.vals = g->exp.keys + hdr[2];
@@ -573,13 +574,18 @@ void upload_instance(tamc_gpu* g, const tamc_host_instance* hi, bool slices, tam
   try {
     UploadPack packs[2];
     inst_prepare(d, hi->h, packs[0], slices ? &packs[1] : nullptr);
+    // waited for on the stream it is on: a synchronous copy from pageable memory may
+    // return before the device has the data, and the run's stream does not wait for it
+    std::lock_guard<std::mutex> lk(g->up_mu);
+    if (!g->up_stream) TAMC_CUDA(cudaStreamCreateWithFlags(&g->up_stream, cudaStreamNonBlocking));
     for (int k = 0; k < 2; ++k) {
       const size_t bytes = packs[k].host.size();
       if (!bytes || !part_alloc(d, bytes, k == 1)) continue;
       void* const arena = k ? d->sl_arena : d->arena;
-      TAMC_CUDA(copy_sync(arena, packs[k].host.data(), bytes, cudaMemcpyHostToDevice));
+      TAMC_CUDA(copy_async(arena, packs[k].host.data(), bytes, cudaMemcpyHostToDevice, g->up_stream));
       packs[k].bind(arena);
     }
+    TAMC_CUDA(cudaStreamSynchronize(g->up_stream));
   } catch (...) {
     tamc_gpu_instance_destroy(d);
     throw;

@@ -26,8 +26,8 @@ namespace tamc {
 
 // Bytes this library has copied between host and device (all contexts, since
 // load), by direction; reported through tamc_copy_bytes.  Every host<->device
-// copy goes through copy_async / copy_sync, or calls count_copy where a
-// captured graph replays a copy.
+// copy goes through copy_async, or calls count_copy where a captured graph
+// replays a copy.
 extern std::atomic<uint64_t> g_h2d_bytes, g_d2h_bytes;
 inline void count_copy(size_t bytes, cudaMemcpyKind kind) {
   if (kind == cudaMemcpyHostToDevice) g_h2d_bytes.fetch_add(bytes, std::memory_order_relaxed);
@@ -36,10 +36,6 @@ inline void count_copy(size_t bytes, cudaMemcpyKind kind) {
 inline cudaError_t copy_async(void* dst, const void* src, size_t bytes, cudaMemcpyKind kind, cudaStream_t st) {
   count_copy(bytes, kind);
   return cudaMemcpyAsync(dst, src, bytes, kind, st);
-}
-inline cudaError_t copy_sync(void* dst, const void* src, size_t bytes, cudaMemcpyKind kind) {
-  count_copy(bytes, kind);
-  return cudaMemcpy(dst, src, bytes, kind);
 }
 
 // A named NVTX range over a host-side scope (nvtx3, header-only: it costs a

@@ -142,3 +142,27 @@ def test_captures_beside_allocations_of_another_thread(tb, gpu):
         stop.set()
         t.join()
     assert not errors
+
+
+def test_uploads_of_several_threads_are_there_when_they_return(tb, gpu):
+    """Contexts in threads of their own, each uploading instances one by one and
+    running them at once, beside the others' copies."""
+    hosts = [tb.HostInstance.parse(gi.qubo_er(n, 6.0, n), qubo=True) for n in (61, 300, 1500)]
+    p = tb.PtParams(6, tb.geometric_betas(0.2, 5.0, 8), 4, 0.5, True, 2, 8)
+    want = [tb.PtRun(gpu.upload(h), p, 2).run().state()[0].tobytes() for h in hosts]
+    wrong = []
+
+    def work(g):
+        try:
+            for k in range(60):
+                if tb.PtRun(g.upload(hosts[k % 3]), p, 2).run().state()[0].tobytes() != want[k % 3]:
+                    wrong.append(k)
+        except Exception as e:
+            wrong.append(e)
+
+    threads = [threading.Thread(target=work, args=(tb.Gpu(0),)) for _ in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
