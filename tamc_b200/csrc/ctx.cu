@@ -159,6 +159,19 @@ uint32_t checkerboard_side(uint32_t L, const std::vector<uint32_t>& perm, const 
 }
 }  // namespace
 
+void kernel_smem(const void* f, size_t smem) {
+  static std::mutex mu;
+  static std::map<std::pair<int, const void*>, size_t> set;
+  int dev = 0;
+  TAMC_CUDA(cudaGetDevice(&dev));
+  std::lock_guard<std::mutex> lk(mu);
+  size_t& cur = set[{dev, f}];
+  if (smem > cur) {
+    TAMC_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    cur = smem;
+  }
+}
+
 std::shared_mutex& capture_lock() {
   static std::shared_mutex m;
   return m;

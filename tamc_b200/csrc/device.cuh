@@ -56,6 +56,9 @@ struct TraceRange {
 // destroying many small runs then costs no cudaMalloc / cudaFree each.
 void* dev_alloc(size_t bytes);
 void dev_free(void* p, size_t bytes);
+// Lets kernel `f` take `smem` bytes of dynamic shared memory.  The limit only grows (per
+// device), so that neither another thread's launch nor a captured one is left without.
+void kernel_smem(const void* f, size_t smem);
 // While a stream captures, a device synchronisation in any thread fails and spoils the
 // capture: captures hold this lock shared, device synchronisations alone.
 std::shared_mutex& capture_lock();

@@ -3445,23 +3445,12 @@ size_t fused_smem_bytes(const PtJob& j, uint32_t T, bool csr_smem) {
   return carve_all(nullptr, nullptr, j.n, j.nw, j.C, j.ntp, j.qps, T, j.F.nnz, csr_smem, j.icm_group, j.icm_uf != 0);
 }
 
-// The fused kernels' dynamic shared-memory limits only grow (per device), so
-// that a captured launch stays valid whatever smaller launches ran since.
 using FusedFn = void (*)(const PtJob*, uint32_t, uint32_t*);
 static FusedFn fused_fn(FusedKind kind) {
   return kind == FUSED_ROWS ? k_pt_rows : kind == FUSED_MIXED ? k_pt_fused<true> : k_pt_fused<false>;
 }
 static void fused_attr(size_t smem, FusedKind kind) {
-  static std::mutex mu;
-  static std::map<std::pair<int, FusedKind>, size_t> set;
-  int dev = 0;
-  TAMC_CUDA(cudaGetDevice(&dev));
-  std::lock_guard<std::mutex> lk(mu);
-  size_t& cur = set[{dev, kind}];
-  if (smem > cur) {
-    TAMC_CUDA(cudaFuncSetAttribute(fused_fn(kind), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    cur = smem;
-  }
+  kernel_smem(reinterpret_cast<const void*>(fused_fn(kind)), smem);
 }
 
 int fused_blocks_per_sm(uint32_t T, size_t smem, FusedKind kind) {
@@ -3510,7 +3499,7 @@ static void plain_launch(void (*k)(KArgs...), uint32_t grid, uint32_t block, siz
 
 void plain_launch_head(cudaStream_t st, const PtJob* d_job, PlainCtl* ctl, long long* acc, int mode, size_t smem,
                        int stage) {
-  TAMC_CUDA(cudaFuncSetAttribute(k_plain_head, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  kernel_smem(reinterpret_cast<const void*>(k_plain_head), smem);
   plain_launch(k_plain_head, 1, 1024, smem, st, d_job, ctl, acc, mode, stage);
 }
 
@@ -3532,7 +3521,7 @@ template <uint32_t CL, uint32_t DEG, uint32_t PS>
 static void launch_icm_cl(cudaStream_t st, uint32_t nclusters, size_t smem, const PtJob* d_job, PlainCtl* ctl,
                           long long* icm_dE, uint32_t* icm_valid, unsigned long long* dm) {
   auto k = k_plain_icm_cl<CL, DEG, PS>;
-  TAMC_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  kernel_smem(reinterpret_cast<const void*>(k), smem);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(nclusters * CL);
   cfg.blockDim = dim3(1024);
@@ -3611,7 +3600,7 @@ static bool plain_launch_icm_lattice(cudaStream_t st, const PtJob& j, const PtJo
   const size_t smem = stage_exch ? lat + exch : std::max(lat, exch);
   const uint32_t grid = (j.C / 2) * (j.nt - j.lo);
   auto go = [&](auto k) {
-    TAMC_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kernel_smem(reinterpret_cast<const void*>(k), smem);
     plain_launch(k, grid, 1024, smem, st, d_job, ctl, icm_dE, icm_valid, dm, stage_exch);
   };
   if (L == 16 && dim == 2) go(k_plain_icm_lat<16, 2>);
@@ -3632,7 +3621,7 @@ bool plain_launch_icm(cudaStream_t st, const PtJob& j, const PtJob* d_job, Plain
   if (plain_icm_smem(j, stage) > smem_limit) stage = 2;
   if (plain_icm_smem(j, stage) > smem_limit) stage = 0;
   const size_t smem = plain_icm_smem(j, stage);
-  TAMC_CUDA(cudaFuncSetAttribute(k_plain_icm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  kernel_smem(reinterpret_cast<const void*>(k_plain_icm), smem);
   plain_launch(k_plain_icm, grid, 1024, smem, st, d_job, ctl, icm_dE, icm_valid, stage, dm);
   return true;
 }
@@ -3640,7 +3629,7 @@ bool plain_launch_icm(cudaStream_t st, const PtJob& j, const PtJob* d_job, Plain
 void plain_launch_exch(cudaStream_t st, const PtJob& j, const PtJob* d_job, PlainCtl* ctl, const long long* icm_dE,
                        uint32_t* icm_valid, unsigned long long* dm) {
   const size_t smem = plain_exch_smem(j.n, j.C, j.ntp);
-  TAMC_CUDA(cudaFuncSetAttribute(k_plain_exch, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  kernel_smem(reinterpret_cast<const void*>(k_plain_exch), smem);
   plain_launch(k_plain_exch, 1, 1024, smem, st, d_job, ctl, icm_dE, icm_valid, dm);
 }
 
@@ -3655,7 +3644,7 @@ template <bool CLOSE>
 static void plain_launch_sweep_t(cudaStream_t st, const PtJob& j, const PtJob* d_job, PlainCtl* ctl,
                                  uint32_t color, uint32_t grid, uint32_t T, size_t smem, long long* acc) {
   auto go = [&](auto k) {
-    TAMC_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kernel_smem(reinterpret_cast<const void*>(k), smem);
     plain_launch(k, grid, T, smem, st, d_job, ctl, color, acc);
   };
   const uint32_t deg = j.F.udeg == 4 || j.F.udeg == 6 ? j.F.udeg : 0;
@@ -3682,7 +3671,7 @@ void plain_launch_sweep(cudaStream_t st, const PtJob& j, const PtJob* d_job, Pla
     const size_t smem = al16((size_t)j.nw * MSC_WORDS * 4) + (size_t)(T / 32) * 32 * 8 +
                         (last ? 2 * al16((size_t)j.C * j.ntp * 8) : 0);
     auto go = [&](auto k) {
-      TAMC_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      kernel_smem(reinterpret_cast<const void*>(k), smem);
       plain_launch(k, grid, T, smem, st, d_job, ctl, color, acc);
     };
     if (j.F.udeg == 4) {

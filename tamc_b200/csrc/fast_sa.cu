@@ -457,7 +457,7 @@ __global__ void k_pack_states(const uint32_t* __restrict__ words, uint32_t n, ui
 
 template <class K>
 void launch_k(K k, cudaStream_t st, const SaFastArgs& a, uint32_t ncta, uint32_t T, size_t smem) {
-  TAMC_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  kernel_smem(reinterpret_cast<const void*>(k), smem);
   k<<<ncta, T, smem, st>>>(a);
   TAMC_CUDA(cudaGetLastError());
 }

@@ -1335,19 +1335,7 @@ void ladder_shape(LadJob& a, int rows, uint32_t cta0) {
   if (const char* e = getenv("TAMC_LADDER_POLLS")) a.polls = (uint32_t)strtoul(e, nullptr, 10);
 }
 
-// The kernel's dynamic shared-memory limit only grows (per device).
-static void ladder_attr(size_t smem) {
-  static std::mutex mu;
-  static std::map<int, size_t> set;
-  int dev = 0;
-  TAMC_CUDA(cudaGetDevice(&dev));
-  std::lock_guard<std::mutex> lk(mu);
-  size_t& cur = set[dev];
-  if (smem > cur) {
-    TAMC_CUDA(cudaFuncSetAttribute(k_pt_ladder, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    cur = smem;
-  }
-}
+static void ladder_attr(size_t smem) { kernel_smem(reinterpret_cast<const void*>(k_pt_ladder), smem); }
 
 size_t ladder_smem_limit(const tamc_gpu* g) {
   static std::atomic<size_t> own{0};  // the kernel's static shared memory

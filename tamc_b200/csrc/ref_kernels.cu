@@ -1120,8 +1120,7 @@ static size_t ref_smem_limit() {
 }
 template <typename K>
 static void ref_smem_attr(K k, size_t bytes) {
-  if (bytes > 40960)
-    TAMC_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ref_smem_limit()));
+  if (bytes > 40960) kernel_smem(reinterpret_cast<const void*>(k), bytes);
 }
 uint32_t ref_icm(cudaStream_t st, const RefInst& I, uint64_t nnz, const RefPt& P, const ExpTable& X, Xo* rng,
                  int* err) {

@@ -166,3 +166,25 @@ def test_uploads_of_several_threads_are_there_when_they_return(tb, gpu):
     for t in threads:
         t.join()
     assert not wrong
+
+
+def test_one_kernel_with_two_sizes_in_several_threads(tb, gpu):
+    """Annealing 16 and 1024 sites takes 5 and 150 KB of the same kernel's shared
+    memory, in each of six threads at once."""
+    b = np.linspace(0.1, 3.0, 4).astype(np.float32)
+    wrong = []
+
+    def work(g, side):
+        try:
+            d = g.upload(tb.HostInstance.parse(gi.lattice(side, 2, "gauss", side)))
+            want = tb.sa_run(d, b, 64, 1, 7)[0].tobytes()
+            wrong.extend(k for k in range(3000) if tb.sa_run(d, b, 64, 1, 7)[0].tobytes() != want)
+        except Exception as e:
+            wrong.append(e)
+
+    threads = [threading.Thread(target=work, args=(tb.Gpu(0), side)) for side in (4, 32) * 3]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
